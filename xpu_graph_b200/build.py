@@ -1,8 +1,9 @@
-"""Builds libxg_sm100.so (the C-ABI kernel library) in-tree with nvcc for sm_100a.
+"""Builds libxg_sm100.so (the C-ABI kernel library) in-tree with nvcc for sm_100a, and libxg_sm100_torch.so (the torch
+operators on top of it) with the host compiler.
 
 Usage: ``python -m xpu_graph_b200.build [--force] [--verbose]``.
-Objects go to ``xpu_graph_b200/csrc/build/``; the shared library lands next to this file so that it
-travels with the source tree. Nothing here needs a GPU: nvcc cross-compiles.
+Objects go to ``xpu_graph_b200/csrc/build/``; the shared libraries land next to this file so that they
+travel with the source tree. Nothing here needs a GPU: nvcc cross-compiles.
 """
 from __future__ import annotations
 
@@ -16,6 +17,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ_DIR = os.path.join(CSRC, "build")
 LIB_PATH = os.path.join(HERE, "libxg_sm100.so")
+TORCH_LIB_PATH = os.path.join(HERE, "libxg_sm100_torch.so")
+TORCH_SOURCE = "torch_ops.cpp"
 
 SOURCES = [
     "abi.cu",
@@ -49,6 +52,31 @@ def _nvcc() -> str:
     return cand
 
 
+def _cuda_home() -> str:
+    return os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+
+
+def _compile_torch_ops(src: str, obj: str) -> str:
+    import sysconfig
+
+    import torch
+
+    inc = os.path.join(os.path.dirname(torch.__file__), "include")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-isystem", inc, "-isystem", os.path.join(inc, "torch", "csrc", "api", "include"), "-isystem", sysconfig.get_paths()["include"],
+           "-isystem", os.path.join(_cuda_home(), "include"), "-c", src, "-o", obj]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed for {src}:\n{proc.stdout}\n{proc.stderr}")
+    return ""
+
+
+def _link(cmd) -> None:
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError(f"link failed:\n{proc.stdout}\n{proc.stderr}")
+
+
 def _deps_mtime() -> float:
     paths = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
     paths.append(os.path.join(HERE, "..", "include", "xg_sm100.h"))
@@ -68,32 +96,33 @@ def _compile_one(nvcc: str, src: str, obj: str, verbose: bool) -> str:
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile every kernel source and link the shared library. Returns the library path."""
+    """Compile every source and link the two shared libraries. Returns the kernel library's path."""
     nvcc = _nvcc()
     os.makedirs(OBJ_DIR, exist_ok=True)
     hdr_time = _deps_mtime()
-    jobs = []
-    objs = []
-    for name in SOURCES:
-        src = os.path.join(CSRC, name)
-        obj = os.path.join(OBJ_DIR, name.replace(".cu", ".o"))
-        objs.append(obj)
+
+    def job(name):
+        src, obj = os.path.join(CSRC, name), os.path.join(OBJ_DIR, os.path.splitext(name)[0] + ".o")
         stale = force or not os.path.exists(obj) or os.path.getmtime(obj) < max(os.path.getmtime(src), hdr_time)
-        if stale:
-            jobs.append((src, obj))
-    if jobs:
-        with cf.ThreadPoolExecutor(max_workers=min(8, len(jobs))) as pool:
-            futs = [pool.submit(_compile_one, nvcc, s, o, verbose) for s, o in jobs]
-            for f in futs:
-                out = f.result()
-                if out:
-                    print(out, file=sys.stderr)
-    need_link = bool(jobs) or not os.path.exists(LIB_PATH)
-    if need_link:
-        cmd = [nvcc, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", LIB_PATH, *objs]
-        proc = subprocess.run(cmd, capture_output=True, text=True)
-        if proc.returncode != 0:
-            raise RuntimeError(f"link failed:\n{proc.stdout}\n{proc.stderr}")
+        return src, obj, stale
+
+    kernels = [job(name) for name in SOURCES]
+    torch_src, torch_obj, torch_stale = job(TORCH_SOURCE)
+    with cf.ThreadPoolExecutor(max_workers=8) as pool:
+        futs = [pool.submit(_compile_torch_ops, torch_src, torch_obj)] if torch_stale else []
+        futs += [pool.submit(_compile_one, nvcc, s, o, verbose) for s, o, stale in kernels if stale]
+        for f in futs:
+            out = f.result()
+            if out:
+                print(out, file=sys.stderr)
+    if any(stale for _, _, stale in kernels) or not os.path.exists(LIB_PATH):
+        _link([nvcc, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", LIB_PATH, *[o for _, o, _ in kernels]])
+    if torch_stale or not os.path.exists(TORCH_LIB_PATH):
+        import torch
+
+        torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+        _link([os.environ.get("CXX", "g++"), "-shared", "-o", TORCH_LIB_PATH, torch_obj, f"-L{HERE}", "-l:libxg_sm100.so", "-Wl,-rpath,$ORIGIN",
+               f"-L{torch_lib}", f"-Wl,-rpath,{torch_lib}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch_python"])
     return LIB_PATH
 
 

@@ -1,8 +1,8 @@
-"""ctypes binding of libxg_sm100.so (the C ABI declared in include/xg_sm100.h).
+"""ctypes binding of libxg_sm100.so (the C ABI declared in include/xg_sm100.h), and the loader of libxg_sm100_torch.so
+(the torch operators, which call the same C ABI natively).
 
-The library is loaded lazily and only from this package's directory. There is no fallback: if the
-shared object is missing, fails to load, or lacks a symbol, ``XgLibraryError`` is raised and every
-op that needs it fails loudly.
+The libraries are loaded only from this package's directory. There is no fallback: if a shared object is missing, fails to
+load, or lacks a symbol, ``XgLibraryError`` is raised and every op that needs it fails loudly.
 """
 from __future__ import annotations
 
@@ -14,6 +14,7 @@ from ctypes import POINTER, c_char_p, c_float, c_int, c_int64, c_uint, c_uint8, 
 
 LIB_NAME = "libxg_sm100.so"
 LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), LIB_NAME)
+TORCH_LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "libxg_sm100_torch.so")
 
 XG_OK = 0
 XG_F32, XG_BF16, XG_F16 = 0, 1, 2
@@ -84,6 +85,7 @@ SIGNATURES = {
 
 _lock = threading.Lock()
 _lib = None
+_torch_lib = None
 
 
 def load(path: str | None = None) -> ctypes.CDLL:
@@ -114,6 +116,26 @@ def load(path: str | None = None) -> ctypes.CDLL:
         if path is None:
             _lib = lib
         return lib
+
+
+def load_torch_ops() -> ctypes.PyDLL:
+    """Load the operators of torch.ops.xg_sm100 (once)."""
+    global _torch_lib
+    import torch  # noqa: F401  (the library links against it)
+
+    load()
+    with _lock:
+        if _torch_lib is None:
+            if not os.path.exists(TORCH_LIB_PATH):
+                raise XgLibraryError(f"{TORCH_LIB_PATH} not found: build it with `python -m xpu_graph_b200.build`.")
+            try:
+                lib = ctypes.PyDLL(TORCH_LIB_PATH)
+            except OSError as e:  # pragma: no cover - depends on the environment
+                raise XgLibraryError(f"cannot load {TORCH_LIB_PATH}: {e}") from e
+            lib.xg_torch_set_hook.argtypes = [ctypes.py_object, ctypes.py_object]
+            lib.xg_torch_set_hook.restype = None
+            _torch_lib = lib
+    return _torch_lib
 
 
 def last_error() -> str:
@@ -151,9 +173,9 @@ QUERY_ENTRY_POINTS = frozenset({"xg_version", "xg_device_arch_ok", "xg_last_erro
 
 @contextlib.contextmanager
 def call_hook(before=None, after=None):
-    """While active, every call into the library made through ``load()`` is reported: ``before(name, args)`` just
-    before the C function runs and ``after(name, args, rc)`` just after it returned (both optional; ``args`` are the
-    marshalled arguments in the header's order). For observers that live outside the ops - launch counters, timers
+    """While active, every call into the library made through ``load()`` or by a torch operator is reported:
+    ``before(name, args)`` just before the C function runs and ``after(name, args, rc)`` just after it returned (both
+    optional; ``args`` are the marshalled arguments in the header's order; the operators report no queries). For observers that live outside the ops - launch counters, timers
     that bracket a kernel with events on the launching stream, call logs. Not thread-safe; do not nest."""
     lib = load()
     saved = {}
@@ -170,8 +192,11 @@ def call_hook(before=None, after=None):
             return rc
 
         setattr(lib, name, wrapped)
+    torch_lib = load_torch_ops()
+    torch_lib.xg_torch_set_hook(before, after)
     try:
         yield lib
     finally:
+        torch_lib.xg_torch_set_hook(None, None)
         for name, fn in saved.items():
             setattr(lib, name, fn)

@@ -10,13 +10,14 @@ tensors and no library handles, so compiled graphs stay picklable for the compil
 """
 from __future__ import annotations
 
-from typing import List, Optional, Sequence, Tuple
+from types import SimpleNamespace
 
 import torch
 
 from . import ops  # noqa: F401  (registers torch.ops.xg_sm100.*)
 
-_X = torch.ops.xg_sm100
+# the operators' overloads, looked up once: torch.ops.xg_sm100.<op>(...) resolves its overload on every call
+_X = SimpleNamespace(**{name: getattr(torch.ops.xg_sm100, name).default for name in ops.OP_NAMES})
 
 _SUPPORTED = (torch.float32, torch.bfloat16, torch.float16)
 # Device types on which the fusions are applied. The kernels exist for CUDA only; the host-side test
