@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 
@@ -21,6 +22,71 @@ inline int check_launch(const char* what) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(XG_ERR_LAUNCH, "%s: %s", what, cudaGetErrorString(e));
     return XG_OK;
+}
+
+// ---- launches ---------------------------------------------------------------------------------
+// Kernels are launched with programmatic stream serialisation: the next kernel's CTAs may be placed, and set up their
+// barriers and tensor memory, while this one drains. A kernel therefore calls pdl_wait() before its first access to global
+// memory (it returns once the previous kernel has completed and its writes are visible) and pdl_trigger() once its own CTA
+// holds all the resources it will ask for (tensor memory above all: a successor that took columns a CTA of this grid still
+// needs would wait for a kernel that waits for it). Every kernel has to reach pdl_wait(), or its own successor would not be
+// ordered behind its predecessor. What it saves on B200 is the set-up and launch latency between two kernels of a stream.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// for kernels without a set-up worth overlapping
+__device__ __forceinline__ void pdl_sync() {
+    pdl_trigger();
+    pdl_wait();
+}
+
+struct LaunchOptions {
+    unsigned cluster = 0;  // CTAs per thread-block cluster where the kernel does not fix it itself
+    // false: plain stream order. For grids below a full set of resident CTAs of which several fit one SM: placed early,
+    // they pack onto the few SMs that the previous kernel leaves free and share them for good (a 128-CTA fp32 dense layer
+    // at two CTAs per SM took 1.7 x as long behind a tensor-core kernel).
+    bool early = true;
+};
+template <typename... P, typename... A>
+void launch_with(const LaunchOptions& o, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    unsigned n = 0;
+    if (o.early) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (o.cluster) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = o.cluster;
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    (void)cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);  // the caller's check_launch() picks up a failure
+}
+template <typename... P, typename... A>
+void launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
+    launch_with(LaunchOptions{}, kern, grid, block, smem, st, args...);
+}
+
+// Opt a kernel in to `bytes` of dynamic shared memory, once per device (`done`: one bit per device).
+template <typename K>
+bool reserve_smem(K kern, int bytes, std::atomic<uint64_t>& done) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    const uint64_t bit = 1ull << (dev & 63);
+    if (done.load(std::memory_order_acquire) & bit) return true;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    done.fetch_or(bit, std::memory_order_release);
+    return true;
 }
 
 inline int num_sms() {

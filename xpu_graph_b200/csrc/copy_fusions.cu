@@ -44,6 +44,7 @@ __device__ __forceinline__ U zero_unit() {
 
 template <typename U>
 __global__ void __launch_bounds__(kCopyThreads) seg_copy_kernel(const __grid_constant__ SegCopyParams p) {
+    pdl_sync();
     __shared__ SegDesc segs[kMaxSegs];
     __shared__ uint32_t lut[kLutMax];
     for (int k = threadIdx.x; k < p.nseg; k += kCopyThreads) segs[k] = p.seg[k];
@@ -117,7 +118,7 @@ template <typename U>
 int launch_seg_copy(const SegCopyParams& p, cudaStream_t st) {
     const int64_t grid = (p.rows + p.rows_per_cta - 1) / p.rows_per_cta;
     if (grid > 0x7fffffffLL) return fail(XG_ERR_TOO_LARGE, "xg_seg_copy: too many row tiles");
-    seg_copy_kernel<U><<<(unsigned)grid, kCopyThreads, 0, st>>>(p);
+    launch(seg_copy_kernel<U>, (unsigned)grid, kCopyThreads, 0, st, p);
     return check_launch("xg_seg_copy");
 }
 
@@ -158,6 +159,7 @@ struct GatherParams {
 
 template <typename U>
 __global__ void __launch_bounds__(kCopyThreads) gather_rows_kernel(const __grid_constant__ GatherParams p) {
+    pdl_sync();
     __shared__ const char* tab[kMaxSegs];
     __shared__ int64_t trows[kMaxSegs];
     for (int k = threadIdx.x; k < p.F; k += kCopyThreads) {
@@ -202,7 +204,7 @@ template <typename U>
 int launch_gather(const GatherParams& p, cudaStream_t st) {
     const int64_t grid = (p.rows + kGatherRows - 1) / kGatherRows;
     if (grid > 0x7fffffffLL) return fail(XG_ERR_TOO_LARGE, "xg_gather_rows: too many tiles");
-    gather_rows_kernel<U><<<(unsigned)grid, kCopyThreads, 0, st>>>(p);
+    launch(gather_rows_kernel<U>, (unsigned)grid, kCopyThreads, 0, st, p);
     return check_launch("xg_gather_rows");
 }
 

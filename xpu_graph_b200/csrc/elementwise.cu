@@ -22,6 +22,7 @@ struct RopeParams {
 // grid.x covers (s, half-vector) of one (b, h) plane with 32-bit index math; grid.y strides over planes.
 template <typename T>
 __global__ void __launch_bounds__(256) rope_vec_kernel(const RopeParams p) {
+    pdl_sync();
     constexpr int EPV = Vec16<T>::N;
     const int hv_per_row = (int)(p.D / 2 / EPV);
     const uint32_t per_plane = (uint32_t)p.S * (uint32_t)hv_per_row;
@@ -55,6 +56,7 @@ __global__ void __launch_bounds__(256) rope_vec_kernel(const RopeParams p) {
 
 template <typename T>
 __global__ void __launch_bounds__(256) rope_scalar_kernel(const RopeParams p) {
+    pdl_sync();
     const int64_t half = p.D / 2;
     const int64_t total = p.B * p.H * p.S * half;
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -92,12 +94,12 @@ int launch_rope(const RopeParams& p, cudaStream_t st) {
         if (gy < 1) gy = 1;
         if (gy > 65535) gy = 65535;
         if (gy > planes) gy = planes;
-        rope_vec_kernel<T><<<dim3((unsigned)gx, (unsigned)gy), 256, 0, st>>>(p);
+        launch(rope_vec_kernel<T>, dim3((unsigned)gx, (unsigned)gy), 256, 0, st, p);
     } else {
         const int64_t total = p.B * p.H * p.S * half;
         const int64_t grid = (total + 255) / 256;
         if (grid > 0x7fffffffLL) return fail(XG_ERR_TOO_LARGE, "xg_rope: tensor too large");
-        rope_scalar_kernel<T><<<(unsigned)grid, 256, 0, st>>>(p);
+        launch(rope_scalar_kernel<T>, (unsigned)grid, 256, 0, st, p);
     }
     return check_launch("xg_rope");
 }
@@ -128,6 +130,7 @@ __device__ __forceinline__ float silu_f(float g) {
 // same column of all ROWS rows at once (2*ROWS loads in flight, no index division anywhere).
 template <typename T, int ROWS>
 __global__ void __launch_bounds__(256) swiglu_vec_kernel(const SwigluParams p) {
+    pdl_sync();
     constexpr int EPV = Vec16<T>::N;
     const int vec_per_row = (int)(p.cols / EPV);
     const int64_t r0 = (int64_t)blockIdx.x * ROWS;
@@ -163,6 +166,7 @@ __global__ void __launch_bounds__(256) swiglu_vec_kernel(const SwigluParams p) {
 // leaves no idle lanes at the end of every row.
 template <typename T, int U>
 __global__ void __launch_bounds__(256) swiglu_flat_kernel(const SwigluParams p, int64_t total_vec) {
+    pdl_sync();
     constexpr int EPV = Vec16<T>::N;
     const T* gp = reinterpret_cast<const T*>(p.gate);
     const T* up = reinterpret_cast<const T*>(p.up);
@@ -192,6 +196,7 @@ __global__ void __launch_bounds__(256) swiglu_flat_kernel(const SwigluParams p, 
 
 template <typename T>
 __global__ void __launch_bounds__(256) swiglu_scalar_kernel(const SwigluParams p) {
+    pdl_sync();
     const int64_t total = p.rows * p.cols;
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
@@ -212,15 +217,15 @@ int launch_swiglu(const SwigluParams& p, cudaStream_t st) {
         const int64_t total_vec = p.rows * (p.cols / EPV);
         const int64_t grid = (total_vec + 256 * UNROLL - 1) / (256 * UNROLL);
         if (grid > 0x7fffffffLL) return fail(XG_ERR_TOO_LARGE, "xg_swiglu: tensor too large");
-        if (grid > 0) swiglu_flat_kernel<T, UNROLL><<<(unsigned)grid, 256, 0, st>>>(p, total_vec);
+        if (grid > 0) launch(swiglu_flat_kernel<T, UNROLL>, (unsigned)grid, 256, 0, st, p, total_vec);
     } else if (vec_ok && p.cols / EPV < 0x7fffffffLL) {
         const int64_t grid = (p.rows + UNROLL - 1) / UNROLL;
         if (grid > 0x7fffffffLL) return fail(XG_ERR_TOO_LARGE, "xg_swiglu: tensor too large");
-        swiglu_vec_kernel<T, UNROLL><<<(unsigned)grid, 256, 0, st>>>(p);
+        launch(swiglu_vec_kernel<T, UNROLL>, (unsigned)grid, 256, 0, st, p);
     } else {
         const int64_t grid = (p.rows * p.cols + 255) / 256;
         if (grid > 0x7fffffffLL) return fail(XG_ERR_TOO_LARGE, "xg_swiglu: tensor too large");
-        swiglu_scalar_kernel<T><<<(unsigned)grid, 256, 0, st>>>(p);
+        launch(swiglu_scalar_kernel<T>, (unsigned)grid, 256, 0, st, p);
     }
     return check_launch("xg_swiglu");
 }

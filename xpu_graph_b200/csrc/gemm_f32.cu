@@ -139,6 +139,7 @@ __device__ __forceinline__ void gemm_f32_tile(const GemmF32Params& p) {
 
 template <typename T, int TM, int TN, int BK>
 __global__ void __launch_bounds__(256) gemm_f32_kernel(const GemmF32Params p) {
+    pdl_sync();
     gemm_f32_tile<T, TM, TN, BK>(p);
 }
 
@@ -165,6 +166,7 @@ __device__ __forceinline__ GemmF32Params entry_params(const GemmF32Params& p, co
 
 template <typename T, int TM, int TN, int BK>
 __global__ void __launch_bounds__(256) gemm_f32_group_kernel(const GemmF32Params p, const __grid_constant__ GemmF32Group g) {
+    pdl_sync();
     const GemmF32Params pe = entry_params(p, g);
     gemm_f32_tile<T, TM, TN, BK>(pe);
 }
@@ -256,11 +258,13 @@ __device__ __forceinline__ void gemm_f32_panel_tile(const GemmF32Params& p) {
 
 template <int TM, int TN>
 __global__ void __launch_bounds__(128) gemm_f32_panel_kernel(const GemmF32Params p) {
+    pdl_sync();
     gemm_f32_panel_tile<TM, TN>(p);
 }
 
 template <int TM, int TN>
 __global__ void __launch_bounds__(128) gemm_f32_panel_group_kernel(const GemmF32Params p, const __grid_constant__ GemmF32Group g) {
+    pdl_sync();
     const GemmF32Params pe = entry_params(p, g);
     gemm_f32_panel_tile<TM, TN>(pe);
 }
@@ -270,13 +274,10 @@ int launch_panel_group(const GemmF32Params& p, const GemmF32Group& g, int count,
     constexpr int BM = 8 * TM, BN = 16 * TN;
     constexpr int smem = (BM + BN) * kPanelPitch * (int)sizeof(float);
     auto kern = gemm_f32_panel_group_kernel<TM, TN>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return fail(XG_ERR_LAUNCH, "xg_gemm_group_bias_act(f32): cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    }
+    static std::atomic<uint64_t> reserved{0};
+    if (!reserve_smem(kern, smem, reserved)) return fail(XG_ERR_LAUNCH, "xg_gemm_group_bias_act(f32): cannot reserve %d bytes of shared memory", smem);
     dim3 grid((unsigned)((p.N + BN - 1) / BN), (unsigned)((p.M + BM - 1) / BM), (unsigned)count);
-    kern<<<grid, 128, smem, st>>>(p, g);
+    launch_with({.early = false}, kern, grid, 128, smem, st, p, g);
     return check_launch("xg_gemm_group_bias_act(f32)");
 }
 
@@ -285,13 +286,10 @@ int launch_panel(const GemmF32Params& p, cudaStream_t st) {
     constexpr int BM = 8 * TM, BN = 16 * TN;
     constexpr int smem = (BM + BN) * kPanelPitch * (int)sizeof(float);
     auto kern = gemm_f32_panel_kernel<TM, TN>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return fail(XG_ERR_LAUNCH, "xg_gemm_bias_act(f32): cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    }
+    static std::atomic<uint64_t> reserved{0};
+    if (!reserve_smem(kern, smem, reserved)) return fail(XG_ERR_LAUNCH, "xg_gemm_bias_act(f32): cannot reserve %d bytes of shared memory", smem);
     dim3 grid((unsigned)((p.N + BN - 1) / BN), (unsigned)((p.M + BM - 1) / BM));
-    kern<<<grid, 128, smem, st>>>(p);
+    launch_with({.early = false}, kern, grid, 128, smem, st, p);
     return check_launch("xg_gemm_bias_act(f32)");
 }
 
@@ -313,11 +311,11 @@ int gemm_f32_entry(const void* A, const void* B, const void* bias, const void* r
     if (big_tiles >= 2LL * num_sms()) {
         dim3 grid((unsigned)((N + 127) / 128), (unsigned)((M + 127) / 128));
         if ((M + 127) / 128 > 65535) return fail(XG_ERR_TOO_LARGE, "xg_gemm_bias_act(f32): M too large");
-        gemm_f32_kernel<float, 8, 8, 16><<<grid, 256, 0, st>>>(p);
+        launch_with({.early = false}, gemm_f32_kernel<float, 8, 8, 16>, grid, 256, 0, st, p);
     } else {
         dim3 grid((unsigned)((N + 63) / 64), (unsigned)((M + 63) / 64));
         if ((M + 63) / 64 > 65535) return fail(XG_ERR_TOO_LARGE, "xg_gemm_bias_act(f32): M too large");
-        gemm_f32_kernel<float, 4, 4, 16><<<grid, 256, 0, st>>>(p);
+        launch_with({.early = false}, gemm_f32_kernel<float, 4, 4, 16>, grid, 256, 0, st, p);
     }
     return check_launch("xg_gemm_bias_act(f32)");
 }
@@ -334,11 +332,11 @@ int gemm_simt16_entry(const void* A, const void* B, const void* bias, const void
     if ((M + bm - 1) / bm > 65535) return fail(XG_ERR_TOO_LARGE, "xg_gemm_bias_act: M too large for the unaligned 16-bit path");
     dim3 grid((unsigned)((N + bm - 1) / bm), (unsigned)((M + bm - 1) / bm));
     if (dtype == XG_BF16) {
-        if (big) gemm_f32_kernel<__nv_bfloat16, 8, 8, 16><<<grid, 256, 0, st>>>(p);
-        else gemm_f32_kernel<__nv_bfloat16, 4, 4, 16><<<grid, 256, 0, st>>>(p);
+        if (big) launch_with({.early = false}, gemm_f32_kernel<__nv_bfloat16, 8, 8, 16>, grid, 256, 0, st, p);
+        else launch_with({.early = false}, gemm_f32_kernel<__nv_bfloat16, 4, 4, 16>, grid, 256, 0, st, p);
     } else {
-        if (big) gemm_f32_kernel<__half, 8, 8, 16><<<grid, 256, 0, st>>>(p);
-        else gemm_f32_kernel<__half, 4, 4, 16><<<grid, 256, 0, st>>>(p);
+        if (big) launch_with({.early = false}, gemm_f32_kernel<__half, 8, 8, 16>, grid, 256, 0, st, p);
+        else launch_with({.early = false}, gemm_f32_kernel<__half, 4, 4, 16>, grid, 256, 0, st, p);
     }
     return check_launch("xg_gemm_bias_act (16-bit, FMA path)");
 }
@@ -375,11 +373,11 @@ int gemm_f32_group_entry(const void* const* A, const void* const* W, const void*
             rc = tiles_32x64 * 3 >= 2LL * num_sms() ? launch_panel_group<4, 4>(p, g, n, st) : launch_panel_group<2, 2>(p, g, n, st);
         } else if (((M + 127) / 128) * ((N + 127) / 128) * n >= 2LL * num_sms()) {
             dim3 grid((unsigned)((N + 127) / 128), (unsigned)((M + 127) / 128), (unsigned)n);
-            gemm_f32_group_kernel<float, 8, 8, 16><<<grid, 256, 0, st>>>(p, g);
+            launch_with({.early = false}, gemm_f32_group_kernel<float, 8, 8, 16>, grid, 256, 0, st, p, g);
             rc = check_launch("xg_gemm_group_bias_act(f32)");
         } else {
             dim3 grid((unsigned)((N + 63) / 64), (unsigned)((M + 63) / 64), (unsigned)n);
-            gemm_f32_group_kernel<float, 4, 4, 16><<<grid, 256, 0, st>>>(p, g);
+            launch_with({.early = false}, gemm_f32_group_kernel<float, 4, 4, 16>, grid, 256, 0, st, p, g);
             rc = check_launch("xg_gemm_group_bias_act(f32)");
         }
         if (rc != XG_OK) return rc;

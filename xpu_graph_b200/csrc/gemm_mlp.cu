@@ -135,6 +135,7 @@ mlp_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
+    pdl_sync();  // the tensor memory is held
 
     if (warp == 0) {
         // ------------------------------ TMA producer ------------------------------
@@ -378,14 +379,11 @@ int launch_mlp(const char* who, const void* x, int layers, const void* const* w,
     }
     if (!maps_ok) return fail(XG_ERR_UNSUPPORTED, "%s: tensor-map encoding failed", who);
     auto kern = mlp_kernel<T>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MLP_SMEM_BYTES);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return fail(XG_ERR_LAUNCH, "%s: cannot reserve shared memory: %s", who, cudaGetErrorString(e));
-    }
+    static std::atomic<uint64_t> reserved{0};
+    if (!reserve_smem(kern, MLP_SMEM_BYTES, reserved)) return fail(XG_ERR_LAUNCH, "%s: cannot reserve shared memory", who);
     const int sms = num_sms();
     const unsigned grid = (unsigned)(p.num_m_blocks < sms ? p.num_m_blocks : sms);
-    kern<<<grid, MLP_THREADS, MLP_SMEM_BYTES, st>>>(tx, tw[0], tw[1], tw[2], p);
+    launch(kern, grid, MLP_THREADS, MLP_SMEM_BYTES, st, tx, tw[0], tw[1], tw[2], p);
     return check_launch(who);
 }
 

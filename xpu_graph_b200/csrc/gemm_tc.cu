@@ -468,6 +468,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
+    pdl_sync();  // the tensor memory is held
 
     const int tiles_per_entry = p.num_m_blocks * p.num_n_blocks;
     const int num_tiles = tiles_per_entry * p.splits * batch_of(p);  // work units: (batch entry, tile, split); batch > 1 has no splits
@@ -685,6 +686,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     ptx::cluster_sync();  // both CTAs' barriers are initialised before anyone signals across the pair
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
+    pdl_sync();  // the tensor memory is held
 
     const int num_tiles = p.num_m_blocks * p.num_n_blocks;  // 256-row blocks x OUT_BN-column blocks
     const int nkb = p.num_k_blocks;
@@ -799,12 +801,8 @@ template <typename T, bool SWIGLU>
 int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tb2, const GemmParams& p,
                      cudaStream_t st) {
     auto kern = gemm_tc_pair_kernel<T, SWIGLU>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM_BYTES);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return fail(XG_ERR_LAUNCH, "xg_gemm_bias_act: cannot reserve %d bytes of shared memory: %s", PAIR_SMEM_BYTES,
-                    cudaGetErrorString(e));
-    }
+    static std::atomic<uint64_t> reserved{0};
+    if (!reserve_smem(kern, PAIR_SMEM_BYTES, reserved)) return fail(XG_ERR_LAUNCH, "xg_gemm_bias_act: cannot reserve %d bytes of shared memory", PAIR_SMEM_BYTES);
     const int tiles = p.num_m_blocks * p.num_n_blocks;
     // as many pairs as can be resident at once (a pair needs two free SMs of one TPC)
     static thread_local int max_pairs_cached[2] = {0, 0};
@@ -829,16 +827,16 @@ int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtenso
         max_pairs = n < num_sms() / 2 ? n : num_sms() / 2;
     }
     const int pairs = tiles < max_pairs ? tiles : max_pairs;
-    kern<<<2 * pairs, kGemmThreads, PAIR_SMEM_BYTES, st>>>(ta, tb, tb2, p);
+    // plain stream order: a persistent kernel of hundreds of microseconds hides no set-up, and placed early (pairs starting
+    // at different times) it ran 1.4 % (decoder layer of 16384 tokens) to 2.5 % slower
+    launch_with({.early = false}, kern, 2 * pairs, kGemmThreads, PAIR_SMEM_BYTES, st, ta, tb, tb2, p);
     return check_launch("xg_gemm_bias_act (CTA pairs)");
 }
 
 // Second pass of split-K: out = act(sum_s partial[s] + bias + residual), 4 columns per thread.
 template <typename T>
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const GemmParams p) {
-    // Launched with programmatic stream serialisation: its CTAs may be placed while the GEMM is still draining; this
-    // returns once the GEMM grid has completed and its partial sums are visible.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_sync();
     const int64_t n4 = (p.N + 3) / 4;
     const int64_t total = p.M * n4;
     const int64_t idx = (int64_t)blockIdx.x * 256 + threadIdx.x;
@@ -885,34 +883,16 @@ int launch_gemm_tc(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
                    cudaStream_t st) {
     using Cfg = GemmCfg<BN>;
     auto kern = gemm_tc_kernel<T, BN, SWIGLU, B_MN>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return fail(XG_ERR_LAUNCH, "xg_gemm_bias_act: cannot reserve %d bytes of shared memory: %s", Cfg::SMEM_BYTES,
-                    cudaGetErrorString(e));
-    }
+    static std::atomic<uint64_t> reserved{0};
+    if (!reserve_smem(kern, Cfg::SMEM_BYTES, reserved)) return fail(XG_ERR_LAUNCH, "xg_gemm_bias_act: cannot reserve %d bytes of shared memory", Cfg::SMEM_BYTES);
     const int64_t tiles = (int64_t)p.num_m_blocks * p.num_n_blocks * p.splits * batch_of(p);
     const int grid = (int)(tiles < num_sms() ? tiles : num_sms());
-    kern<<<grid, kGemmThreads, Cfg::SMEM_BYTES, st>>>(ta, tb, tb2, p);
+    launch(kern, grid, kGemmThreads, Cfg::SMEM_BYTES, st, ta, tb, tb2, p);
     int rc = check_launch("xg_gemm_bias_act");
     if (rc != XG_OK || p.splits <= 1) return rc;
     const int64_t total = p.M * ((p.N + 3) / 4);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((total + 255) / 256));
-    cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = st;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;  // overlap this launch's latency with the GEMM's tail
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    cudaError_t le = cudaLaunchKernelEx(&cfg, splitk_reduce_kernel<T>, p);
-    if (le != cudaSuccess) {
-        cudaGetLastError();
-        return fail(XG_ERR_LAUNCH, "xg_gemm_bias_act (split-K reduce): %s", cudaGetErrorString(le));
-    }
-    return XG_OK;
+    launch(splitk_reduce_kernel<T>, (unsigned)((total + 255) / 256), 256, 0, st, p);
+    return check_launch("xg_gemm_bias_act (split-K reduce)");
 }
 
 
@@ -969,6 +949,7 @@ gemm_tc_group_kernel(const __grid_constant__ GroupTable tab, const GemmParams p,
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
+    pdl_sync();  // the tensor memory is held
 
     const int tiles_per_entry = p.num_m_blocks * p.num_n_blocks;
     const int num_tiles = tiles_per_entry * count;  // work units: (entry, tile)
@@ -1085,15 +1066,11 @@ template <typename T, int BN, bool B_MN>
 int launch_gemm_group(const GroupTable& tab, const GemmParams& p, int count, cudaStream_t st) {
     using Cfg = GemmCfg<BN>;
     auto kern = gemm_tc_group_kernel<T, BN, B_MN>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return fail(XG_ERR_LAUNCH, "xg_gemm_group_bias_act: cannot reserve %d bytes of shared memory: %s", Cfg::SMEM_BYTES,
-                    cudaGetErrorString(e));
-    }
+    static std::atomic<uint64_t> reserved{0};
+    if (!reserve_smem(kern, Cfg::SMEM_BYTES, reserved)) return fail(XG_ERR_LAUNCH, "xg_gemm_group_bias_act: cannot reserve %d bytes of shared memory", Cfg::SMEM_BYTES);
     const int64_t tiles = (int64_t)p.num_m_blocks * p.num_n_blocks * count;
     const int grid = (int)(tiles < num_sms() ? tiles : num_sms());
-    kern<<<grid, kGemmThreads, Cfg::SMEM_BYTES, st>>>(tab, p, count);
+    launch(kern, grid, kGemmThreads, Cfg::SMEM_BYTES, st, tab, p, count);
     return check_launch("xg_gemm_group_bias_act");
 }
 

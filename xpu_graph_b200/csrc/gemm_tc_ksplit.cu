@@ -181,6 +181,7 @@ gemm_tc_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     ptx::cluster_sync();  // every CTA's barriers exist before anyone signals across the cluster
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
+    pdl_sync();  // the tensor memory is held
 
     if (warp == 0) {
         // ------------------------------ TMA producer (every CTA) ------------------------------
@@ -371,16 +372,9 @@ int launch_ksplit(const void* A, const void* W, const void* bias, const void* re
                   int64_t K, int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int act, int S, int tn, cudaStream_t st) {
     constexpr bool is_bf16 = std::is_same<T, __nv_bfloat16>::value;
     auto kern = gemm_tc_ksplit_kernel<T>;
-    static thread_local bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, KS_SMEM_BYTES);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            return fail(XG_ERR_LAUNCH, "xg_gemm_bias_act: cannot reserve %d bytes of shared memory: %s", KS_SMEM_BYTES,
-                        cudaGetErrorString(e));
-        }
-        attr_set = true;
-    }
+    static std::atomic<uint64_t> reserved{0};
+    if (!reserve_smem(kern, KS_SMEM_BYTES, reserved))
+        return fail(XG_ERR_LAUNCH, "xg_gemm_bias_act: cannot reserve %d bytes of shared memory", KS_SMEM_BYTES);
     CUtensorMap ta, tw;
     if (!make_tmap_2d_16bit(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BM, BK, is_bf16) ||
         !make_tmap_2d_16bit(&tw, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, (uint32_t)(tn / 2), BK, is_bf16))
@@ -402,24 +396,8 @@ int launch_ksplit(const void* A, const void* W, const void* bias, const void* re
     p.stages = S > 1 ? KS_STAGES_SPLIT : KS_STAGES_WHOLE;
     const int64_t tiles = (int64_t)p.num_m_blocks * p.num_n_blocks;
     if (tiles * 2 * S > 0x7fffffffLL) return fail(XG_ERR_TOO_LARGE, "xg_gemm_bias_act: too many tiles for one launch");
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(tiles * 2 * S));
-    cfg.blockDim = dim3(KS_THREADS);
-    cfg.dynamicSmemBytes = KS_SMEM_BYTES;
-    cfg.stream = st;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = (unsigned)(2 * S);
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    cudaError_t le = cudaLaunchKernelEx(&cfg, kern, ta, tw, p);
-    if (le != cudaSuccess) {
-        cudaGetLastError();
-        return fail(XG_ERR_LAUNCH, "xg_gemm_bias_act (k-split clusters of %d): %s", 2 * S, cudaGetErrorString(le));
-    }
-    return XG_OK;
+    launch_with({.cluster = (unsigned)(2 * S)}, kern, (unsigned)(tiles * 2 * S), KS_THREADS, KS_SMEM_BYTES, st, ta, tw, p);
+    return check_launch("xg_gemm_bias_act (k-split clusters)");
 }
 
 bool ksplit_shape_ok(int S, int tn, int64_t nkb) {

@@ -88,6 +88,7 @@ __device__ __noinline__ void ms_layer(const float* __restrict__ in, float* __res
 
 template <typename T>
 __global__ void __launch_bounds__(MS_THREADS) mlp_small_kernel(const MlpSmallParams p) {
+    pdl_sync();
     extern __shared__ __align__(16) float ms_smem[];
     // [weights of layer 0 | 1 | 2: Kp x N each, rows k >= K zero][biases][activation buffer A][activation buffer B]
     float* w_s[3] = {ms_smem, ms_smem, ms_smem};
@@ -231,16 +232,15 @@ template <typename T>
 int launch_small(const MlpSmallParams& p, cudaStream_t st) {
     const int smem = (int)(smem_floats(p.dims, p.layers) * 4);
     auto kern = mlp_small_kernel<T>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return fail(XG_ERR_LAUNCH, "xg_mlp_small_bias_act: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    }
+    static std::atomic<uint64_t> reserved{0};
+    constexpr int kMostSmem = 160 * 1024;  // above (24576 weights + 3 x 128 biases + 2 x 32 x 132 activations) x 4 bytes
+    if (smem > kMostSmem || !reserve_smem(kern, kMostSmem, reserved))
+        return fail(XG_ERR_LAUNCH, "xg_mlp_small_bias_act: cannot reserve %d bytes of shared memory", smem);
     const int64_t blocks = (p.M + MS_ROWS - 1) / MS_ROWS;
     int per_sm = (200 * 1024) / (smem + 1024);  // CTAs that fit an SM by shared memory; 8 x 256 threads at most
     per_sm = per_sm < 1 ? 1 : (per_sm > 8 ? 8 : per_sm);
     const int64_t cap = (int64_t)per_sm * num_sms();
-    kern<<<(unsigned)(blocks < cap ? blocks : cap), MS_THREADS, smem, st>>>(p);
+    launch(kern, (unsigned)(blocks < cap ? blocks : cap), MS_THREADS, smem, st, p);
     return check_launch("xg_mlp_small_bias_act");
 }
 

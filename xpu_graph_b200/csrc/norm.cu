@@ -49,6 +49,7 @@ __device__ __forceinline__ void load_coef(const void* p, int w_is_f32, int64_t e
 // V = 16-byte vectors per lane, WPR = warps per row. WPR == 1: 4 independent rows per CTA.
 template <typename T, int V, int WPR, bool LN, bool BIAS>
 __global__ void __launch_bounds__((WPR == 1 ? 4 : WPR) * 32) norm_vec_kernel(const NormParams p) {
+    pdl_sync();
     constexpr int EPV = Vec16<T>::N;
     constexpr int WARPS = (WPR == 1 ? 4 : WPR);
     const int lane = threadIdx.x & 31;
@@ -179,6 +180,7 @@ __global__ void __launch_bounds__((WPR == 1 ? 4 : WPR) * 32) norm_vec_kernel(con
 // L1/L2 for each pass. Only ragged or unaligned shapes land here.
 template <typename T, bool LN>
 __global__ void __launch_bounds__(128) norm_generic_kernel(const NormParams p) {
+    pdl_sync();
     __shared__ float red[4];
     __shared__ float bcast;
     const int64_t row = blockIdx.x;
@@ -236,7 +238,7 @@ template <typename T, int V, int WPR, bool LN, bool BIAS>
 void launch_vec(const NormParams& p, cudaStream_t st) {
     constexpr int WARPS = (WPR == 1 ? 4 : WPR);
     const int64_t grid = (WPR == 1) ? (p.rows + WARPS - 1) / WARPS : p.rows;
-    norm_vec_kernel<T, V, WPR, LN, BIAS><<<(unsigned)grid, WARPS * 32, 0, st>>>(p);
+    launch(norm_vec_kernel<T, V, WPR, LN, BIAS>, (unsigned)grid, WARPS * 32, 0, st, p);
 }
 
 template <typename T, bool LN, bool BIAS>
@@ -258,7 +260,7 @@ int launch_norm(const NormParams& p, cudaStream_t st, const char* name) {
         else if (nvec <= 32 * 8 * 8) launch_vec<T, 8, 8, LN, BIAS>(p, st);
         else launch_vec<T, 8, 16, LN, BIAS>(p, st);
     } else {
-        norm_generic_kernel<T, LN><<<(unsigned)p.rows, 128, 0, st>>>(p);
+        launch(norm_generic_kernel<T, LN>, (unsigned)p.rows, 128, 0, st, p);
     }
     return check_launch(name);
 }

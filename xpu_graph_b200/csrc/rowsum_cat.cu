@@ -32,6 +32,7 @@ struct RowSumParams {
 
 template <typename T, int V, bool MUL>
 __global__ void __launch_bounds__(256) rowsum_cat_kernel(const __grid_constant__ RowSumParams p) {
+    pdl_sync();
     const int k = blockIdx.y;
     const int cv = p.C / V;  // column vectors per row
     const T* a = reinterpret_cast<const T*>(p.a[k]);
@@ -102,6 +103,7 @@ __global__ void __launch_bounds__(256) rowsum_cat_kernel(const __grid_constant__
 // Segments share a[0], a_bs[0] and r0[0]; r1 ascending (slot[] maps back to the caller's order).
 template <typename T, int V>
 __global__ void __launch_bounds__(256) rowsum_prefix_kernel(const __grid_constant__ RowSumParams p) {
+    pdl_sync();
     const int cv = p.C / V;
     const T* a = reinterpret_cast<const T*>(p.a[0]);
     const int64_t total = p.B * cv;
@@ -163,16 +165,16 @@ int launch_rowsum(const RowSumParams& p, bool mul, bool prefix, bool vec, cudaSt
     const int64_t cap = 32LL * num_sms();
     const unsigned gx = (unsigned)(work < cap ? (work > 0 ? work : 1) : cap);
     if (prefix) {
-        if (vec) rowsum_prefix_kernel<T, V><<<gx, 256, 0, st>>>(p);
-        else rowsum_prefix_kernel<T, 1><<<gx, 256, 0, st>>>(p);
+        if (vec) launch(rowsum_prefix_kernel<T, V>, gx, 256, 0, st, p);
+        else launch(rowsum_prefix_kernel<T, 1>, gx, 256, 0, st, p);
     } else {
         dim3 grid(gx, (unsigned)p.n);
         if (mul) {
-            if (vec) rowsum_cat_kernel<T, V, true><<<grid, 256, 0, st>>>(p);
-            else rowsum_cat_kernel<T, 1, true><<<grid, 256, 0, st>>>(p);
+            if (vec) launch(rowsum_cat_kernel<T, V, true>, grid, 256, 0, st, p);
+            else launch(rowsum_cat_kernel<T, 1, true>, grid, 256, 0, st, p);
         } else {
-            if (vec) rowsum_cat_kernel<T, V, false><<<grid, 256, 0, st>>>(p);
-            else rowsum_cat_kernel<T, 1, false><<<grid, 256, 0, st>>>(p);
+            if (vec) launch(rowsum_cat_kernel<T, V, false>, grid, 256, 0, st, p);
+            else launch(rowsum_cat_kernel<T, 1, false>, grid, 256, 0, st, p);
         }
     }
     return check_launch("xg_rowsum_cat");

@@ -185,6 +185,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
     volatile FlashStride* stride = reinterpret_cast<volatile FlashStride*>(tmem_slot + 2);
 
     if ((ptx::smem_u32(smem) & 1023u) != 0) {  // uniform over the CTA: the swizzled tiles need this alignment
+        pdl_sync();
         if (threadIdx.x == 0) atomicOr(&g_sdpa_status[0], 128u);
         return;
     }
@@ -223,6 +224,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_sync();  // the tensor memory is held
     constexpr int fmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
 
     if (warp == 0) {
@@ -583,17 +585,14 @@ int launch_flash_tc(const SdpaParams& p, cudaStream_t st) {
     fp.causal = p.causal;
     const bool masked = p.mask != nullptr || p.Skv % FN != 0 || !(p.scale > 0.f);
     auto kern = masked ? flash_tc_kernel<T, D, true> : flash_tc_kernel<T, D, false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return fail(XG_ERR_LAUNCH, "xg_sdpa_fwd: cannot reserve shared memory: %s", cudaGetErrorString(e));
-    }
+    static std::atomic<uint64_t> reserved[2];
+    if (!reserve_smem(kern, Cfg::SMEM_BYTES, reserved[masked])) return fail(XG_ERR_LAUNCH, "xg_sdpa_fwd: cannot reserve shared memory");
     const int64_t tiles = p.B * p.H * ((p.Sq + FM - 1) / FM);
     if (tiles > 0x7fffffffLL) return fail(XG_ERR_TOO_LARGE, "xg_sdpa_fwd: too many tiles");
     const int64_t resident = 2LL * num_sms();  // persistent CTAs, two per SM
     const int64_t pairs = (tiles + 1) / 2;      // a CTA takes tiles in neighbouring (heavy, light) pairs
     const unsigned grid = (unsigned)(pairs < resident ? pairs : resident);
-    kern<<<grid, kFlashThreads, Cfg::SMEM_BYTES, st>>>(tq, tk, tv, fp);
+    launch_with({.early = grid == resident}, kern, grid, kFlashThreads, Cfg::SMEM_BYTES, st, tq, tk, tv, fp);
     return check_launch("xg_sdpa_fwd");
 }
 
@@ -608,6 +607,7 @@ constexpr int kSimtKeys = 16;  // key / value rows whose loads are in flight tog
 
 template <typename T>
 __global__ void __launch_bounds__(kSimtWarps * 32) sdpa_simt_kernel(const SdpaParams p) {
+    pdl_sync();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t gr = (int64_t)blockIdx.x * kSimtWarps + warp;  // global query row over (b, h, i)
     if (gr >= p.B * p.H * p.Sq) return;
@@ -725,6 +725,7 @@ struct TileCfg {
 
 template <typename T, int D>
 __global__ void __launch_bounds__(kTileThreads) sdpa_tile_kernel(const SdpaParams p) {
+    pdl_sync();
     using Cfg = TileCfg<D>;
     constexpr int KS = Cfg::KS;
     constexpr int NU = D / 32;  // output columns per lane
@@ -877,14 +878,11 @@ template <typename T, int D>
 int launch_tile(const SdpaParams& p, cudaStream_t st) {
     using Cfg = TileCfg<D>;
     auto kern = sdpa_tile_kernel<T, D>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return fail(XG_ERR_LAUNCH, "xg_sdpa_fwd: cannot reserve shared memory: %s", cudaGetErrorString(e));
-    }
+    static std::atomic<uint64_t> reserved{0};
+    if (!reserve_smem(kern, Cfg::SMEM_BYTES, reserved)) return fail(XG_ERR_LAUNCH, "xg_sdpa_fwd: cannot reserve shared memory");
     const int64_t qt = (p.Sq + kTileQ - 1) / kTileQ, bh = p.B * p.H;
     if (qt > 0x7fffffffLL || bh > 65535) return -1;  // the caller falls back to the row-per-warp kernel
-    kern<<<dim3((unsigned)qt, (unsigned)bh), kTileThreads, Cfg::SMEM_BYTES, st>>>(p);
+    launch_with({.early = false}, kern, dim3((unsigned)qt, (unsigned)bh), kTileThreads, Cfg::SMEM_BYTES, st, p);
     return check_launch("xg_sdpa_fwd");
 }
 
@@ -903,7 +901,7 @@ int launch_simt(const SdpaParams& p, cudaStream_t st) {
     const int64_t rows = p.B * p.H * p.Sq;
     const int64_t grid = (rows + kSimtWarps - 1) / kSimtWarps;
     if (grid > 0x7fffffffLL) return fail(XG_ERR_TOO_LARGE, "xg_sdpa_fwd: too many rows");
-    sdpa_simt_kernel<T><<<(unsigned)grid, kSimtWarps * 32, 0, st>>>(p);
+    launch(sdpa_simt_kernel<T>, (unsigned)grid, kSimtWarps * 32, 0, st, p);
     return check_launch("xg_sdpa_fwd");
 }
 

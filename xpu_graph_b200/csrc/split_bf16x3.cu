@@ -18,6 +18,7 @@ __device__ __forceinline__ void split3(float x, __nv_bfloat16& a, __nv_bfloat16&
 template <bool TRANSPOSE>
 __global__ void __launch_bounds__(256) split_bf16x3_kernel(const float* __restrict__ x, int64_t rows, int64_t K, int64_t ld,
                                                            int64_t Kp, __nv_bfloat16* __restrict__ out) {
+    pdl_sync();
     const int64_t groups = Kp / 8;  // 8 consecutive k per thread: one 16-byte store per plane
     const int64_t total = rows * groups;
     for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < total; e += (int64_t)gridDim.x * 256) {
@@ -71,8 +72,8 @@ extern "C" int xg_split_bf16x3(const void* x, int64_t rows, int64_t K, int64_t l
     const unsigned grid = (unsigned)(work < cap ? work : cap);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (transpose)
-        split_bf16x3_kernel<true><<<grid, 256, 0, st>>>(reinterpret_cast<const float*>(x), rows, K, ld, Kp, reinterpret_cast<__nv_bfloat16*>(out3));
+        launch(split_bf16x3_kernel<true>, grid, 256, 0, st, reinterpret_cast<const float*>(x), rows, K, ld, Kp, reinterpret_cast<__nv_bfloat16*>(out3));
     else
-        split_bf16x3_kernel<false><<<grid, 256, 0, st>>>(reinterpret_cast<const float*>(x), rows, K, ld, Kp, reinterpret_cast<__nv_bfloat16*>(out3));
+        launch(split_bf16x3_kernel<false>, grid, 256, 0, st, reinterpret_cast<const float*>(x), rows, K, ld, Kp, reinterpret_cast<__nv_bfloat16*>(out3));
     return check_launch("xg_split_bf16x3");
 }

@@ -22,6 +22,7 @@ struct Sum3dParams {
 
 template <typename T>
 __global__ void __launch_bounds__(256) sum3d_kernel(const __grid_constant__ Sum3dParams p) {
+    pdl_sync();
     const int t = blockIdx.y;
     const T* x = reinterpret_cast<const T*>(p.in[t]);
     T* o = reinterpret_cast<T*>(p.out[t]);
@@ -96,9 +97,9 @@ extern "C" int xg_sum3d(const void* const* inputs, void* const* outputs, const i
         const unsigned gx = (unsigned)(max_work < cap ? max_work : cap);
         dim3 grid(gx, (unsigned)p.n);
         switch (dtype) {
-            case XG_F32: sum3d_kernel<float><<<grid, 256, 0, st>>>(p); break;
-            case XG_BF16: sum3d_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(p); break;
-            default: sum3d_kernel<__half><<<grid, 256, 0, st>>>(p); break;
+            case XG_F32: launch(sum3d_kernel<float>, grid, 256, 0, st, p); break;
+            case XG_BF16: launch(sum3d_kernel<__nv_bfloat16>, grid, 256, 0, st, p); break;
+            default: launch(sum3d_kernel<__half>, grid, 256, 0, st, p); break;
         }
         int rc = check_launch("xg_sum3d");
         if (rc != XG_OK) return rc;
