@@ -52,8 +52,8 @@ const char* xg_last_error(void);
 /*
  * Status word of the tensor-core kernels on the current device: 0 = healthy; non-zero = a bounded
  * wait inside a kernel expired (bit 0 producer, bit 1 MMA issuer, bit 2 epilogue, bits 4-6 the same
- * roles of the attention kernel, bits 8-10 of the cluster dense kernel, bits 16-18 of the chained-layer kernel) and that
- * launch's output is invalid. This is the one entry point
+ * roles of the attention kernel, bits 8-10 of the cluster dense kernel, bits 16-18 of the chained-layer kernel, bits 24-25
+ * of the fp32 FMA kernel) and that launch's output is invalid. This is the one entry point
  * that synchronises (it copies the word back); reset != 0 clears it. No reference counterpart.
  */
 int xg_tc_status(unsigned int* status, int reset);
@@ -140,6 +140,10 @@ int xg_gemm_bias_act_ws(const void* A, const void* B, const void* bias, const vo
                         int64_t ldr, int trans_b, int act, int dtype, void* workspace,
                         int64_t workspace_bytes, void* stream);
 int64_t xg_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int dtype);
+/* Further scratch with which xg_gemm_bias_act_ws first copies operands whose rows no tensor map can address into rows that
+ * it can (0 when there are none, or K is so short that the copies do not pay); without it they are read as they are. */
+int64_t xg_gemm_copy_bytes(const void* A, const void* B, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int trans_b,
+                           int dtype);
 
 /*
  * The same dense layer (16-bit dtypes, W given as [N,K]) on the thread-block-cluster kernel with the caller's
@@ -198,6 +202,14 @@ int64_t xg_gemm_f32x3_padded_k(int64_t K);
 int xg_split_bf16x3(const void* x, int64_t rows, int64_t K, int64_t ld, int transpose, void* out3, void* stream);
 int xg_gemm_f32x3(const void* A3, const void* W3, const void* bias, const void* residual, void* out, int64_t M,
                   int64_t N, int64_t K, int64_t ldc, int64_t ldr, int act, int out_planes, void* stream);
+
+/*
+ * Operand copy for rows that no tensor map can address: out[r][c] = src[r][c] (transpose = 0) or src[c][r] for r < rows,
+ * c < cols, zero for cols <= c < out_ld; ld and out_ld in elements of elem_size (2 or 4) bytes. out is 16-byte aligned and
+ * out_ld a multiple of 16 bytes; src needs only its element alignment. No reference counterpart.
+ */
+int xg_pad_rows(const void* src, int64_t rows, int64_t cols, int64_t ld, int transpose, void* out, int64_t out_ld, int elem_size,
+                void* stream);
 
 /*
  * Batched form: out[b] = act( A[b] @ W[b] + bias[b] + residual[b] ), batch strides in elements

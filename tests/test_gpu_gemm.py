@@ -821,3 +821,45 @@ def test_config3_cell(cuda_device, M, N, act):
         lin = DenseLayerModule(False)(x, w, True, None, "none")
         lin_b = DenseLayerModule(False)(x, w, True, b, "none")
         assert ((lin_b.float() - lin.float()) - b.float()).abs().max().item() < 0.05
+
+
+@pytest.mark.parametrize("with_res", [False, True])
+@pytest.mark.parametrize("M,K,N", [(1, 4, 1), (7, 32, 33), (8, 36, 64), (9, 260, 129), (16, 256, 32), (17, 1000, 31), (33, 96, 500),
+                                   (128, 2052, 40), (5, 4100, 8), (700, 64, 96)])
+def test_dense_fp32_fma_tiles(cuda_device, M, K, N, with_res):
+    """The tiled fp32 kernel at the edges of its tiles (8 / 16 rows, 32 / 64 / 128 columns), of its K slices (32) and with
+    K split over clusters. Bound: rounding of a K-term fp32 sum, sqrt(K) * 2^-24 of the terms' 2-norm at four sigma."""
+    g = torch.Generator().manual_seed(51)
+    x, w, b = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g), torch.randn(N, generator=g)
+    r = torch.randn(M, N, generator=g) if with_res else None
+    out = torch.ops.xg_sm100.dense(x.to(cuda_device), w.to(cuda_device), True, b.to(cuda_device), r.to(cuda_device) if with_res else None, "relu")
+    want = x.double() @ w.double().t() + b.double() + (r.double() if with_res else 0.0)
+    diff = (out.cpu().double() - want.clamp_min(0)).abs()
+    terms = (x.double().square() @ w.double().square().t()).sqrt() + b.double().abs() + (r.double().abs() if with_res else 0.0)
+    assert (diff <= 4 * K ** 0.5 * 2.0 ** -24 * terms + 1e-30).all(), diff.max().item()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,K,N,weight_trans,offset", [(3, 97, 5, True, 0), (40, 131, 70, False, 0), (130, 203, 264, True, 1), (1, 1001, 33, False, 1),
+                                                       (260, 96, 31, False, 0)])
+def test_dense_operands_copied_into_addressable_rows(cuda_device, M, K, N, weight_trans, offset, dtype):
+    """Row lengths and bases that are no multiples of 16 bytes, [K, N] weights: the operands are copied into rows the fast
+    kernels can address inside the one call; same result as with the scratch withheld (the kernel that reads them in place)."""
+    from xpu_graph_b200 import lib
+
+    g = torch.Generator().manual_seed(52)
+    flat = torch.randn(M * K + offset, generator=g).to(dtype).to(cuda_device)
+    x = flat[offset:].view(M, K)
+    wflat = (torch.randn(N * K + offset, generator=g) * K ** -0.5).to(dtype).to(cuda_device)
+    w = wflat[offset:].view((N, K) if weight_trans else (K, N))
+    b = torch.randn(N, generator=g).to(dtype).to(cuda_device)
+    with LaunchCounter() as calls:
+        got = torch.ops.xg_sm100.dense(x, w, weight_trans, b, None, "silu")
+    assert calls.names == ["xg_gemm_bias_act_ws"]
+    want = torch.empty_like(got)
+    L = lib.load()
+    lib.check(L.xg_gemm_bias_act(x.data_ptr(), w.data_ptr(), b.data_ptr(), None, want.data_ptr(), M, N, K, x.stride(0), w.stride(0), N, 0,
+                                 1 if weight_trans else 0, lib.ACT_CODES["silu"],
+                                 {torch.float32: lib.XG_F32, torch.bfloat16: lib.XG_BF16, torch.float16: lib.XG_F16}[dtype],
+                                 torch.cuda.current_stream().cuda_stream), "xg_gemm_bias_act")
+    assert_parity(got, want.cpu(), f"dense {M}x{K}x{N} {dtype} through copies")

@@ -32,6 +32,7 @@ SOURCES = [
     "mlp_small.cu",
     "gemm_f32.cu",
     "split_bf16x3.cu",
+    "pad_rows.cu",
     "sdpa.cu",
     "sum3d.cu",
     "rowsum_cat.cu",

@@ -342,12 +342,10 @@ Tensor dense(const Tensor& x_in, const Tensor& weight, bool weight_trans, const 
         XG_CALL(xg_gemm_f32x3, ptr(a3), ptr(w3), ptr(bias), ptr(residual), mut(out), M, N, K, N, ldr, a, 0, on.stream);
         return out;
     }
-    Tensor ws;
-    int64_t ws_bytes = 0;
-    if (dt != at::kFloat && M <= 128) {
-        ws_bytes = xg_gemm_workspace_bytes(M, N, K, code);
-        if (ws_bytes > 0) ws = new_tensor({ws_bytes}, at::kByte, x);  // split-K scratch for weight-streaming shapes (small M)
-    }
+    // scratch: split-K partial sums of weight-streaming shapes (small M), copies of operands no tensor map addresses
+    int64_t ws_bytes = dt != at::kFloat && M <= 128 ? xg_gemm_workspace_bytes(M, N, K, code) : 0;
+    ws_bytes += xg_gemm_copy_bytes(ptr(x), ptr(w.t), M, N, K, row_stride(x), row_stride(w.t), w.trans ? 1 : 0, code);
+    const Tensor ws = ws_bytes > 0 ? new_tensor({ws_bytes}, at::kByte, x) : Tensor();
     XG_CALL(xg_gemm_bias_act_ws, ptr(x), ptr(w.t), ptr(bias), ptr(residual), mut(out), M, N, K, row_stride(x), row_stride(w.t), N, ldr,
             w.trans ? 1 : 0, a, code, mut(ws), ws_bytes, on.stream);
     return out;

@@ -47,6 +47,7 @@ SIGNATURES = {
     "xg_gemm_bias_act_ws": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64,
                                     c_int64, c_int64, c_int64, c_int, c_int, c_int, c_void_p, c_int64, c_void_p]),
     "xg_gemm_workspace_bytes": (c_int64, [c_int64, c_int64, c_int64, c_int]),
+    "xg_gemm_copy_bytes": (c_int64, [c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_int64, c_int, c_int]),
     "xg_gemm_bias_act_cluster": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64,
                                          c_int64, c_int64, c_int64, c_int, c_int, c_int, c_int, c_void_p]),
     "xg_gemm_cluster_plan": (c_int, [c_int64, c_int64, c_int64, c_int, POINTER(c_int), POINTER(c_int)]),
@@ -77,6 +78,7 @@ SIGNATURES = {
     "xg_split_bf16x3": (c_int, [c_void_p, c_int64, c_int64, c_int64, c_int, c_void_p, c_void_p]),
     "xg_gemm_f32x3": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_int64,
                               c_int, c_int, c_void_p]),
+    "xg_pad_rows": (c_int, [c_void_p, c_int64, c_int64, c_int64, c_int, c_void_p, c_int64, c_int, c_void_p]),
     "xg_sum3d": (c_int, [_VPP, _VPP, _I64P, c_int64, c_int, c_int, c_void_p]),
     "xg_rowsum_cat": (c_int, [_VPP, _VPP, _I64P, _I64P, _I64P, c_int64, c_int64, c_int64, c_void_p, c_int64, c_int, c_void_p]),
     "xg_gather_rows": (c_int, [_VPP, _I64P, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_int, c_void_p, c_int64,
@@ -166,7 +168,7 @@ def tc_status(reset: bool = True) -> int:
 
 
 # entry points that enqueue no kernel (queries and status reads)
-QUERY_ENTRY_POINTS = frozenset({"xg_version", "xg_device_arch_ok", "xg_last_error", "xg_tc_status", "xg_gemm_workspace_bytes",
+QUERY_ENTRY_POINTS = frozenset({"xg_version", "xg_device_arch_ok", "xg_last_error", "xg_tc_status", "xg_gemm_workspace_bytes", "xg_gemm_copy_bytes",
                                 "xg_gemm_static_scratch_bytes", "xg_gemm_f32x3_padded_k", "xg_gemm_cluster_plan",
                                 "xg_mlp2_supported", "xg_mlp3_supported", "xg_mlp_small_supported"})
 
