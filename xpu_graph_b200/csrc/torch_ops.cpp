@@ -18,6 +18,7 @@
 #include <torch/library.h>
 
 #include <atomic>
+#include <cmath>
 #include <cstdlib>
 #include <initializer_list>
 #include <string>
@@ -158,11 +159,12 @@ Tensor coef(const Tensor& w, at::ScalarType dtype) {
     return (w.scalar_type() == at::kFloat || w.scalar_type() == dtype ? w : w.to(at::kFloat)).contiguous();
 }
 
-// [B, H, S, D] output that keeps x's memory layout when x is a [B, S, H, D] buffer viewed with dims 1 and 2 swapped (so
-// that the transpose + reshape after attention stays a view); contiguous otherwise.
+// [B, H, S, D] output in the order of x's memory: a [B, S, H, D] buffer with dims 1 and 2 swapped when x's heads lie closer
+// together than its positions, as in projections and packed QKV buffers (so that the transpose + reshape after attention
+// stays a view); contiguous otherwise.
 Tensor empty_like_layout(const Tensor& x) {
     const int64_t B = x.size(0), H = x.size(1), S = x.size(2), D = x.size(3);
-    if (x.stride(3) == 1 && x.stride(1) == D && x.stride(2) == H * D && x.stride(0) == S * H * D && H > 1 && S > 1)
+    if (x.stride(3) == 1 && x.stride(1) < x.stride(2) && H > 1 && S > 1)
         return new_tensor({B, S, H, D}, x.scalar_type(), x).transpose(1, 2);
     return new_tensor({B, H, S, D}, x.scalar_type(), x);
 }
@@ -887,6 +889,87 @@ Tensor mul_sum_cat(at::TensorList lhs, at::TensorList rhs) {
     return sums.run();
 }
 
+// ---- whole graphs --------------------------------------------------------------------------------------------
+// The fused op sequences of fused_graphs.py as one operator each. With a Python frame, a module call, an operator dispatch
+// and several tensor views per kernel the host needed 90-105 us for the seven to nine launches of a small graph, more than
+// the kernels; from here a launch costs 4 us. The operators are for inference only: nothing below is seen by autograd.
+Tensor heads_view(const Tensor& rows, int64_t B, int64_t S, int64_t H, int64_t D, int64_t col0) {
+    const int64_t ld = rows.stride(0);
+    return rows.as_strided({B, H, S, D}, {S * ld, D, ld, 1}, rows.storage_offset() + col0);
+}
+Tensor heads_to_rows(const Tensor& a, int64_t rows, int64_t cols) { return a.transpose(1, 2).reshape({rows, cols}); }
+
+// LayerNorm | dense | attention | dense + residual | LayerNorm | dense + GELU | dense + residual.
+// params: (weight, bias) of ln1, qkv, proj, ln2, fc1, fc2
+Tensor encoder_block(const Tensor& x, const c10::List<optional<Tensor>>& params, double eps1, double eps2, int64_t heads) {
+    at::AutoDispatchBelowADInplaceOrView no_grad;
+    TORCH_CHECK_VALUE(x.dim() == 3 && params.size() == 12, "xg_sm100::encoder_block: x is [B, S, hidden], params are six (weight, bias) pairs");
+    auto weight = [&](int i) -> Tensor { return params.get(2 * i).value(); };
+    auto bias = [&](int i) -> optional<Tensor> { return params.get(2 * i + 1); };
+    const int64_t B = x.size(0), S = x.size(1), C = x.size(2), D = C / heads, T = B * S;
+    const Tensor x0 = x.reshape({T, C});
+    const Tensor qkv = dense(norm<false>(x0, {}, weight(0), or_none(bias(0)), eps1, false).first, weight(1), true, bias(1), std::nullopt, "none");
+    const Tensor a = sdpa(heads_view(qkv, B, S, heads, D, 0), heads_view(qkv, B, S, heads, D, C), heads_view(qkv, B, S, heads, D, 2 * C),
+                          std::nullopt, 1.0 / std::sqrt((double)D), false);
+    const Tensor x1 = dense(heads_to_rows(a, T, C), weight(2), true, bias(2), x0, "none");
+    const Tensor h = dense(norm<false>(x1, {}, weight(3), or_none(bias(3)), eps2, false).first, weight(4), true, bias(4), std::nullopt, "gelu");
+    return dense(h, weight(5), true, bias(5), x1, "none").view({B, S, C});
+}
+
+// RMSNorm | q, k with RoPE, v | causal attention | dense + residual | RMSNorm | SwiGLU | dense + residual.
+// weights: input norm, q, k, v, o, post norm, gate, up, down
+Tensor decoder_layer(const Tensor& x, const Tensor& cos, const Tensor& sin, at::TensorList w, double eps1, double eps2, int64_t heads,
+                     bool fuse_rope, bool fuse_swiglu) {
+    at::AutoDispatchBelowADInplaceOrView no_grad;
+    TORCH_CHECK_VALUE(x.dim() == 3 && w.size() == 9, "xg_sm100::decoder_layer: x is [B, S, hidden], nine weights");
+    const int64_t B = x.size(0), S = x.size(1), C = x.size(2), D = C / heads, T = B * S;
+    const Tensor x0 = x.reshape({T, C});
+    auto linear = [&](const Tensor& in, const Tensor& weight, const optional<Tensor>& residual) {
+        return dense(in, weight, true, std::nullopt, residual, "none");
+    };
+    const Tensor h = norm<true>(x0, {}, w[0], {}, eps1, false).first;
+    Tensor q, k;
+    if (fuse_rope) {
+        q = heads_view(dense_rope(h, w[1], cos, sin, S, D), B, S, heads, D, 0);
+        k = heads_view(dense_rope(h, w[2], cos, sin, S, D), B, S, heads, D, 0);
+    } else {
+        q = rope(heads_view(linear(h, w[1], std::nullopt), B, S, heads, D, 0), cos, sin);
+        k = rope(heads_view(linear(h, w[2], std::nullopt), B, S, heads, D, 0), cos, sin);
+    }
+    const Tensor v = heads_view(linear(h, w[3], std::nullopt), B, S, heads, D, 0);
+    const Tensor a = sdpa(q, k, v, std::nullopt, 1.0 / std::sqrt((double)D), true);
+    const Tensor x1 = linear(heads_to_rows(a, T, C), w[4], x0);
+    const Tensor h2 = norm<true>(x1, {}, w[5], {}, eps2, false).first;
+    const Tensor g = fuse_swiglu ? dense_swiglu(h2, w[6], w[7]) : swiglu(linear(h2, w[6], std::nullopt), linear(h2, w[7], std::nullopt));
+    return linear(g, w[8], x1).view({B, S, C});
+}
+
+// Slices of the dense features and the masked lookups side by side in one buffer, then the dense layers (ReLU).
+Tensor recommender(const Tensor& features, const Tensor& idx, const Tensor& mask, at::TensorList tables, at::IntArrayRef starts,
+                   at::IntArrayRef ends, at::TensorList weights, const c10::List<optional<Tensor>>& biases) {
+    at::AutoDispatchBelowADInplaceOrView no_grad;
+    TORCH_CHECK_VALUE(!weights.empty() && biases.size() == weights.size(), "xg_sm100::recommender: one bias entry per weight");
+    Tensor h = cat_lastdim({slice_cat(features, starts, ends, std::nullopt, false), gather_stack(tables, idx, mask, true)}, std::nullopt, false);
+    const int64_t M = h.size(0);
+    bool tower = h.scalar_type() == at::kFloat;
+    int64_t k = h.size(1);
+    for (const Tensor& w : weights) {
+        tower = tower && f32_on_tensor_cores(M, w.size(0), k);
+        k = w.size(0);
+    }
+    if (tower) {
+        c10::List<bool> trans;
+        std::string acts;
+        for (size_t i = 0; i < weights.size(); ++i) {
+            trans.push_back(true);
+            acts += i ? ",relu" : "relu";
+        }
+        return dense_tower(h, weights, trans, biases, acts);
+    }
+    for (size_t i = 0; i < weights.size(); ++i) h = dense(h, weights[i], true, biases.get(i), std::nullopt, "relu");
+    return h;
+}
+
 // ---- registration --------------------------------------------------------------------------------------------
 const char* const kSchemas[] = {
     "rms_norm(Tensor x, Tensor weight, float eps) -> Tensor",
@@ -920,10 +1003,19 @@ const char* const kSchemas[] = {
     "mul_sum_cat(Tensor[] lhs, Tensor[] rhs) -> Tensor",
 };
 
+const char* const kGraphSchemas[] = {
+    "encoder_block(Tensor x, Tensor?[] params, float eps1, float eps2, SymInt heads) -> Tensor",
+    "decoder_layer(Tensor x, Tensor cos, Tensor sin, Tensor[] weights, float eps1, float eps2, SymInt heads, bool fuse_rope, "
+    "bool fuse_swiglu) -> Tensor",
+    "recommender(Tensor features, Tensor idx, Tensor mask, Tensor[] tables, SymInt[] starts, SymInt[] ends, Tensor[] weights, "
+    "Tensor?[] biases) -> Tensor",
+};
+
 }  // namespace
 
 TORCH_LIBRARY(xg_sm100, m) {
     for (const char* s : kSchemas) m.def(s, {at::Tag::pt2_compliant_tag});
+    for (const char* s : kGraphSchemas) m.def(s, {at::Tag::pt2_compliant_tag});
 }
 
 TORCH_LIBRARY_IMPL(xg_sm100, CUDA, m) {
@@ -956,6 +1048,9 @@ TORCH_LIBRARY_IMPL(xg_sm100, CUDA, m) {
     XG_IMPL(slice_sum_cat);
     XG_IMPL(sum_cat);
     XG_IMPL(mul_sum_cat);
+    XG_IMPL(encoder_block);
+    XG_IMPL(decoder_layer);
+    XG_IMPL(recommender);
 #undef XG_IMPL
 }
 
@@ -964,6 +1059,10 @@ TORCH_LIBRARY_IMPL(xg_sm100, Autograd, m) {
     for (const char* s : kSchemas) {
         const std::string schema(s);
         m.impl(schema.substr(0, schema.find('(')).c_str(), torch::autograd::autogradNotImplementedFallback());
+    }
+    for (const char* s : kGraphSchemas) {
+        const std::string schema(s);
+        m.impl(schema.substr(0, schema.find('(')).c_str(), torch::CppFunction::makeFallthrough());
     }
 }
 

@@ -62,11 +62,11 @@ def _row_stride(x2: torch.Tensor) -> int:
 
 
 def _empty_like_layout(x: torch.Tensor) -> torch.Tensor:
-    """[B, H, S, D] output that keeps x's memory layout when x is a [B, S, H, D] buffer viewed with
-    dims 1 and 2 swapped (so that the transpose + reshape after attention stays a view); contiguous
+    """[B, H, S, D] output in the order of x's memory: a [B, S, H, D] buffer with dims 1 and 2 swapped when x's heads lie
+    closer together than its positions (so that the transpose + reshape after attention stays a view); contiguous
     otherwise."""
     B, H, S, D = x.shape
-    if x.stride(3) == 1 and x.stride(1) == D and x.stride(2) == H * D and x.stride(0) == S * H * D and H > 1 and S > 1:
+    if x.stride(3) == 1 and x.stride(1) < x.stride(2) and H > 1 and S > 1:
         return torch.empty((B, S, H, D), dtype=x.dtype, device=x.device).transpose(1, 2)
     return torch.empty((B, H, S, D), dtype=x.dtype, device=x.device)
 
@@ -615,6 +615,27 @@ mul_sum_cat = NativeOp("mul_sum_cat")
 def _(lhs, rhs):
     batch = max(max(a.shape[0], b.shape[0]) for a, b in zip(lhs, rhs))
     return torch.empty((batch, len(lhs) * lhs[0].shape[2]), dtype=lhs[0].dtype, device=lhs[0].device)
+
+
+# ---- whole graphs (fused_graphs.py) -----------------------------------------------------------------
+encoder_block = NativeOp("encoder_block")
+decoder_layer = NativeOp("decoder_layer")
+recommender = NativeOp("recommender")
+
+
+@encoder_block.register_fake
+def _(x, params, eps1, eps2, heads):
+    return torch.empty(x.shape, dtype=x.dtype, device=x.device)
+
+
+@decoder_layer.register_fake
+def _(x, cos, sin, weights, eps1, eps2, heads, fuse_rope, fuse_swiglu):
+    return torch.empty(x.shape, dtype=x.dtype, device=x.device)
+
+
+@recommender.register_fake
+def _(features, idx, mask, tables, starts, ends, weights, biases):
+    return torch.empty((features.shape[0], weights[-1].shape[0]), dtype=features.dtype, device=features.device)
 
 
 OP_NAMES = tuple(name for name, op in list(globals().items()) if isinstance(op, (NativeOp, torch.library.CustomOpDef)))
