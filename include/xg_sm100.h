@@ -314,6 +314,19 @@ int xg_sdpa_fwd(const void* q, const void* k, const void* v, const void* mask, v
                 const int64_t* k_strides3, const int64_t* v_strides3, const int64_t* o_strides3,
                 const int64_t* mask_strides4, float scale, int causal, int dtype, void* stream);
 
+/*
+ * Same with a mask in either form - mask_bool != 0: bytes, zero hides the key (what a boolean attn_mask means); 0: additive, in
+ * the tensors' dtype - and with scratch memory: where there are few query tiles and many keys (decoding steps), the 16-bit
+ * kernel shares a tile's keys out over several CTAs, which leave unnormalised fp32 parts in `workspace`, and a second pass
+ * adds them. xg_sdpa_workspace_bytes: what a shape would like (0: not split); less or none only means no split.
+ */
+int xg_sdpa_fwd_ws(const void* q, const void* k, const void* v, const void* mask, void* out, int64_t B,
+                   int64_t H, int64_t Sq, int64_t Skv, int64_t D, const int64_t* q_strides3,
+                   const int64_t* k_strides3, const int64_t* v_strides3, const int64_t* o_strides3,
+                   const int64_t* mask_strides4, float scale, int causal, int dtype, int mask_bool, void* workspace,
+                   int64_t workspace_bytes, void* stream);
+int64_t xg_sdpa_workspace_bytes(int64_t B, int64_t H, int64_t Sq, int64_t Skv, int64_t D, int dtype);
+
 /* ---- copy fusions (bit-exact) ---------------------------------------------------------- */
 
 /*

@@ -185,3 +185,56 @@ def test_config4_prefill_shape(cuda_device):
         assert_parity(got[b:b + 1, h:h + 1], want, f"prefill pair ({b},{h})")
     ones = SDPAModule()(q, k, torch.ones_like(v), None, None, True)
     assert (ones.float() - 1.0).abs().max().item() < 1e-2
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("B,H,Sq,Skv,D", [(2, 3, 64, 64, 64), (3, 2, 130, 65, 128), (2, 2, 1, 700, 64), (1, 3, 33, 127, 128), (70, 1, 20, 90, 64),
+                                          (2, 160, 129, 200, 64)])
+def test_boolean_key_masks(cuda_device, B, H, Sq, Skv, D, dtype, causal):
+    """Boolean masks that hide the same keys from every query of a sequence (padding): lengths at the edges of a 64-key
+    block, holes inside a block, whole blocks hidden at the front, more batch entries than the kernel keeps lengths of."""
+    q, k, v = _qkv(B, H, Sq, Skv, D, dtype, 60)
+    g = torch.Generator().manual_seed(61)
+    mask = torch.zeros(B, 1, 1, Skv, dtype=torch.bool)
+    for b in range(B):
+        n = [Skv, max(1, Skv // 64 * 64), min(Skv, 65), int(torch.randint(1, Skv + 1, (1,), generator=g))][b % 4]
+        mask[b, :, :, :n] = torch.rand(1, 1, n, generator=g) < 0.8
+        if not causal and b % 3 == 2 and n > 64:
+            mask[b, :, :, :64] = False
+        mask[b, :, :, 0 if causal else n - 1] = True  # every row sees a key
+    got = _run(cuda_device, q, k, v, mask, None, causal)
+    full = mask.expand(B, 1, Sq, Skv)
+    if causal:  # torch's own function takes a mask or the causal flag, not both
+        full = full & torch.ones(Sq, Skv, dtype=torch.bool).tril()
+    want = ref_ops.sdpa_math(q.double(), k.double(), v.double(), torch.zeros(full.shape, dtype=torch.double).masked_fill(~full, float("-inf")),
+                             None, False).to(dtype)
+    assert_parity(got, want, f"key mask {B}x{H}x{Sq}x{Skv}x{D} causal={causal} {dtype}")
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("B,H,Sq,Skv,D,mask_kind", [(1, 2, 1, 768, 128, "none"), (2, 3, 5, 1000, 64, "keys"), (1, 1, 300, 2049, 64, "none"),
+                                                    (1, 4, 128, 832, 128, "keys"), (1, 2, 17, 900, 128, "add"), (3, 5, 129, 1024, 64, "none")])
+def test_flash_tc_split_keys(cuda_device, B, H, Sq, Skv, D, mask_kind, causal):
+    """Few query tiles against many keys: a tile's keys are shared out over several CTAs and the parts added afterwards,
+    also where the causal limit or the mask leaves a part without keys."""
+    from xpu_graph_b200 import lib
+
+    assert lib.load().xg_sdpa_workspace_bytes(B, H, Sq, Skv, D, lib.XG_F16) > 0, "shape expected to be split"
+    q, k, v = _qkv(B, H, Sq, Skv, D, torch.float16, 62)
+    g = torch.Generator().manual_seed(63)
+    mask = None
+    if mask_kind == "keys":
+        mask = (torch.arange(Skv) < torch.randint(1, Skv // 2, (B, 1, 1, 1), generator=g))
+    elif mask_kind == "add":
+        mask = torch.randn(1, 1, Sq, Skv, generator=g).to(torch.float16)
+    got = _run(cuda_device, q, k, v, mask, None, causal)
+    add = torch.zeros(B, 1, Sq, Skv, dtype=torch.double)
+    if mask_kind == "keys":
+        add = add.masked_fill(~mask, float("-inf"))
+    elif mask_kind == "add":
+        add = add + mask.double()
+    if causal:
+        add = add.masked_fill(~torch.ones(Sq, Skv, dtype=torch.bool).tril(), float("-inf"))
+    want = ref_ops.sdpa_math(q.double(), k.double(), v.double(), add, None, False).to(torch.float16)
+    assert_parity(got, want, f"split keys {B}x{H}x{Sq}x{Skv}x{D} {mask_kind} causal={causal}")

@@ -9,8 +9,8 @@
 //   packed 16-bit pairs over the first half of the same score buffer, so a block's softmax never waits
 //   for the previous block's P V. O accumulates in TMEM and is rescaled lazily.
 //   Causal tiles beyond the diagonal are skipped.
-// Everything else runs in true fp32 on SIMT kernels: a shared-memory tiled kernel (head dim 32 / 64 / 128, no additive
-// mask) and a warp-per-query kernel (masks, other head dims).
+// Everything else runs in true fp32 on SIMT kernels: a shared-memory tiled kernel (head dim 32 / 64 / 128) and a
+// warp-per-query kernel (other head dims).
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 
@@ -39,6 +39,13 @@ struct SdpaParams {
     int64_t m_sb, m_sh, m_sq, m_sk;
     float scale;
     int causal;
+    int mask_kind;  // MaskKind
+};
+
+enum MaskKind : int {
+    kMaskNone = 0,
+    kMaskAdd = 1,   // added to the scaled scores, in the tensors' dtype
+    kMaskBool = 2,  // bytes: zero hides the key
 };
 
 // ---------------------------------------------------------------------------------------
@@ -50,17 +57,21 @@ struct SdpaParams {
 struct FlashParams {
     const void* mask;
     void* out;
+    float* partial;  // split keys: [tile][split][FM][D] unnormalised outputs, then [tile][split][FM] (maximum, row sum) pairs
     int64_t o_sb, o_sh, o_ss;
     int64_t m_sb, m_sh, m_sq, m_sk;
     int B, H, Sq, Skv;
     float scale;
-    int causal;
+    int16_t causal, mask_kind;
+    int16_t single;  // one tile per CTA (the tiles fit the chip at once) instead of a list of tile pairs
+    int16_t splits;  // CTAs that share a tile's keys (single only)
 };
 static_assert(sizeof(FlashParams) <= 128, "flash kernel parameter block must stay within 512 bytes");
 
 constexpr int FM = 128;  // query rows per CTA
 constexpr int FN = 64;   // keys per block
 constexpr int kFlashThreads = 192;
+constexpr int kFlashMaxB = 64;  // batch entries whose number of key blocks is kept in shared memory
 constexpr float kRescaleThreshold = 8.0f;  // log2 units: the running max may lag by up to 2^8
 
 template <int D>
@@ -71,7 +82,7 @@ struct FlashCfg {
     // Two CTAs share an SM, and the window carries no alignment slack: the kernel checks that the
     // dynamic shared-memory window starts on a 1024-byte boundary and reports if it does not.
     static constexpr int O_STAGE_BYTES = 4 * 32 * 128;  // a 32-row, 64-column slab per softmax warp
-    static constexpr int SMEM_BYTES = Q_BYTES + 4 * KV_BYTES + O_STAGE_BYTES + 256;  // tiles + staging + barriers
+    static constexpr int SMEM_BYTES = Q_BYTES + 4 * KV_BYTES + O_STAGE_BYTES + 256 + 4 * kFlashMaxB;  // tiles + staging + barriers + key blocks
     static_assert(2 * (SMEM_BYTES + 1024) <= 233472, "two CTAs must fit in one SM's shared memory");
     // S0 [0,64) S1 [64,128) O [128, 128+D); P of block n overlays columns [0,32) of score buffer n & 1
     static constexpr int TMEM_COLS = 256;
@@ -84,9 +95,10 @@ struct FlashCfg {
 // add up to the same number of key blocks, so a CTA that takes every gridDim.x-th tile gets an even share
 // (the host makes gridDim.x even).
 struct FlashTile {
-    int b, h, q0, nblk;
+    int b, h, q0;
+    int j0, nblk;  // key blocks [j0, j0 + nblk)
 };
-__device__ __forceinline__ FlashTile flash_tile(const FlashParams& p, int b, int h, int k, int q_tiles) {
+__device__ __forceinline__ FlashTile flash_tile(const FlashParams& p, const volatile int* kv_blocks, int b, int h, int k, int q_tiles) {
     const int qt = p.causal ? ((k & 1) ? (k >> 1) : (q_tiles - 1 - (k >> 1))) : k;
     FlashTile t;
     t.h = h;
@@ -96,6 +108,13 @@ __device__ __forceinline__ FlashTile flash_tile(const FlashParams& p, int b, int
     if (p.causal) {
         const int lim = (t.q0 + FM - 1) / FN + 1;  // last block that any row of this tile can see
         if (lim < t.nblk) t.nblk = lim;
+    }
+    if (kv_blocks != nullptr && kv_blocks[b] < t.nblk) t.nblk = kv_blocks[b];
+    t.j0 = 0;
+    if (p.splits > 1) {
+        const int sp = (int)blockIdx.x % p.splits, n = t.nblk;
+        t.j0 = n * sp / p.splits;
+        t.nblk = n * (sp + 1) / p.splits - t.j0;
     }
     return t;
 }
@@ -125,7 +144,7 @@ __device__ __forceinline__ FlashStride flash_stride(const FlashParams& p, int q_
 }
 __device__ __forceinline__ FlashCursor flash_cursor(const FlashParams& p, int q_tiles) {
     FlashCursor c;
-    c.L = 2 * (int)blockIdx.x;
+    c.L = p.single ? (int)blockIdx.x / p.splits : 2 * (int)blockIdx.x;
     const int bh = c.L / q_tiles;
     c.k = c.L - bh * q_tiles;
     c.b = bh / p.H;
@@ -134,8 +153,9 @@ __device__ __forceinline__ FlashCursor flash_cursor(const FlashParams& p, int q_
 }
 // i-th tile of this CTA (i = 0, 1, 2, ... in order). Returns 0 with the tile in t, -1 when the CTA is done, -2 for
 // the missing second half of a trailing odd pair.
-__device__ __forceinline__ int flash_next(FlashCursor& c, const volatile FlashStride* stride, int i, int num_tiles, int q_tiles,
-                                          const FlashParams& p, FlashTile& t) {
+__device__ __forceinline__ int flash_next(FlashCursor& c, const volatile FlashStride* stride, const volatile int* kv_blocks, int i,
+                                          int num_tiles, int q_tiles, const FlashParams& p, FlashTile& t) {
+    if (p.single && i > 0) return -1;
     if ((i & 1) == 0) {
         if (i > 0) {
             c.L += 2 * (int)gridDim.x;
@@ -145,20 +165,25 @@ __device__ __forceinline__ int flash_next(FlashCursor& c, const volatile FlashSt
             flash_carry(c.b, c.h, c.k, q_tiles, p.H);  // k < 2 q_tiles and h <= 2 H - 1 here: one carry each is enough
         }
         if (c.L >= num_tiles) return -1;
-        t = flash_tile(p, c.b, c.h, c.k, q_tiles);
+        t = flash_tile(p, kv_blocks, c.b, c.h, c.k, q_tiles);
         return 0;
     }
     if (c.L + 1 >= num_tiles) return -2;
     int b = c.b, h = c.h, k = c.k + 1;
     flash_carry(b, h, k, q_tiles, p.H);
-    t = flash_tile(p, b, h, k, q_tiles);
+    t = flash_tile(p, kv_blocks, b, h, k, q_tiles);
     return 0;
 }
 
-// MASKED: the kernel carries the general masking code (additive mask, key count that is not a multiple of the block,
-// non-positive scale). The common case is compiled without it: the code of a tile boundary runs once per tile, its
-// instruction fetches miss the instruction caches, and a smaller kernel keeps more of it resident.
-template <typename T, int D, bool MASKED>
+// MASK: what the kernel can hide beside the causal diagonal. 0: nothing. 1: keys, the same ones for every query row of a head
+// (a key count that is not a multiple of the block; a boolean padding mask): two 32-bit words per block, which a warp
+// gathers with a ballot while the previous block is in work, and blocks behind the batch entry's last valid key are not
+// visited at all. 2: the general code (additive or per-row masks, non-positive scale), which reads a mask element per
+// score. (4 x 32 x 500 x 500, head dim 64, padding: 74 us with the general code, see launch_flash_tc for the others.) The
+// common cases are compiled without it: the code of a tile boundary runs once per tile, its instruction fetches miss the
+// instruction caches, and a smaller kernel keeps more of it resident.
+// SPLIT: a tile's keys are shared out over several CTAs; each leaves its unnormalised part in scratch memory.
+template <typename T, int D, int MASK, bool SPLIT>
 __global__ void __launch_bounds__(kFlashThreads, 2)
 flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUtensorMap tmk,
                 const __grid_constant__ CUtensorMap tmv, const FlashParams p) {
@@ -183,6 +208,9 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     volatile FlashStride* stride = reinterpret_cast<volatile FlashStride*>(tmem_slot + 2);
+    int* kv_blocks_s = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(bars) + 256);
+    const bool trim = MASK == 1 && p.mask != nullptr && (p.m_sh == 0 || p.H == 1) && p.B <= kFlashMaxB && (int64_t)p.B * p.Skv <= 65536;
+    const volatile int* kv_blocks = trim ? kv_blocks_s : nullptr;
 
     if ((ptx::smem_u32(smem) & 1023u) != 0) {  // uniform over the CTA: the swizzled tiles need this alignment
         pdl_sync();
@@ -225,6 +253,20 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_sync();  // the tensor memory is held
+    if (MASK == 1 && trim) {  // blocks up to each batch entry's last valid key
+        for (int b = threadIdx.x; b < p.B; b += kFlashThreads) kv_blocks_s[b] = 0;
+        __syncthreads();
+        const uint8_t* m = reinterpret_cast<const uint8_t*>(p.mask);
+        for (int b = 0; b < p.B; ++b) {
+            int last = -1;
+#pragma unroll 8
+            for (int c = threadIdx.x; c < p.Skv; c += kFlashThreads)
+                if (m[b * p.m_sb + c * p.m_sk]) last = c;
+            last = __reduce_max_sync(0xffffffffu, last);
+            if ((threadIdx.x & 31) == 0 && last >= 0) atomicMax(&kv_blocks_s[b], last / FN + 1);
+        }
+        __syncthreads();
+    }
     constexpr int fmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
 
     if (warp == 0) {
@@ -239,7 +281,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
             FlashCursor cur = flash_cursor(p, q_tiles);
             for (int i = 0; ok; ++i) {
                 FlashTile t;
-                const int tile_state = flash_next(cur, stride, i, num_tiles, q_tiles, p, t);
+                const int tile_state = flash_next(cur, stride, kv_blocks, i, num_tiles, q_tiles, p, t);
                 if (tile_state == -1) break;
                 if (tile_state == -2) continue;
                 const uint32_t tile_par = tile_n++ & 1u;
@@ -255,12 +297,12 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
                     ptx::mbar_arrive_expect_tx(&k_full[s], Cfg::KV_BYTES);
 #pragma unroll
                     for (int db = 0; db < Cfg::DB; ++db)
-                        ptx::tma_load_4d(k_s + s * Cfg::KV_BYTES + db * (FN * 128), &tmk, &k_full[s], db * 64, j * FN, t.h, t.b);
+                        ptx::tma_load_4d(k_s + s * Cfg::KV_BYTES + db * (FN * 128), &tmk, &k_full[s], db * 64, (t.j0 + j) * FN, t.h, t.b);
                     if (!ptx::mbar_wait_bounded(&v_empty[s], ph ^ 1u, abort_flag)) { ok = false; break; }
                     ptx::mbar_arrive_expect_tx(&v_full[s], Cfg::KV_BYTES);
 #pragma unroll
                     for (int db = 0; db < Cfg::DB; ++db)
-                        ptx::tma_load_4d(v_s + s * Cfg::KV_BYTES + db * (FN * 128), &tmv, &v_full[s], db * 64, j * FN, t.h, t.b);
+                        ptx::tma_load_4d(v_s + s * Cfg::KV_BYTES + db * (FN * 128), &tmv, &v_full[s], db * 64, (t.j0 + j) * FN, t.h, t.b);
                 }
             }
             if (!ok) {
@@ -305,7 +347,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
             };
             for (int i = 0; ok; ++i) {
                 FlashTile t;
-                const int tile_state = flash_next(cur, stride, i, num_tiles, q_tiles, p, t);
+                const int tile_state = flash_next(cur, stride, kv_blocks, i, num_tiles, q_tiles, p, t);
                 if (tile_state == -1) break;
                 if (tile_state == -2) continue;
                 if (!ptx::mbar_wait_bounded(q_full, tile_n++ & 1u, abort_flag)) { ok = false; break; }
@@ -361,14 +403,24 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
 
         for (int i = 0; ok; ++i) {
             FlashTile t;
-            const int tile_state = flash_next(cur, stride, i, num_tiles, q_tiles, p, t);
+            const int tile_state = flash_next(cur, stride, kv_blocks, i, num_tiles, q_tiles, p, t);
             if (tile_state == -1) break;
             if (tile_state == -2) continue;
             const int q0 = t.q0, nblk = t.nblk;
             const int row = q0 + r_in_tile;
-            const T* mrow = nullptr;
-            if (MASKED && p.mask != nullptr && row < p.Sq)
-                mrow = reinterpret_cast<const T*>(p.mask) + (int64_t)t.b * p.m_sb + (int64_t)t.h * p.m_sh + (int64_t)row * p.m_sq;
+            const int64_t m_off = (int64_t)t.b * p.m_sb + (int64_t)t.h * p.m_sh + (MASK == 2 ? (int64_t)row * p.m_sq : 0);
+            const bool has_mask = MASK != 0 && p.mask != nullptr && (MASK == 1 || row < p.Sq);
+            const bool idle = q0 + quad * 32 >= p.Sq;  // none of this warp's rows exists: only the hand-shakes are kept up
+            // MASK == 1: keys lane and lane + 32 of a block
+            auto key_ok = [&](int col) {
+                return col < skv && (!has_mask || reinterpret_cast<const uint8_t*>(p.mask)[m_off + (int64_t)col * p.m_sk] != 0);
+            };
+            bool key0 = true, key1 = true;
+            if (MASK == 1 && nblk > 0) {
+                const int first = has_mask ? t.j0 : t.j0 + nblk - 1;
+                key0 = key_ok(first * FN + lane);
+                key1 = key_ok(first * FN + 32 + lane);
+            }
             float m_run = -INFINITY, l_run = 0.f;  // running maximum (log2 domain, scaled) and row sum
 
             for (int j = 0; j < nblk; ++j, ++n) {
@@ -377,13 +429,27 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
                 if (!__all_sync(0xffffffffu, ptx::mbar_wait_bounded(&s_full[sb], (n >> 1) & 1u, abort_flag))) { ok = false; break; }
                 ptx::tc_fence_after();
                 const uint32_t s_taddr = tmem_base + lane_field + (uint32_t)(sb * FN);
-                const int col_base = j * FN;
+                const int col_base = (t.j0 + j) * FN;
+                if (idle) {  // (whatever the score buffer holds is multiplied into output rows that nobody reads)
+                    ptx::tc_fence_before();
+                    ptx::mbar_arrive(&p_full[sb]);
+                    continue;
+                }
+                uint32_t keys0 = 0xffffffffu, keys1 = 0xffffffffu;
+                if (MASK == 1 && (has_mask || col_base + FN > skv)) {  // (without a mask only the last block lacks keys)
+                    keys0 = __ballot_sync(0xffffffffu, key0);
+                    keys1 = __ballot_sync(0xffffffffu, key1);
+                    if (has_mask && j + 1 < nblk) {  // the next block's, in flight meanwhile
+                        key0 = key_ok(col_base + FN + lane);
+                        key1 = key_ok(col_base + FN + 32 + lane);
+                    }
+                }
                 // A block needs the general masking code when it carries an additive mask, crosses the end of the
                 // keys or has a non-positive scale. A block that is only cut by the causal diagonal is classified per
                 // warp (a warp owns 32 consecutive query rows): all keys visible, some, or none.
-                const bool general_mask = MASKED && ((p.mask != nullptr) || (col_base + FN > skv) || !(sl2 > 0.f));
+                const bool general_mask = MASK == 2 && ((p.mask != nullptr) || (col_base + FN > skv) || !(sl2 > 0.f));
                 const int warp_row0 = q0 + quad * 32;
-                const bool diag_none = !general_mask && p.causal && (col_base > warp_row0 + 31);
+                const bool diag_none = (!general_mask && p.causal && (col_base > warp_row0 + 31)) || (MASK == 1 && (keys0 | keys1) == 0);
                 const bool diag_some = !general_mask && p.causal && !diag_none && (col_base + FN - 1 > warp_row0);
                 if (diag_none) {
                     // every key of the block lies beyond the diagonal for these rows: the probabilities are zero and
@@ -416,13 +482,26 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
                     for (int i = 0; i < FN; ++i)
                         if (i > last_visible) sc[i] = -INFINITY;
                 }
-                if (MASKED && general_mask) {  // uniform over the CTA; scores go to the log2 domain here
+                if (MASK == 1 && (keys0 & keys1) != 0xffffffffu) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) {
+                        if (!((keys0 >> i) & 1u)) sc[i] = -INFINITY;
+                        if (!((keys1 >> i) & 1u)) sc[32 + i] = -INFINITY;
+                    }
+                }
+                if (MASK == 2 && general_mask) {  // uniform over the CTA; scores go to the log2 domain here
+                    const bool additive = p.mask_kind == kMaskAdd;
 #pragma unroll
                     for (int i = 0; i < FN; ++i) {
                         const int col = col_base + i;
+                        bool hidden = col >= skv || (p.causal && col > row);
                         sc[i] *= sl2;
-                        if (mrow != nullptr && col < skv) sc[i] += Cvt<T>::to_f(mrow[(int64_t)col * p.m_sk]) * kLog2e;
-                        if (col >= skv || (p.causal && col > row)) sc[i] = -INFINITY;
+                        if (has_mask && col < skv) {
+                            const int64_t at = m_off + (int64_t)col * p.m_sk;
+                            if (additive) sc[i] += Cvt<T>::to_f(reinterpret_cast<const T*>(p.mask)[at]) * kLog2e;
+                            else hidden = hidden || reinterpret_cast<const uint8_t*>(p.mask)[at] == 0;
+                        }
+                        if (hidden) sc[i] = -INFINITY;
                     }
                     mul = 1.f;
                 }
@@ -508,6 +587,36 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
                 ++tile_n;
             }
             ptx::tc_fence_after();
+            if (SPLIT) {
+                const int64_t unit_row = (int64_t)blockIdx.x * FM + r_in_tile;
+                float* po = p.partial + unit_row * D;
+#pragma unroll 1
+                for (int c = 0; c < D / 32 && !idle; ++c) {
+                    uint32_t o[32];
+                    if (nblk > 0) {
+                        ptx::tmem_ld_32x32(tmem_base + lane_field + Cfg::O_COL + (uint32_t)(c * 32), o);
+                        ptx::tmem_ld_wait();
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) o[i] = 0u;
+                    }
+                    if (row < p.Sq) {
+#pragma unroll
+                        for (int i = 0; i < 32; i += 4)
+                            *reinterpret_cast<uint4*>(po + c * 32 + i) = make_uint4(o[i], o[i + 1], o[i + 2], o[i + 3]);
+                    }
+                }
+                if (row < p.Sq) {
+                    float2* ml = reinterpret_cast<float2*>(p.partial + (int64_t)gridDim.x * FM * D);
+                    ml[unit_row] = make_float2(m_run, l_run);
+                }
+                ptx::tc_fence_before();
+                continue;
+            }
+            if (idle) {
+                ptx::tc_fence_before();
+                continue;
+            }
             const float inv_l = 1.0f / l_run;
             // A thread holds one output row, so storing from registers would touch 32 different lines per
             // instruction. The rows go through a 4 KiB slab of shared memory per warp instead (64 head-dim columns
@@ -566,8 +675,58 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
     }
 }
 
+// The parts of a tile whose keys were split: out = sum_s 2^(m_s - m) O_s / sum_s 2^(m_s - m) l_s. A warp per query row.
 template <typename T, int D>
-int launch_flash_tc(const SdpaParams& p, cudaStream_t st) {
+__global__ void __launch_bounds__(128) flash_combine_kernel(const FlashParams p, int q_tiles) {
+    pdl_sync();
+    const int lane = threadIdx.x & 31;
+    const int64_t row_id = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (row_id >= (int64_t)p.B * p.H * p.Sq) return;
+    const int bh = (int)(row_id / p.Sq), row = (int)(row_id - (int64_t)bh * p.Sq);
+    const int b = bh / p.H, h = bh - b * p.H;
+    // the position of this query tile in the list of its head (see flash_tile)
+    const int qt = row / FM;
+    const int k = p.causal ? (2 * qt + 1 < q_tiles ? 2 * qt + 1 : 2 * (q_tiles - 1 - qt)) : qt;
+    const int64_t units = (int64_t)p.B * p.H * q_tiles * p.splits;
+    const int64_t row0 = (((int64_t)bh * q_tiles + k) * p.splits) * FM + (row - qt * FM);
+    const float2* ml = reinterpret_cast<const float2*>(p.partial + units * FM * D);
+    float m = -INFINITY;
+    for (int s = 0; s < p.splits; ++s) m = fmaxf(m, ml[row0 + (int64_t)s * FM].x);
+    const float m_use = m == -INFINITY ? 0.f : m;
+    float l = 0.f, o[D / 32];
+#pragma unroll
+    for (int i = 0; i < D / 32; ++i) o[i] = 0.f;
+#pragma unroll 4
+    for (int s = 0; s < p.splits; ++s) {
+        const int64_t at = row0 + (int64_t)s * FM;
+        const float2 part = ml[at];
+        const float w = ptx::ex2_approx(part.x - m_use);
+        l += w * part.y;
+        using Piece = typename std::conditional<D == 128, float4, float2>::type;
+        const Piece v = *reinterpret_cast<const Piece*>(p.partial + at * D + lane * (D / 32));
+        const float* e = reinterpret_cast<const float*>(&v);
+#pragma unroll
+        for (int i = 0; i < D / 32; ++i) o[i] += w * e[i];
+    }
+    const float inv_l = 1.0f / l;
+    T* out = reinterpret_cast<T*>(p.out) + (int64_t)b * p.o_sb + (int64_t)h * p.o_sh + (int64_t)row * p.o_ss + lane * (D / 32);
+#pragma unroll
+    for (int i = 0; i < D / 32; i += 2) *reinterpret_cast<uint32_t*>(out + i) = ptx::pack2<T>(o[i] * inv_l, o[i + 1] * inv_l);
+}
+
+// How many CTAs share a query tile's keys. Splitting pays where the tiles leave at least half of the chip's two CTAs per SM
+// idle and a tile walks a dozen key blocks: a block costs a CTA about 0.8 us of latency (scores, softmax, hand-over), the
+// second launch that adds the parts about 3.5 us.
+int flash_splits(int64_t tiles, int64_t Skv) {
+    const int64_t resident = 2LL * num_sms(), nblk = (Skv + FN - 1) / FN;
+    if (tiles <= 0 || 2 * tiles > resident || nblk < 12) return 1;
+    int64_t s = resident / tiles;
+    if (s > nblk / 4) s = nblk / 4;  // four blocks at least
+    return (int)(s < 1 ? 1 : (s > 32 ? 32 : s));
+}
+
+template <typename T, int D>
+int launch_flash_tc(const SdpaParams& p, void* workspace, int64_t ws_bytes, cudaStream_t st) {
     using Cfg = FlashCfg<D>;
     constexpr bool is_bf16 = std::is_same<T, __nv_bfloat16>::value;
     CUtensorMap tq, tk, tv;
@@ -582,18 +741,40 @@ int launch_flash_tc(const SdpaParams& p, cudaStream_t st) {
     fp.m_sb = p.m_sb; fp.m_sh = p.m_sh; fp.m_sq = p.m_sq; fp.m_sk = p.m_sk;
     fp.B = (int)p.B; fp.H = (int)p.H; fp.Sq = (int)p.Sq; fp.Skv = (int)p.Skv;  // the caller keeps these below 2^31
     fp.scale = p.scale;
-    fp.causal = p.causal;
-    const bool masked = p.mask != nullptr || p.Skv % FN != 0 || !(p.scale > 0.f);
-    auto kern = masked ? flash_tc_kernel<T, D, true> : flash_tc_kernel<T, D, false>;
-    static std::atomic<uint64_t> reserved[2];
-    if (!reserve_smem(kern, Cfg::SMEM_BYTES, reserved[masked])) return fail(XG_ERR_LAUNCH, "xg_sdpa_fwd: cannot reserve shared memory");
-    const int64_t tiles = p.B * p.H * ((p.Sq + FM - 1) / FM);
+    fp.causal = (int16_t)p.causal;
+    fp.mask_kind = (int16_t)p.mask_kind;
+    const int q_tiles = (int)((p.Sq + FM - 1) / FM);
+    const int64_t tiles = p.B * p.H * q_tiles;
     if (tiles > 0x7fffffffLL) return fail(XG_ERR_TOO_LARGE, "xg_sdpa_fwd: too many tiles");
     const int64_t resident = 2LL * num_sms();  // persistent CTAs, two per SM
-    const int64_t pairs = (tiles + 1) / 2;      // a CTA takes tiles in neighbouring (heavy, light) pairs
-    const unsigned grid = (unsigned)(pairs < resident ? pairs : resident);
-    launch_with({.early = grid == resident}, kern, grid, kFlashThreads, Cfg::SMEM_BYTES, st, tq, tk, tv, fp);
-    return check_launch("xg_sdpa_fwd");
+    fp.single = tiles <= resident;
+    int splits = fp.single ? flash_splits(tiles, p.Skv) : 1;
+    if (splits > 1 && (!workspace || !aligned16(workspace) || ws_bytes < tiles * splits * FM * (D + 2) * 4)) splits = 1;
+    fp.splits = (int16_t)splits;
+    fp.partial = reinterpret_cast<float*>(workspace);
+    // tiles in a list: a CTA takes neighbouring (heavy, light) pairs
+    const int64_t pairs = (tiles + 1) / 2;
+    const unsigned grid = (unsigned)(fp.single ? tiles * splits : (pairs < resident ? pairs : resident));
+    const bool rows_differ = p.mask != nullptr && (p.mask_kind == kMaskAdd || (p.m_sq != 0 && p.Sq > 1));
+    const int mask = rows_differ || !(p.scale > 0.f) ? 2 : (p.mask != nullptr || p.Skv % FN != 0 ? 1 : 0);
+    static std::atomic<uint64_t> reserved[6];
+    auto run = [&](auto kern, int slot) {
+        if (!reserve_smem(kern, Cfg::SMEM_BYTES, reserved[slot])) return fail(XG_ERR_LAUNCH, "xg_sdpa_fwd: cannot reserve shared memory");
+        launch_with({.early = grid == resident && !fp.single}, kern, grid, kFlashThreads, Cfg::SMEM_BYTES, st, tq, tk, tv, fp);
+        return check_launch("xg_sdpa_fwd");
+    };
+    if (splits == 1) {
+        switch (mask) {
+            case 0: return run(flash_tc_kernel<T, D, 0, false>, 0);
+            case 1: return run(flash_tc_kernel<T, D, 1, false>, 1);
+            default: return run(flash_tc_kernel<T, D, 2, false>, 2);
+        }
+    }
+    const int rc = mask == 0 ? run(flash_tc_kernel<T, D, 0, true>, 3)
+                             : (mask == 1 ? run(flash_tc_kernel<T, D, 1, true>, 4) : run(flash_tc_kernel<T, D, 2, true>, 5));
+    if (rc != XG_OK) return rc;
+    launch(flash_combine_kernel<T, D>, (unsigned)((p.B * p.H * p.Sq + 3) / 4), 128, 0, st, fp, q_tiles);
+    return check_launch("xg_sdpa_fwd (combine)");
 }
 
 // ---------------------------------------------------------------------------------------
@@ -618,7 +799,7 @@ __global__ void __launch_bounds__(kSimtWarps * 32) sdpa_simt_kernel(const SdpaPa
     const T* qrow = reinterpret_cast<const T*>(p.q) + b * p.q_sb + h * p.q_sh + i * p.q_ss;
     const T* kbase = reinterpret_cast<const T*>(p.k) + b * p.k_sb + h * p.k_sh;
     const T* vbase = reinterpret_cast<const T*>(p.v) + b * p.v_sb + h * p.v_sh;
-    const T* mrow = p.mask ? reinterpret_cast<const T*>(p.mask) + b * p.m_sb + h * p.m_sh + i * p.m_sq : nullptr;
+    const int64_t m_off = b * p.m_sb + h * p.m_sh + i * p.m_sq;
     const int nu = (D + 31) / 32;  // head-dim elements (and output columns) per lane
     float qreg[kSimtMaxD / 32];
 #pragma unroll
@@ -663,7 +844,8 @@ __global__ void __launch_bounds__(kSimtWarps * 32) sdpa_simt_kernel(const SdpaPa
                 if (lane == t0 + e) s = part[e] * p.scale;
         }
         if (j < kv_end) {
-            if (mrow) s += Cvt<T>::to_f(mrow[j * p.m_sk]);
+            if (p.mask_kind == kMaskAdd) s += Cvt<T>::to_f(reinterpret_cast<const T*>(p.mask)[m_off + j * p.m_sk]);
+            else if (p.mask_kind == kMaskBool && reinterpret_cast<const uint8_t*>(p.mask)[m_off + j * p.m_sk] == 0) s = -INFINITY;
         } else {
             s = -INFINITY;
         }
@@ -705,7 +887,7 @@ __global__ void __launch_bounds__(kSimtWarps * 32) sdpa_simt_kernel(const SdpaPa
 }
 
 // ---------------------------------------------------------------------------------------
-// Tiled SIMT kernel: true fp32 arithmetic for head dims 32 / 64 / 128 without an additive mask (the encoder block's
+// Tiled SIMT kernel: true fp32 arithmetic for head dims 32 / 64 / 128 (the encoder block's
 // attention). A CTA owns 16 query rows of one (batch, head): 4 warps x 4 rows. Keys and values pass through shared
 // memory in chunks of 128 (each element is read from global memory once per CTA, coalesced, instead of once per query
 // row): lane t holds the scores of keys t, t + 32, t + 64, t + 96 for the warp's four rows (64 FMAs per eight 16-byte
@@ -723,7 +905,7 @@ struct TileCfg {
     static constexpr int SMEM_BYTES = (kTileK * KS + kTileK * D + kTileQ * D + kTileQ * kTileK) * 4;
 };
 
-template <typename T, int D>
+template <typename T, int D, bool MASKED>
 __global__ void __launch_bounds__(kTileThreads) sdpa_tile_kernel(const SdpaParams p) {
     pdl_sync();
     using Cfg = TileCfg<D>;
@@ -752,6 +934,7 @@ __global__ void __launch_bounds__(kTileThreads) sdpa_tile_kernel(const SdpaParam
     int kv_end = Skv;  // keys any row of this CTA can see
     if (p.causal && q0 + kTileQ < kv_end) kv_end = q0 + kTileQ;
 
+    const int64_t m_off = b * p.m_sb + h * p.m_sh;
     const int row0 = q0 + warp * 4;
     float o[4][NU];
     float m_run[4], l_run[4];
@@ -828,7 +1011,13 @@ __global__ void __launch_bounds__(kTileThreads) sdpa_tile_kernel(const SdpaParam
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int key = k0 + lane + 32 * i;
-                if (key >= Skv || (p.causal && key > row)) sc[r][i] = -INFINITY;
+                if (key >= Skv || (p.causal && key > row)) {
+                    sc[r][i] = -INFINITY;
+                } else if (MASKED && row < Sq) {
+                    const int64_t at = m_off + (int64_t)row * p.m_sq + (int64_t)key * p.m_sk;
+                    if (p.mask_kind == kMaskAdd) sc[r][i] += Cvt<T>::to_f(reinterpret_cast<const T*>(p.mask)[at]);
+                    else if (reinterpret_cast<const uint8_t*>(p.mask)[at] == 0) sc[r][i] = -INFINITY;
+                }
                 mx = fmaxf(mx, sc[r][i]);
             }
             const float m_new = fmaxf(m_run[r], warp_max(mx));
@@ -877,13 +1066,15 @@ __global__ void __launch_bounds__(kTileThreads) sdpa_tile_kernel(const SdpaParam
 template <typename T, int D>
 int launch_tile(const SdpaParams& p, cudaStream_t st) {
     using Cfg = TileCfg<D>;
-    auto kern = sdpa_tile_kernel<T, D>;
-    static std::atomic<uint64_t> reserved{0};
-    if (!reserve_smem(kern, Cfg::SMEM_BYTES, reserved)) return fail(XG_ERR_LAUNCH, "xg_sdpa_fwd: cannot reserve shared memory");
     const int64_t qt = (p.Sq + kTileQ - 1) / kTileQ, bh = p.B * p.H;
     if (qt > 0x7fffffffLL || bh > 65535) return -1;  // the caller falls back to the row-per-warp kernel
-    launch_with({.early = false}, kern, dim3((unsigned)qt, (unsigned)bh), kTileThreads, Cfg::SMEM_BYTES, st, p);
-    return check_launch("xg_sdpa_fwd");
+    auto run = [&](auto kern, std::atomic<uint64_t>& reserved) {
+        if (!reserve_smem(kern, Cfg::SMEM_BYTES, reserved)) return fail(XG_ERR_LAUNCH, "xg_sdpa_fwd: cannot reserve shared memory");
+        launch_with({.early = false}, kern, dim3((unsigned)qt, (unsigned)bh), kTileThreads, Cfg::SMEM_BYTES, st, p);
+        return check_launch("xg_sdpa_fwd");
+    };
+    static std::atomic<uint64_t> reserved[2];
+    return p.mask_kind == kMaskNone ? run(sdpa_tile_kernel<T, D, false>, reserved[0]) : run(sdpa_tile_kernel<T, D, true>, reserved[1]);
 }
 
 template <typename T>
@@ -924,10 +1115,20 @@ int read_sdpa_status(unsigned int* host_out, int reset) {
 }
 }  // namespace xg
 
-extern "C" int xg_sdpa_fwd(const void* q, const void* k, const void* v, const void* mask, void* out, int64_t B, int64_t H,
+static bool sdpa_tensor_core_shape(int64_t D, int dtype) { return dtype != XG_F32 && (D == 64 || D == 128); }
+
+extern "C" int64_t xg_sdpa_workspace_bytes(int64_t B, int64_t H, int64_t Sq, int64_t Skv, int64_t D, int dtype) {
+    using namespace xg;
+    if (B <= 0 || H <= 0 || Sq <= 0 || Skv <= 0 || dtype_size(dtype) == 0 || !sdpa_tensor_core_shape(D, dtype)) return 0;
+    const int64_t tiles = B * H * ((Sq + FM - 1) / FM);
+    const int splits = flash_splits(tiles, Skv);
+    return splits > 1 ? tiles * splits * FM * (D + 2) * 4 : 0;
+}
+
+extern "C" int xg_sdpa_fwd_ws(const void* q, const void* k, const void* v, const void* mask, void* out, int64_t B, int64_t H,
                            int64_t Sq, int64_t Skv, int64_t D, const int64_t* q_strides3, const int64_t* k_strides3,
                            const int64_t* v_strides3, const int64_t* o_strides3, const int64_t* mask_strides4, float scale,
-                           int causal, int dtype, void* stream) {
+                           int causal, int dtype, int mask_bool, void* workspace, int64_t workspace_bytes, void* stream) {
     using namespace xg;
     if (!q || !k || !v || !out || !q_strides3 || !k_strides3 || !v_strides3 || !o_strides3)
         return fail(XG_ERR_INVALID_ARG, "xg_sdpa_fwd: null pointer");
@@ -947,20 +1148,22 @@ extern "C" int xg_sdpa_fwd(const void* q, const void* k, const void* v, const vo
     p.m_sq = mask ? mask_strides4[2] : 0; p.m_sk = mask ? mask_strides4[3] : 0;
     p.scale = scale;
     p.causal = causal ? 1 : 0;
+    p.mask_kind = !mask ? kMaskNone : (mask_bool ? kMaskBool : kMaskAdd);
+    if (workspace_bytes < 0) return fail(XG_ERR_INVALID_ARG, "xg_sdpa_fwd: negative workspace size");
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 
     auto tma_ok = [&](const void* ptr, int64_t sb, int64_t sh, int64_t ss, int64_t S) {
         auto okst = [&](int64_t s, int64_t extent) { return extent == 1 || (s > 0 && s % 8 == 0); };
         return aligned16(ptr) && okst(ss, S) && okst(sh, H) && okst(sb, B);
     };
-    const bool tc = (dtype != XG_F32) && (D == 64 || D == 128) && Skv > 0 && tma_ok(q, p.q_sb, p.q_sh, p.q_ss, Sq) &&
+    const bool tc = sdpa_tensor_core_shape(D, dtype) && Skv > 0 && tma_ok(q, p.q_sb, p.q_sh, p.q_ss, Sq) &&
                     tma_ok(k, p.k_sb, p.k_sh, p.k_ss, Skv) && tma_ok(v, p.v_sb, p.v_sh, p.v_ss, Skv) && aligned16(out) &&
                     p.o_ss % 8 == 0 && p.o_sh % 8 == 0 && p.o_sb % 8 == 0 && Sq < 0x7fffff00LL && Skv < 0x7fffff00LL;
     if (tc) {
-        if (dtype == XG_BF16) return D == 128 ? launch_flash_tc<__nv_bfloat16, 128>(p, st) : launch_flash_tc<__nv_bfloat16, 64>(p, st);
-        return D == 128 ? launch_flash_tc<__half, 128>(p, st) : launch_flash_tc<__half, 64>(p, st);
+        if (dtype == XG_BF16) return D == 128 ? launch_flash_tc<__nv_bfloat16, 128>(p, workspace, workspace_bytes, st) : launch_flash_tc<__nv_bfloat16, 64>(p, workspace, workspace_bytes, st);
+        return D == 128 ? launch_flash_tc<__half, 128>(p, workspace, workspace_bytes, st) : launch_flash_tc<__half, 64>(p, workspace, workspace_bytes, st);
     }
-    if (mask == nullptr && Sq < 0x7fffff00LL && Skv < 0x7fffff00LL) {  // -1: not a shape the tiled kernel takes
+    if (Sq < 0x7fffff00LL && Skv < 0x7fffff00LL) {  // -1: not a shape the tiled kernel takes
         int rc = -1;
         switch (dtype) {
             case XG_F32: rc = launch_tile_any<float>(p, st); break;
@@ -974,4 +1177,12 @@ extern "C" int xg_sdpa_fwd(const void* q, const void* k, const void* v, const vo
         case XG_BF16: return launch_simt<__nv_bfloat16>(p, st);
         default: return launch_simt<__half>(p, st);
     }
+}
+
+extern "C" int xg_sdpa_fwd(const void* q, const void* k, const void* v, const void* mask, void* out, int64_t B, int64_t H,
+                           int64_t Sq, int64_t Skv, int64_t D, const int64_t* q_strides3, const int64_t* k_strides3,
+                           const int64_t* v_strides3, const int64_t* o_strides3, const int64_t* mask_strides4, float scale,
+                           int causal, int dtype, void* stream) {
+    return xg_sdpa_fwd_ws(q, k, v, mask, out, B, H, Sq, Skv, D, q_strides3, k_strides3, v_strides3, o_strides3, mask_strides4, scale,
+                          causal, dtype, 0, nullptr, 0, stream);
 }

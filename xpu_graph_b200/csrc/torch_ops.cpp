@@ -593,18 +593,25 @@ Tensor sdpa(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, const op
     const Tensor q = unit_rows(q_in), k = unit_rows(k_in), v = unit_rows(v_in);
     const int64_t B = q.size(0), H = q.size(1), Sq = q.size(2), D = q.size(3), Skv = k.size(2);
     Tensor m;
+    bool mask_bool = false;
     if (mask_in) {
-        m = *mask_in;
-        if (m.scalar_type() == at::kBool)
-            m = at::zeros(m.sizes(), q.options()).masked_fill_(m.logical_not(), -std::numeric_limits<double>::infinity());
-        m = cast(m, q.scalar_type());
+        mask_bool = mask_in->scalar_type() == at::kBool;
+        m = mask_bool ? *mask_in : cast(*mask_in, q.scalar_type());
         while (m.dim() < 4) m = m.unsqueeze(0);
         m = m.expand({B, H, Sq, Skv});
     }
     Tensor out = empty_like_layout(q);
-    XG_CALL(xg_sdpa_fwd, ptr(q), ptr(k), ptr(v), ptr(m), mut(out), B, H, Sq, Skv, D, q.strides().data(), k.strides().data(),
-            v.strides().data(), out.strides().data(), m.defined() ? m.strides().data() : nullptr, scale, is_causal ? 1 : 0,
-            code_of(q.scalar_type()), on.stream);
+    const int code = code_of(q.scalar_type());
+    const int64_t ws_bytes = xg_sdpa_workspace_bytes(B, H, Sq, Skv, D, code);
+    const int64_t* mstr = m.defined() ? m.strides().data() : nullptr;
+    if (ws_bytes == 0 && !mask_bool) {
+        XG_CALL(xg_sdpa_fwd, ptr(q), ptr(k), ptr(v), ptr(m), mut(out), B, H, Sq, Skv, D, q.strides().data(), k.strides().data(),
+                v.strides().data(), out.strides().data(), mstr, scale, is_causal ? 1 : 0, code, on.stream);
+        return out;
+    }
+    const Tensor ws = ws_bytes > 0 ? new_tensor({ws_bytes}, at::kByte, q) : Tensor();
+    XG_CALL(xg_sdpa_fwd_ws, ptr(q), ptr(k), ptr(v), ptr(m), mut(out), B, H, Sq, Skv, D, q.strides().data(), k.strides().data(),
+            v.strides().data(), out.strides().data(), mstr, scale, is_causal ? 1 : 0, code, mask_bool ? 1 : 0, mut(ws), ws_bytes, on.stream);
     return out;
 }
 

@@ -73,6 +73,9 @@ SIGNATURES = {
                              c_int64, c_int64, c_int64, c_int, c_void_p]),
     "xg_sdpa_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64,
                             c_int64, _I64P, _I64P, _I64P, _I64P, _I64P, c_float, c_int, c_int, c_void_p]),
+    "xg_sdpa_fwd_ws": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64,
+                               c_int64, _I64P, _I64P, _I64P, _I64P, _I64P, c_float, c_int, c_int, c_int, c_void_p, c_int64, c_void_p]),
+    "xg_sdpa_workspace_bytes": (c_int64, [c_int64, c_int64, c_int64, c_int64, c_int64, c_int]),
     "xg_seg_copy": (c_int, [_VPP, _VPP, _I64P, _I64P, _I64P, c_int64, c_int64, c_void_p, c_int, c_void_p]),
     "xg_gemm_f32x3_padded_k": (c_int64, [c_int64]),
     "xg_split_bf16x3": (c_int, [c_void_p, c_int64, c_int64, c_int64, c_int, c_void_p, c_void_p]),
@@ -169,6 +172,7 @@ def tc_status(reset: bool = True) -> int:
 
 # entry points that enqueue no kernel (queries and status reads)
 QUERY_ENTRY_POINTS = frozenset({"xg_version", "xg_device_arch_ok", "xg_last_error", "xg_tc_status", "xg_gemm_workspace_bytes", "xg_gemm_copy_bytes",
+                                "xg_sdpa_workspace_bytes",
                                 "xg_gemm_static_scratch_bytes", "xg_gemm_f32x3_padded_k", "xg_gemm_cluster_plan",
                                 "xg_mlp2_supported", "xg_mlp3_supported", "xg_mlp_small_supported"})
 
