@@ -117,3 +117,24 @@ def test_against_reference_fixtures(cuda_device, tag):
     c = G[f"sum_cat_{tag}"]
     mag = ref_ops.sum_cat([t.float().abs() for t in c["xs"]]) * (1e-2 if tag == "bf16" else 1e-3)
     assert_parity(SumCatModule()([t.to(cuda_device) for t in c["xs"]]), c["y"], f"fixture sum_cat {tag}", magnitude=mag)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(16384, 50, 64), (3000, 21, 100), (700, 9, 5), (3, 50, 8)])  # both vector widths, both sides of "small"
+def test_overlapping_ranges_in_one_walk(cuda_device, shape, dtype):
+    """Ranges of one tensor that overlap without a common first row share one walk; every sum takes its rows in ascending
+    order, as it does on its own, so the results have to be the same bits as one launch per range."""
+    from xpu_graph_b200.modules import SliceSumCatModule
+
+    x = _rand(shape, dtype, 61).to(cuda_device)
+    R = shape[1]
+    sets = [[(0, R), (0, R // 2), (0, R // 5), (R // 4, R * 3 // 4)],               # pooling windows
+            [(R - 1, R), (0, R), (0, R), (2, 2), (1, R - 1)],                        # repeated, empty and one-row ranges: five sums
+            [(i, R) for i in range(8)], [(0, 3), (1, 4), (1, 4), (R - 3, R), (R - 3, R)]]  # eight sums; rows of no range between
+    for ranges in sets:
+        got = SliceSumCatModule(ranges)(x)
+        want = torch.cat([SliceSumCatModule([r])(x) for r in ranges], dim=-1)
+        assert torch.equal(got, want), (shape, dtype, ranges)
+    want = ref_ops.slice_sum_cat(x.float().cpu(), sets[0]).to(dtype)
+    mag = ref_ops.slice_sum_cat(x.float().abs().cpu(), sets[0])
+    assert_parity(SliceSumCatModule(sets[0])(x), want, "overlapping ranges", magnitude=mag * (1e-2 if dtype != torch.float32 else 1e-3))
