@@ -11,7 +11,7 @@ namespace xg {
 namespace {
 
 constexpr int kMaxSegs = 64;     // segments per launch (kernel parameter space)
-constexpr int kLutMax = 8192;    // output units per row per launch (32 KiB of shared memory)
+constexpr int kLutMax = 8192;    // output units per row per launch (at most 32 KiB of shared memory)
 constexpr int kCopyThreads = 256;
 constexpr int kCopyUnroll = 4;
 constexpr int kGatherRows = 8;    // rows per CTA in the gather kernel
@@ -46,12 +46,16 @@ template <typename U>
 __global__ void __launch_bounds__(kCopyThreads) seg_copy_kernel(const __grid_constant__ SegCopyParams p) {
     pdl_sync();
     __shared__ SegDesc segs[kMaxSegs];
-    __shared__ uint32_t lut[kLutMax];
+    extern __shared__ uint32_t lut[];  // [width]: no more than the launch needs, so that eight CTAs fit an SM
     for (int k = threadIdx.x; k < p.nseg; k += kCopyThreads) segs[k] = p.seg[k];
     __syncthreads();
-    for (int k = 0; k < p.nseg; ++k) {
-        const int n = segs[k].units, s0 = segs[k].unit_start;
-        for (int j = threadIdx.x; j < n; j += kCopyThreads) lut[s0 + j] = ((uint32_t)k << 24) | (uint32_t)j;
+    // a thread looks its columns' segments up by bisection: one step of latency per doubling of the segments instead of one
+    // per segment (a CTA lives for a few microseconds, and with a pass per segment the table took most of them)
+    for (int c = threadIdx.x; c < p.width; c += kCopyThreads) {
+        int k = 0;
+        for (int step = kMaxSegs / 2; step > 0; step >>= 1)
+            if (k + step < p.nseg && segs[k + step].unit_start <= c) k += step;
+        lut[c] = ((uint32_t)k << 24) | (uint32_t)(c - segs[k].unit_start);
     }
     __syncthreads();
 
@@ -118,7 +122,7 @@ template <typename U>
 int launch_seg_copy(const SegCopyParams& p, cudaStream_t st) {
     const int64_t grid = (p.rows + p.rows_per_cta - 1) / p.rows_per_cta;
     if (grid > 0x7fffffffLL) return fail(XG_ERR_TOO_LARGE, "xg_seg_copy: too many row tiles");
-    launch(seg_copy_kernel<U>, (unsigned)grid, kCopyThreads, 0, st, p);
+    launch(seg_copy_kernel<U>, (unsigned)grid, kCopyThreads, (size_t)p.width * sizeof(uint32_t), st, p);
     return check_launch("xg_seg_copy");
 }
 
