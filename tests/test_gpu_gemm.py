@@ -863,3 +863,44 @@ def test_dense_operands_copied_into_addressable_rows(cuda_device, M, K, N, weigh
                                  {torch.float32: lib.XG_F32, torch.bfloat16: lib.XG_BF16, torch.float16: lib.XG_F16}[dtype],
                                  torch.cuda.current_stream().cuda_stream), "xg_gemm_bias_act")
     assert_parity(got, want.cpu(), f"dense {M}x{K}x{N} {dtype} through copies")
+
+
+def _planes(x):
+    """fp32 -> its three bf16 planes, as fp32 tensors."""
+    a = x.bfloat16().float()
+    b = (x - a).bfloat16().float()
+    return a, b, (x - a - b).bfloat16().float()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 64, 512), (130, 96, 700), (256, 100, 1728), (257, 520, 1000), (500, 1024, 1728), (2100, 256, 512)])
+def test_f32x3_few_tiles(cuda_device, M, N, K):
+    """fp32 layers of few tiles, planes in, fp32 or planes out: rows and columns past the last tile, padded planes. The yardstick
+    is fp64 math; the products left out are below 2^-24 of |x||w|, the sums are fp32."""
+    import ctypes
+
+    from xpu_graph_b200 import lib
+
+    L = lib.load()
+    x, w, b = (t.to(cuda_device) for t in _mk(M, K, N, torch.float32, 71))
+    r = torch.randn(M, N, device=cuda_device)
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    kp, np_ = L.xg_gemm_f32x3_padded_k(K), L.xg_gemm_f32x3_padded_k(N)
+    x3, w3 = (torch.empty(n, 3 * kp, dtype=torch.bfloat16, device=cuda_device) for n in (M, N))
+    assert L.xg_split_bf16x3(x.data_ptr(), M, K, K, 0, x3.data_ptr(), st) == 0
+    assert L.xg_split_bf16x3(w.data_ptr(), N, K, K, 0, w3.data_ptr(), st) == 0
+    y = x.double() @ w.double().t() + b.double()
+    mag = (x.double().abs() @ w.double().abs().t()).float().cpu()
+    out = torch.full((M, N), 7.0, device=cuda_device)
+    assert L.xg_gemm_f32x3(x3.data_ptr(), w3.data_ptr(), b.data_ptr(), r.data_ptr(), out.data_ptr(), M, N, K, N, N, 1, 0, st) == 0
+    torch.cuda.synchronize()
+    assert lib.tc_status() == 0
+    assert_parity(out, ref_ops._ACTS["gelu"](y + r.double()).float().cpu(), f"f32x3 {M}x{N}x{K} fp32 out", magnitude=mag)
+    # sigmoid(0) != 0: the padding columns have to be zero, not the activation of zero
+    out3 = torch.full((M, 3 * np_), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    assert L.xg_gemm_f32x3(x3.data_ptr(), w3.data_ptr(), b.data_ptr(), None, out3.data_ptr(), M, N, K, N, 0, 4, 1, st) == 0
+    torch.cuda.synchronize()
+    parts = out3.float().view(M, 3, np_)
+    assert_parity(parts.sum(1)[:, :N], torch.sigmoid(y).float().cpu(), f"f32x3 {M}x{N}x{K} planes out")
+    assert (parts[:, :, N:] == 0).all()
+    for got, want in zip(parts[:, :, :N].unbind(1), _planes(parts.sum(1)[:, :N])):
+        assert torch.equal(got, want)

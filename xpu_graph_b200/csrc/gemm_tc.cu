@@ -41,6 +41,9 @@ int gemm_tc_ksplit_entry(const void* A, const void* W, const void* bias, const v
                          int64_t N, int64_t K, int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int act, int dtype, int S,
                          int tn, cudaStream_t st);
 
+int gemm_f32x3_ksplit_entry(const void* A3, const void* W3, const void* bias, const void* residual, void* out, int64_t M, int64_t N,
+                            int64_t Kp, int64_t ldc, int64_t ldr, int act, bool out_planes, bool* taken, cudaStream_t st);
+
 struct GemmPlan {
     int bn;      // tile width: 64, 128 or 256
     int splits;  // split-K factor (1 = none)
@@ -1428,6 +1431,9 @@ int gemm_f32x3_entry(const void* A3, const void* W3, const void* bias, const voi
         return fail(XG_ERR_UNSUPPORTED, "xg_gemm_f32x3: the plane output must be 16-byte aligned and takes no residual");
     if (M > (int64_t)BM * 0x7fffff || N > (int64_t)64 * 0x7fffff || 6 * Kp > 0x7fffffff)
         return fail(XG_ERR_TOO_LARGE, "xg_gemm_f32x3: extent too large");
+    bool taken = false;
+    const int rc = gemm_f32x3_ksplit_entry(A3, W3, bias, residual, out, M, N, Kp, ldc, ldr, act, out_planes != 0, &taken, st);
+    if (taken) return rc;
     GemmParams p;
     p.out = out;
     p.bias = bias;

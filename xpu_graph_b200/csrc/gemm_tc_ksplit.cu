@@ -1,4 +1,5 @@
-// Dense layer for problems with few output tiles (small M: the weight-streaming regime), 16-bit inputs.
+// Dense layer for problems with few output tiles (small M: the weight-streaming regime): 16-bit inputs, or fp32 as three
+// bf16 planes per operand (six plane pairs, six times the k-blocks: sharing them out over the pairs pays early).
 //
 // A 256 x 256 output tile belongs to a thread-block cluster of 2*S CTAs = S CTA pairs. Pair s computes the tile over
 // its share of the k-blocks with tcgen05.mma.cta_group::2 (each CTA loads 128 activation rows and 128 weight rows per
@@ -52,6 +53,11 @@ struct KsplitParams {
     int S;            // pairs per cluster = k-splits
     int tn;           // tile width (weight rows per tile): a multiple of 32 in [64, 256], at least 32 * S
     int stages;       // pipeline depth
+    // fp32 problems only (see GemmParams in gemm_tc.cu): k-blocks run over plane pairs, out is fp32 or (out_kp > 0) the
+    // next layer's three bf16 planes of out_kp columns
+    int seg_blocks;
+    uint32_t seg_a, seg_b;
+    int out_kp;
 };
 static_assert(KS_SMEM_BYTES <= 232448, "shared memory of one CTA");
 static_assert(KS_STAGES_WHOLE * KS_STAGE_BYTES <= KS_STAGES_SPLIT * KS_STAGE_BYTES + KS_RECV_CHUNKS * KS_CHUNK_BYTES, "S = 1 layout");
@@ -121,7 +127,60 @@ __device__ __forceinline__ void store_cols16(const KsplitParams& p, float (&v)[1
     }
 }
 
-template <typename T>
+// ... of an fp32 problem: fp32 bias, residual and result, or the three bf16 planes of the result (columns up to out_kp, those
+// past N zero)
+__device__ __forceinline__ float act_f32(float v, int act) {
+    return act == XG_ACT_GELU ? 0.5f * v * (1.0f + erff(v * 0.70710678118654752f)) : act_of(v, act);
+}
+__device__ __forceinline__ void store_cols16_f32(const KsplitParams& p, float (&v)[16], const float* bias_s, int64_t row, bool row_ok,
+                                                 int64_t col0) {
+#pragma unroll
+    for (int i = 0; i < 16; i += 4) {
+        const float4 b4 = *reinterpret_cast<const float4*>(bias_s + i);
+        v[i] += b4.x; v[i + 1] += b4.y; v[i + 2] += b4.z; v[i + 3] += b4.w;
+    }
+    if (!row_ok) return;
+    if (p.out_kp > 0) {
+        __nv_bfloat16* o3 = reinterpret_cast<__nv_bfloat16*>(p.out) + row * (3 * (int64_t)p.out_kp) + col0;
+#pragma unroll
+        for (int i = 0; i < 16; i += 8) {
+            Vec16<__nv_bfloat16> q0, q1, q2;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float x = (col0 + i + j < p.N) ? act_f32(v[i + j], p.act) : 0.f;
+                q0.v[j] = __float2bfloat16_rn(x);
+                const float r1 = x - __bfloat162float(q0.v[j]);
+                q1.v[j] = __float2bfloat16_rn(r1);
+                q2.v[j] = __float2bfloat16_rn(r1 - __bfloat162float(q1.v[j]));
+            }
+            st16(o3 + i, q0);
+            st16(o3 + p.out_kp + i, q1);
+            st16(o3 + 2 * (int64_t)p.out_kp + i, q2);
+        }
+        return;
+    }
+    const float* rr = p.residual ? reinterpret_cast<const float*>(p.residual) + row * p.ldr + col0 : nullptr;
+    float* orow = reinterpret_cast<float*>(p.out) + row * p.ldc + col0;
+    if (col0 + 16 <= p.N && p.vec_ok) {
+#pragma unroll
+        for (int i = 0; i < 16; i += 4) {
+            float4 o = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+            if (rr != nullptr) {
+                const float4 r4 = *reinterpret_cast<const float4*>(rr + i);
+                o.x += r4.x; o.y += r4.y; o.z += r4.z; o.w += r4.w;
+            }
+            *reinterpret_cast<float4*>(orow + i) =
+                make_float4(act_f32(o.x, p.act), act_f32(o.y, p.act), act_f32(o.z, p.act), act_f32(o.w, p.act));
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (col0 + i < p.N) orow[i] = act_f32(v[i] + (rr != nullptr ? rr[i] : 0.f), p.act);
+    }
+}
+
+// F32X3: T is bf16, the operands are planes of fp32 matrices
+template <typename T, bool F32X3>
 __global__ void __launch_bounds__(KS_THREADS, 1)
 gemm_tc_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
                       const KsplitParams p) {
@@ -196,8 +255,14 @@ gemm_tc_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                 if (r == 0) ptx::mbar_arrive_expect_tx(&full_bar[stage], 2u * ((uint32_t)A_BYTES + w_bytes));
                 const uint32_t full_leader = ptx::map_to_cta(ptx::smem_u32(&full_bar[stage]), leader);
                 uint8_t* st = smem + stage * KS_STAGE_BYTES;
-                ptx::tma_load_2d_pair(st, &tmap_a, full_leader, kb * BK, mb * TILE + (int)r * BM);
-                ptx::tma_load_2d_pair(st + A_BYTES, &tmap_w, full_leader, kb * BK, nb * TN + (int)r * (TN / 2));
+                int ka = kb * BK, kw = ka;
+                if (F32X3) {
+                    const int pair = kb / p.seg_blocks, kk = kb - pair * p.seg_blocks;
+                    ka = ((int)((p.seg_a >> (4 * pair)) & 15u) * p.seg_blocks + kk) * BK;
+                    kw = ((int)((p.seg_b >> (4 * pair)) & 15u) * p.seg_blocks + kk) * BK;
+                }
+                ptx::tma_load_2d_pair(st, &tmap_a, full_leader, ka, mb * TILE + (int)r * BM);
+                ptx::tma_load_2d_pair(st + A_BYTES, &tmap_w, full_leader, kw, nb * TN + (int)r * (TN / 2));
                 if (++stage == STAGES) { stage = 0; phase ^= 1u; }
             }
             if (!ok) atomicOr(&g_ksplit_status[0], 1u);
@@ -249,7 +314,8 @@ gemm_tc_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         // the tile's bias row, once, while the main loop runs
         for (int i = (int)threadIdx.x - 64; i < TN; i += KS_EPI_WARPS * 32) {
             const int64_t col = (int64_t)nb * TN + i;
-            bias_s[i] = (p.bias != nullptr && col < p.N) ? Cvt<T>::to_f(reinterpret_cast<const T*>(p.bias)[col]) : 0.f;
+            using Bias = typename std::conditional<F32X3, float, T>::type;
+            bias_s[i] = (p.bias != nullptr && col < p.N) ? Cvt<Bias>::to_f(reinterpret_cast<const Bias*>(p.bias)[col]) : 0.f;
         }
         bool ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(tmem_full, 0, abort_flag));
         // All MMAs of this pair have completed: the accumulator is final and the pipeline buffers are idle.
@@ -309,15 +375,18 @@ gemm_tc_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                         }
                     }
                 }
-                store_cols16<T>(p, v, bias_s + (my_lo + cl) * 32 + half * 16, row, row < p.M, unit_col0(u));
+                const float* unit_bias = bias_s + (my_lo + cl) * 32 + half * 16;
+                if (F32X3) store_cols16_f32(p, v, unit_bias, row, row < p.M, unit_col0(u));
+                else store_cols16<T>(p, v, unit_bias, row, row < p.M, unit_col0(u));
             };
+            const int64_t cols = F32X3 && p.out_kp > 0 ? p.out_kp : p.N;
             // two units per round: both accumulator reads are in flight before either is used (a round is mostly the
             // latency of the TMEM read and of the stores, so a warp with three units to finish pays for two rounds, not three)
 #pragma unroll 1
             for (int u = grp; u < 2 * mine; u += 2 * GROUPS) {
-                if (unit_col0(u) >= p.N) break;  // warp-uniform; later units of this warp lie further right
+                if (unit_col0(u) >= cols) break;  // warp-uniform; later units of this warp lie further right
                 const int u2 = u + GROUPS;
-                const bool second = u2 < 2 * mine && unit_col0(u2) < p.N;
+                const bool second = u2 < 2 * mine && unit_col0(u2) < cols;
                 uint32_t own[16], own2[16];
                 ptx::tmem_ld_32x16(unit_taddr(u), own);
                 if (second) ptx::tmem_ld_32x16(unit_taddr(u2), own2);
@@ -340,11 +409,11 @@ gemm_tc_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 }
 
 // How many clusters of 2*S CTAs of this kernel can be resident at once (cached per S and kernel instantiation).
-template <typename T>
+template <typename T, bool F32X3 = false>
 int max_active_clusters(int S) {
     static thread_local int cached[KS_MAX_SPLIT + 1] = {0, 0, 0, 0, 0};
     if (cached[S] > 0) return cached[S];
-    auto kern = gemm_tc_ksplit_kernel<T>;
+    auto kern = gemm_tc_ksplit_kernel<T, F32X3>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(2 * S * 64));
     cfg.blockDim = dim3(KS_THREADS);
@@ -367,11 +436,12 @@ int max_active_clusters(int S) {
     return n;
 }
 
-template <typename T>
+template <typename T, bool F32X3 = false>
 int launch_ksplit(const void* A, const void* W, const void* bias, const void* residual, void* out, int64_t M, int64_t N,
-                  int64_t K, int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int act, int S, int tn, cudaStream_t st) {
+                  int64_t K, int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int act, int S, int tn, cudaStream_t st,
+                  bool out_planes = false) {
     constexpr bool is_bf16 = std::is_same<T, __nv_bfloat16>::value;
-    auto kern = gemm_tc_ksplit_kernel<T>;
+    auto kern = gemm_tc_ksplit_kernel<T, F32X3>;
     static std::atomic<uint64_t> reserved{0};
     if (!reserve_smem(kern, KS_SMEM_BYTES, reserved))
         return fail(XG_ERR_LAUNCH, "xg_gemm_bias_act: cannot reserve %d bytes of shared memory", KS_SMEM_BYTES);
@@ -386,11 +456,19 @@ int launch_ksplit(const void* A, const void* W, const void* bias, const void* re
     p.residual = residual;
     p.M = M; p.N = N; p.ldc = ldc; p.ldr = ldr;
     p.act = act;
-    p.vec_ok = (ldc % 8 == 0) && aligned16(out) && (!residual || (ldr % 8 == 0 && aligned16(residual)));
+    constexpr int64_t kVec = F32X3 ? 4 : 8;  // elements in 16 bytes
+    p.vec_ok = (ldc % kVec == 0) && aligned16(out) && (!residual || (ldr % kVec == 0 && aligned16(residual)));
     p.bias_vec_ok = bias ? aligned16(bias) : 0;
+    p.out_kp = out_planes ? (int)((N + BK - 1) / BK * BK) : 0;
     p.num_m_blocks = (int)((M + TILE - 1) / TILE);
-    p.num_n_blocks = (int)((N + tn - 1) / tn);
+    p.num_n_blocks = (int)(((out_planes ? p.out_kp : N) + tn - 1) / tn);  // the planes' padding is written too
     p.num_k_blocks = (int)((K + BK - 1) / BK);
+    if (F32X3) {
+        p.seg_blocks = p.num_k_blocks / 3;  // K counts the three planes
+        p.num_k_blocks *= 2;
+        p.seg_a = 0x010120u;  // pairs (A plane, W plane): (0,2) (2,0) (1,1) (0,1) (1,0) (0,0)
+        p.seg_b = 0x001102u;
+    }
     p.S = S;
     p.tn = tn;
     p.stages = S > 1 ? KS_STAGES_SPLIT : KS_STAGES_WHOLE;
@@ -419,8 +497,9 @@ bool ksplit_shape_ok(int S, int tn, int64_t nkb) {
 // about 127 KB/us per SM plus 3 us. The cluster kernel runs when it comes out at least 10 % ahead, which for
 // K = 4096 means 128 < M <= 512 at N = 4096 (13.3 vs 15.7 us at M = 256, 19.6 vs 26.9 us at M = 512) and M <= 256 at
 // N = 11008 (22.3 vs 36.3 us), and shapes with between one and two waves of 256 x 256 tiles (512 x 11008: 43 vs
-// 51 us for the pair kernel). Smaller M stays with split-K through scratch, which is ahead there.
-bool plan_ksplit(int64_t M, int64_t N, int64_t K, int dtype, int* S_out, int* tn_out) {
+// 51 us for the pair kernel). Smaller M stays with split-K through scratch, which is ahead there; fp32 problems
+// (`f32x3`, K = 6 x the padded K) have no such path and come here at any M.
+static bool plan_clusters(bool f32x3, int64_t M, int64_t N, int64_t K, int dtype, int* S_out, int* tn_out) {
     static const int forced_s = []() {
         const char* e = getenv("XG_GEMM_KSPLIT");
         return e ? atoi(e) : -1;
@@ -439,7 +518,7 @@ bool plan_ksplit(int64_t M, int64_t N, int64_t K, int dtype, int* S_out, int* tn
         *tn_out = forced_tn;
         return true;
     }
-    if (M <= 128 || nkb < 8) return false;  // small M: split-K through scratch is ahead; short K: nothing to stream
+    if ((M <= 128 && !f32x3) || nkb < 8) return false;  // small M: split-K through scratch is ahead; short K: nothing to stream
     const int sms = num_sms();
     const int64_t tiles256 = mblk * ((N + 255) / 256);
     if (tiles256 >= sms) return false;  // two full waves or more of 256 x 256 tiles: the persistent pair kernel's regime
@@ -456,7 +535,7 @@ bool plan_ksplit(int64_t M, int64_t N, int64_t K, int dtype, int* S_out, int* tn
         const int nch = tn / 32;
         for (int S = 1; S <= KS_MAX_SPLIT; ++S) {
             if (!ksplit_shape_ok(S, tn, nkb) || (S > 1 && nkb < 8 * S)) continue;
-            const int active = dtype == XG_BF16 ? max_active_clusters<__nv_bfloat16>(S) : max_active_clusters<__half>(S);
+            const int active = f32x3 ? max_active_clusters<__nv_bfloat16, true>(S) : dtype == XG_BF16 ? max_active_clusters<__nv_bfloat16>(S) : max_active_clusters<__half>(S);
             const double waves = (double)((tiles + active - 1) / active);
             const int own = (nch + S - 1) / S, sent = nch - nch / S;
             double wave = (double)((nkb + S - 1) / S) * per_kblock(16.0 + tn / 2 * 0.125, tn) + 3.6 + 0.9 * rounds(own);
@@ -483,6 +562,19 @@ bool plan_ksplit(int64_t M, int64_t N, int64_t K, int dtype, int* S_out, int* tn
     *S_out = best_s;
     *tn_out = best_tn;
     return true;
+}
+
+bool plan_ksplit(int64_t M, int64_t N, int64_t K, int dtype, int* S_out, int* tn_out) {
+    return plan_clusters(false, M, N, K, dtype, S_out, tn_out);
+}
+
+// The fp32 problem of gemm_f32x3_entry (operands [M, 3 Kp] and [N, 3 Kp]) on clusters; *taken says whether it was launched.
+int gemm_f32x3_ksplit_entry(const void* A3, const void* W3, const void* bias, const void* residual, void* out, int64_t M, int64_t N,
+                            int64_t Kp, int64_t ldc, int64_t ldr, int act, bool out_planes, bool* taken, cudaStream_t st) {
+    int S = 0, tn = 0;
+    *taken = plan_clusters(true, M, N, 6 * Kp, XG_BF16, &S, &tn);
+    if (!*taken) return XG_OK;
+    return launch_ksplit<__nv_bfloat16, true>(A3, W3, bias, residual, out, M, N, 3 * Kp, 3 * Kp, 3 * Kp, ldc, ldr, act, S, tn, st, out_planes);
 }
 
 int gemm_tc_ksplit_entry(const void* A, const void* W, const void* bias, const void* residual, void* out, int64_t M,
