@@ -361,6 +361,19 @@ int xg_gather_rows(const void* const* tables, const int64_t* table_rows, int64_t
                    int elem_size, void* stream);
 
 /*
+ * Slices of a row and table lookups side by side, fp32, as the operand of xg_gemm_f32x3: columns of row r are
+ *   src[r*src_ld + starts[k] .. + lens[k]) for every slice, then zero_row(r) ? 0 : tables[f][idx(r,f)*D + j] for every table
+ * and out3 is [rows, 3*Kp], Kp = xg_gemm_f32x3_padded_k(columns): the three bf16 planes of that matrix (xg_split_bf16x3),
+ * zero-padded. starts, lens, src_ld and D are multiples of 4, all pointers 16-byte aligned, at most 64 slices and 64 tables
+ * and 4096 sliced columns, else XG_ERR_UNSUPPORTED. Indices as in xg_gather_rows.
+ * Replaces: the copies in front of a recommender's fp32 tower (slices + cat, embedding lookups + where + stack).
+ */
+int xg_gather_planes(const void* src, int64_t src_ld, const int64_t* starts, const int64_t* lens, int64_t nslices,
+                     const void* const* tables, const int64_t* table_rows, int64_t F, const int64_t* idx,
+                     int64_t idx_row_stride, int64_t idx_col_stride, const uint8_t* row_mask, int mask_zero_when,
+                     void* out3, int64_t rows, int64_t D, void* stream);
+
+/*
  * Batched sum over one dim of n contiguous 3-D tensors in one launch: outputs[k] = sum(inputs[k], dim),
  * shapes3 = HOST array [n][3] of (s0, s1, s2); dim 0 -> [s1, s2], dim 1 -> [s0, s2], dim 2 -> [s0, s1]
  * (contiguous, same dtype, fp32 accumulation). inputs/outputs: HOST arrays of device pointers.

@@ -158,3 +158,74 @@ def test_combo_sum(cuda_device, dim, dtype):
     assert len(got) == len(want)
     for a, e in zip(got, want):
         assert_parity(a, e.to(dtype), f"combo_sum dim {dim}")
+
+
+@pytest.mark.parametrize("rows,widths,F,D", [(1, (8, 4), 3, 64), (501, (4,) * 16, 26, 64), (4099, (100, 12), 5, 36), (64, (), 40, 4), (37, (512,), 1, 2048)])
+@pytest.mark.parametrize("masked", [True, False])
+def test_gather_planes(cuda_device, rows, widths, F, D, masked):
+    """Slices and lookups written as bf16 planes by one kernel vs the split of the assembled matrix, bit for bit: rows that do
+    not fill a group, masked rows, indices outside their table, padding columns."""
+    import ctypes
+
+    from xpu_graph_b200 import lib
+
+    L = lib.load()
+    g = torch.Generator().manual_seed(81)
+    src = torch.randn(rows, sum(widths) + 8, generator=g).to(cuda_device)
+    starts = [sum(widths[i + 1:]) + 4 for i in range(len(widths))]  # back to front
+    tables = [torch.randn(20 + f, D, generator=g).to(cuda_device) for f in range(F)]
+    idx = torch.randint(-2, 24, (rows, F), generator=g).to(cuda_device)
+    mask = (torch.rand(rows, generator=g) < 0.3).to(cuda_device) if masked else None
+    parts = [src[:, s:s + w] for s, w in zip(starts, widths)]
+    for f, t in enumerate(tables):
+        ok = (idx[:, f] >= 0) & (idx[:, f] < t.shape[0])
+        if masked:
+            ok = ok & ~mask
+        parts.append(torch.where(ok[:, None], t[idx[:, f].clamp(0, t.shape[0] - 1)], torch.zeros((), device=cuda_device)))
+    whole = torch.cat(parts, dim=1).contiguous()
+    K = whole.shape[1]
+    Kp = L.xg_gemm_f32x3_padded_k(K)
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    want, got = (torch.full((rows, 3 * Kp), v, dtype=torch.bfloat16, device=cuda_device) for v in (3.0, 7.0))
+    assert L.xg_split_bf16x3(whole.data_ptr(), rows, K, K, 0, want.data_ptr(), st) == 0
+    rc = L.xg_gather_planes(src.data_ptr(), src.stride(0), lib.i64_array(starts), lib.i64_array(widths), len(widths),
+                            lib.ptr_array([t.data_ptr() for t in tables]), lib.i64_array([t.shape[0] for t in tables]), F, idx.data_ptr(), F, 1,
+                            mask.data_ptr() if masked else None, 1, got.data_ptr(), rows, D, st)
+    assert rc == 0, lib.last_error()
+    torch.cuda.synchronize()
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+
+
+def test_recommender_forms(cuda_device):
+    """The recommender on inputs that the one-kernel assembly takes and on forms it leaves to the separate copies (slices that
+    are no whole 16-byte units, strided features, indices and tables): the same result within fp32 sums."""
+    from xpu_graph_b200 import lib, ops  # noqa: F401
+
+    g = torch.Generator().manual_seed(82)
+    rows, F, D = 700, 20, 64
+    tables = [torch.randn(50, D, generator=g).to(cuda_device) for _ in range(F)]
+    idx = torch.randint(0, 50, (rows, F), generator=g).to(cuda_device)
+    mask = (torch.rand(rows, 1, generator=g) < 0.3).to(cuda_device)
+    wide = torch.randn(rows, 65, generator=g).to(cuda_device)
+
+    def check(feats, idx, tables, starts, ends, dims):
+        k = sum(e - s for s, e in zip(starts, ends)) + F * D
+        ws = [(torch.randn(n, m, generator=g) * m ** -0.5).to(cuda_device) for m, n in zip([k] + dims, dims)]
+        bs = [torch.randn(n, generator=g).to(cuda_device) for n in dims]
+        got = torch.ops.xg_sm100.recommender(feats, idx, mask, tables, starts, ends, ws, bs)
+        emb = torch.stack([t[idx[:, f]] for f, t in enumerate(tables)], 1).masked_fill(mask[:, :, None], 0).flatten(1)
+        h = torch.cat([feats[:, s:e] for s, e in zip(starts, ends)] + [emb], 1).double()
+        for w, b in zip(ws, bs):
+            h = torch.relu(h @ w.double().t() + b.double())
+        torch.cuda.synchronize()
+        assert lib.tc_status() == 0
+        rel = ((got.double() - h).norm() / h.norm()).item()
+        assert rel < 5e-6, rel  # fp32 sums over 1300 products, three layers
+
+    even = wide[:, :64].contiguous()
+    for dims in ([1024, 1024, 256], [1024, 64], [1024]):  # planes to planes, planes to the FMA layers, one layer
+        check(even, idx, tables, [32, 0], [64, 32], dims)
+    check(even, idx, tables, [1, 30], [30, 64], [1024])
+    check(wide[:, 1:], idx, tables, [32, 0], [64, 32], [1024])
+    check(wide.t().contiguous().t(), idx, tables, [0], [64], [1024])
+    check(even, idx.t().contiguous().t(), [t.t().contiguous().t() for t in tables], [0], [64], [1024])

@@ -212,8 +212,150 @@ int launch_gather(const GatherParams& p, cudaStream_t st) {
     return check_launch("xg_gather_rows");
 }
 
+// ---------------------------------------------------------------------------------------
+// slices and lookups side by side, as the three bf16 planes that the fp32 tensor-core layers read
+// ---------------------------------------------------------------------------------------
+// out3[r][s * Kp + k], s = 0..2: columns 0..K-1 are the slices of src's row r, then the rows idx[r][f] of the tables (zeros
+// where the mask hides the row or the index is outside its table), columns up to Kp are zero. A unit is four columns of one
+// row; a thread takes the same unit of four rows (four index loads, then four 16-byte loads in flight). HBM-bound: reading the
+// tables and writing 6 bytes per column is all the traffic. As separate copies, a gather and a split the fp32 matrix was
+// written and read twice: 16384 rows of 64 + 26 x 64 took 152 us, 1.7 KB of reads and 10.4 KB of writes per row.
+constexpr int kPlaneRows = 4;
+constexpr int kPlaneMaxSliceUnits = 1024;
+struct PlanesParams {
+    const float* table[kMaxSegs];
+    int32_t table_rows[kMaxSegs];
+    int32_t start[kMaxSegs];       // slices: first unit in the source row ...
+    int32_t unit_start[kMaxSegs];  // ... and in the output row
+    const float* src;
+    const int64_t* idx;
+    const uint8_t* mask;
+    __nv_bfloat16* out3;
+    int64_t rows, src_ld, idx_rs, idx_cs, Kp;
+    int32_t nslices, slice_units, F, units_per_lookup, zero_when;
+};
+static_assert(sizeof(PlanesParams) <= 4096, "kernel parameter space");
+
+__device__ __forceinline__ void split3(float x, __nv_bfloat16& a, __nv_bfloat16& b, __nv_bfloat16& c) {
+    a = __float2bfloat16_rn(x);
+    const float r1 = x - __bfloat162float(a);
+    b = __float2bfloat16_rn(r1);
+    c = __float2bfloat16_rn(r1 - __bfloat162float(b));
+}
+
+__global__ void __launch_bounds__(kCopyThreads) gather_planes_kernel(const __grid_constant__ PlanesParams p) {
+    pdl_sync();
+    __shared__ const float* tab[kMaxSegs];
+    __shared__ int trows[kMaxSegs];
+    __shared__ int src_unit[kPlaneMaxSliceUnits];
+    for (int f = threadIdx.x; f < p.F; f += blockDim.x) {
+        tab[f] = p.table[f];
+        trows[f] = p.table_rows[f];
+    }
+    for (int c = threadIdx.x; c < p.slice_units; c += blockDim.x) {
+        int k = 0;
+        for (int step = kMaxSegs / 2; step > 0; step >>= 1)
+            if (k + step < p.nslices && p.unit_start[k + step] <= c) k += step;
+        src_unit[c] = p.start[k] + c - p.unit_start[k];
+    }
+    __syncthreads();
+    const int64_t r0 = (int64_t)blockIdx.x * kPlaneRows;
+    const int units = (int)(p.Kp / 4), used = p.slice_units + p.F * p.units_per_lookup;
+    bool hidden[kPlaneRows];
+#pragma unroll
+    for (int k = 0; k < kPlaneRows; ++k)
+        hidden[k] = r0 + k >= p.rows || (p.mask != nullptr && ((p.mask[r0 + k] != 0) == (p.zero_when != 0)));
+    for (int c = threadIdx.x; c < units; c += blockDim.x) {
+        float4 v[kPlaneRows];
+#pragma unroll
+        for (int k = 0; k < kPlaneRows; ++k) v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (c < p.slice_units) {
+            const float* s = p.src + 4 * (int64_t)src_unit[c];
+#pragma unroll
+            for (int k = 0; k < kPlaneRows; ++k)
+                if (r0 + k < p.rows) v[k] = *reinterpret_cast<const float4*>(s + (r0 + k) * p.src_ld);
+        } else if (c < used) {
+            const int f = (c - p.slice_units) / p.units_per_lookup, u = c - p.slice_units - f * p.units_per_lookup;
+            int64_t ix[kPlaneRows];
+#pragma unroll
+            for (int k = 0; k < kPlaneRows; ++k) ix[k] = hidden[k] ? -1 : p.idx[(r0 + k) * p.idx_rs + f * p.idx_cs];
+#pragma unroll
+            for (int k = 0; k < kPlaneRows; ++k)
+                if (ix[k] >= 0 && ix[k] < trows[f])
+                    v[k] = reinterpret_cast<const float4*>(tab[f])[ix[k] * p.units_per_lookup + u];
+        }
+#pragma unroll
+        for (int k = 0; k < kPlaneRows; ++k) {
+            if (r0 + k >= p.rows) break;
+            const float x[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+            __align__(8) __nv_bfloat16 q[3][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) split3(x[i], q[0][i], q[1][i], q[2][i]);
+            __nv_bfloat16* o = p.out3 + (r0 + k) * (3 * p.Kp) + 4 * c;
+#pragma unroll
+            for (int s = 0; s < 3; ++s) *reinterpret_cast<uint2*>(o + s * p.Kp) = *reinterpret_cast<const uint2*>(q[s]);
+        }
+    }
+}
+
 }  // namespace
 }  // namespace xg
+
+extern "C" int xg_gather_planes(const void* src, int64_t src_ld, const int64_t* starts, const int64_t* lens, int64_t nslices,
+                                const void* const* tables, const int64_t* table_rows, int64_t F, const int64_t* idx,
+                                int64_t idx_row_stride, int64_t idx_col_stride, const uint8_t* row_mask, int mask_zero_when,
+                                void* out3, int64_t rows, int64_t D, void* stream) {
+    using namespace xg;
+    if (rows < 0 || nslices < 0 || F < 0 || D < 0) return fail(XG_ERR_INVALID_ARG, "xg_gather_planes: negative extent");
+    if (rows == 0) return XG_OK;
+    if (!out3 || (nslices > 0 && (!src || !starts || !lens)) || (F > 0 && (!tables || !table_rows || !idx)))
+        return fail(XG_ERR_INVALID_ARG, "xg_gather_planes: null pointer");
+    if (nslices > kMaxSegs || F > kMaxSegs) return fail(XG_ERR_UNSUPPORTED, "xg_gather_planes: more than %d slices or tables", kMaxSegs);
+    if (D % 4 != 0 || !aligned16(src) || src_ld % 4 != 0 || !aligned16(out3))
+        return fail(XG_ERR_UNSUPPORTED, "xg_gather_planes: rows must be 16-byte addressable");
+    PlanesParams p;
+    int64_t units = 0;
+    p.nslices = 0;
+    for (int64_t k = 0; k < nslices; ++k) {
+        if (starts[k] < 0 || lens[k] < 0 || (rows > 1 && starts[k] + lens[k] > src_ld))
+            return fail(XG_ERR_INVALID_ARG, "xg_gather_planes: slice %lld is outside its row", (long long)k);
+        if (starts[k] % 4 != 0 || lens[k] % 4 != 0 || starts[k] > 0x7fffffffLL || units + lens[k] / 4 > kPlaneMaxSliceUnits)
+            return fail(XG_ERR_UNSUPPORTED, "xg_gather_planes: slices must be whole units of four columns, %d units at most", kPlaneMaxSliceUnits);
+        if (lens[k] == 0) continue;
+        p.start[p.nslices] = (int32_t)(starts[k] / 4);
+        p.unit_start[p.nslices++] = (int32_t)units;
+        units += lens[k] / 4;
+    }
+    for (int64_t f = 0; f < F; ++f) {
+        if (!tables[f] || table_rows[f] < 0) return fail(XG_ERR_INVALID_ARG, "xg_gather_planes: bad table %lld", (long long)f);
+        if (!aligned16(tables[f]) || table_rows[f] > 0x7fffffffLL) return fail(XG_ERR_UNSUPPORTED, "xg_gather_planes: table %lld", (long long)f);
+        p.table[f] = reinterpret_cast<const float*>(tables[f]);
+        p.table_rows[f] = (int32_t)table_rows[f];
+    }
+    const int64_t K = 4 * units + F * D;
+    if (K == 0) return XG_OK;
+    if (D > 0x1000000LL) return fail(XG_ERR_TOO_LARGE, "xg_gather_planes: row too wide");
+    p.src = reinterpret_cast<const float*>(src);
+    p.src_ld = src_ld;
+    p.idx = idx;
+    p.idx_rs = idx_row_stride;
+    p.idx_cs = idx_col_stride;
+    p.mask = row_mask;
+    p.zero_when = mask_zero_when;
+    p.out3 = reinterpret_cast<__nv_bfloat16*>(out3);
+    p.rows = rows;
+    p.Kp = xg_gemm_f32x3_padded_k(K);
+    p.slice_units = (int32_t)units;
+    p.F = D > 0 ? (int32_t)F : 0;
+    p.units_per_lookup = D > 0 ? (int32_t)(D / 4) : 1;
+    const int64_t grid = (rows + kPlaneRows - 1) / kPlaneRows;
+    if (grid > 0x7fffffffLL) return fail(XG_ERR_TOO_LARGE, "xg_gather_planes: too many rows");
+    // a row's units in equal steps: 432 of them are two steps of 216 threads (224), not one and a half of 256
+    const int64_t steps = (p.Kp / 4 + kCopyThreads - 1) / kCopyThreads;
+    const unsigned threads = (unsigned)(((p.Kp / 4 + steps - 1) / steps + 31) / 32 * 32);
+    launch(gather_planes_kernel, (unsigned)grid, threads, 0, reinterpret_cast<cudaStream_t>(stream), p);
+    return check_launch("xg_gather_planes");
+}
 
 extern "C" int xg_seg_copy(const void* const* src_ptrs, void* const* dst_ptrs, const int64_t* src_ld_bytes,
                            const int64_t* dst_ld_bytes, const int64_t* len_bytes, int64_t nseg, int64_t rows,

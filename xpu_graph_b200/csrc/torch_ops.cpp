@@ -951,29 +951,81 @@ Tensor decoder_layer(const Tensor& x, const Tensor& cos, const Tensor& sin, at::
     return linear(g, w[8], x1).view({B, S, C});
 }
 
-// Slices of the dense features and the masked lookups side by side in one buffer, then the dense layers (ReLU).
+// The fp32 input of a recommender's first layer - slices of the features, then the masked lookups - as that layer's three bf16
+// planes, in one kernel. Undefined where the inputs are not what the kernel takes (whole 16-byte units throughout); they then
+// go through slice_cat, gather_stack and cat_lastdim, which also report what is wrong with them.
+Tensor recommender_planes(const Tensor& features, const Tensor& idx, const Tensor& mask, at::TensorList tables, at::IntArrayRef starts,
+                          at::IntArrayRef ends, int64_t* K) {
+    const int64_t F = (int64_t)tables.size();
+    if (features.dim() != 2 || features.scalar_type() != at::kFloat || (features.size(1) > 1 && features.stride(1) != 1) || F < 1 || F > 64 || starts.size() > 64 ||
+        starts.size() != ends.size() || idx.dim() != 2 || idx.size(1) != F || idx.scalar_type() != at::kLong)
+        return {};
+    const int64_t rows = features.size(0), ld = row_stride(features), D = tables[0].dim() == 2 ? tables[0].size(1) : 0;
+    auto aligned = [](const Tensor& t) { return (reinterpret_cast<uintptr_t>(ptr(t)) & 15u) == 0; };
+    if (features.numel() == 0 || idx.size(0) != rows || mask.numel() != rows || D == 0 || D % 4 != 0 || D > 1 << 20 || ld % 4 != 0 || !aligned(features)) return {};
+    Buf<const void*> ptrs;
+    Buf<int64_t> table_rows, first, len;
+    for (const Tensor& t : tables) {
+        if (t.dim() != 2 || t.size(1) != D || t.scalar_type() != at::kFloat || !t.is_contiguous() || !aligned(t) || t.size(0) > 0x7fffffff ||
+            t.numel() == 0)
+            return {};
+        ptrs.push_back(ptr(t));
+        table_rows.push_back(t.size(0));
+    }
+    int64_t cols = 0;
+    for (const auto& s : clamp_slices(features.size(1), starts, ends)) {
+        if (s.first % 4 != 0 || s.second % 4 != 0) return {};
+        first.push_back(s.first);
+        len.push_back(s.second - s.first);
+        cols += s.second - s.first;
+    }
+    if (cols > 4096 || (rows > 1 && ld < features.size(1))) return {};
+    *K = cols + F * D;
+    const On on(features);
+    const Tensor hide = mask_bytes(mask, rows);
+    Tensor out = new_tensor({rows, 3 * xg_gemm_f32x3_padded_k(*K)}, at::kBFloat16, features);
+    XG_CALL(xg_gather_planes, ptr(features), ld, first.data(), len.data(), (int64_t)first.size(), ptrs.data(), table_rows.data(), F,
+            static_cast<const int64_t*>(ptr(idx)), idx.stride(0), idx.stride(1), static_cast<const uint8_t*>(ptr(hide)), 1, mut(out), rows, D,
+            on.stream);
+    return out;
+}
+
+// Slices of the dense features and the masked lookups side by side in one buffer, then the dense layers (ReLU). Neighbouring
+// layers on the tensor cores hand their result over as bf16 planes.
 Tensor recommender(const Tensor& features, const Tensor& idx, const Tensor& mask, at::TensorList tables, at::IntArrayRef starts,
                    at::IntArrayRef ends, at::TensorList weights, const c10::List<optional<Tensor>>& biases) {
     at::AutoDispatchBelowADInplaceOrView no_grad;
     TORCH_CHECK_VALUE(!weights.empty() && biases.size() == weights.size(), "xg_sm100::recommender: one bias entry per weight");
-    Tensor h = cat_lastdim({slice_cat(features, starts, ends, std::nullopt, false), gather_stack(tables, idx, mask, true)}, std::nullopt, false);
-    const int64_t M = h.size(0);
-    bool tower = h.scalar_type() == at::kFloat;
-    int64_t k = h.size(1);
-    for (const Tensor& w : weights) {
-        tower = tower && f32_on_tensor_cores(M, w.size(0), k);
-        k = w.size(0);
-    }
-    if (tower) {
-        c10::List<bool> trans;
-        std::string acts;
-        for (size_t i = 0; i < weights.size(); ++i) {
-            trans.push_back(true);
-            acts += i ? ",relu" : "relu";
+    const int64_t M = features.dim() == 2 ? features.size(0) : 0;
+    auto on_tensor_cores = [&](size_t i, int64_t k) {
+        return i < weights.size() && weights[i].dim() == 2 && weights[i].scalar_type() == at::kFloat && weights[i].size(1) == k &&
+               f32_on_tensor_cores(M, weights[i].size(0), k);
+    };
+    size_t i = 0;
+    Tensor h;
+    int64_t k = 0;
+    // (the first weight's own width stands for the assembled row's: it has to be that)
+    if (on_tensor_cores(0, weights[0].dim() == 2 ? weights[0].size(1) : 0))
+        h = recommender_planes(features, idx, mask, tables, starts, ends, &k);
+    if (h.defined()) {
+        TORCH_CHECK_VALUE(weights[0].size(1) == k, "xg_sm100::dense: inner dimensions differ");
+        const On on(features);
+        for (bool planes = true; planes; ++i) {
+            const int64_t N = weights[i].size(0);
+            const Tensor w = unit_rows(weights[i]);
+            const Tensor w3 = weight_planes(w, true, N, k, on.stream);
+            const auto b = biases.get(i);
+            const Tensor bias = b ? cast(*b, at::kFloat).contiguous() : Tensor();
+            planes = on_tensor_cores(i + 1, N);
+            Tensor out = planes ? new_tensor({M, 3 * xg_gemm_f32x3_padded_k(N)}, at::kBFloat16, h) : new_tensor({M, N}, at::kFloat, h);
+            XG_CALL(xg_gemm_f32x3, ptr(h), ptr(w3), ptr(bias), nullptr, mut(out), M, N, k, N, 0, act_code("relu"), planes ? 1 : 0, on.stream);
+            h = out;
+            k = N;
         }
-        return dense_tower(h, weights, trans, biases, acts);
+    } else {
+        h = cat_lastdim({slice_cat(features, starts, ends, std::nullopt, false), gather_stack(tables, idx, mask, true)}, std::nullopt, false);
     }
-    for (size_t i = 0; i < weights.size(); ++i) h = dense(h, weights[i], true, biases.get(i), std::nullopt, "relu");
+    for (; i < weights.size(); ++i) h = dense(h, weights[i], true, biases.get(i), std::nullopt, "relu");
     return h;
 }
 

@@ -86,6 +86,8 @@ SIGNATURES = {
     "xg_rowsum_cat": (c_int, [_VPP, _VPP, _I64P, _I64P, _I64P, c_int64, c_int64, c_int64, c_void_p, c_int64, c_int, c_void_p]),
     "xg_gather_rows": (c_int, [_VPP, _I64P, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_int, c_void_p, c_int64,
                                c_int64, c_int64, c_int, c_void_p]),
+    "xg_gather_planes": (c_int, [c_void_p, c_int64, _I64P, _I64P, c_int64, _VPP, _I64P, c_int64, c_void_p, c_int64, c_int64, c_void_p,
+                                 c_int, c_void_p, c_int64, c_int64, c_void_p]),
 }
 
 _lock = threading.Lock()
