@@ -297,6 +297,16 @@ int xg_gemm_swiglu(const void* A, const void* Wg, const void* Wu, void* out, int
 int xg_gemm_rope(const void* A, const void* W, const void* cos, const void* sin, void* out, int64_t M, int64_t N,
                  int64_t K, int64_t lda, int64_t ldw, int64_t ldc, int64_t S, int64_t D, int dtype, void* stream);
 
+/*
+ * `count` (at most 12) bias-free layers of one input in one launch: out[e] = A @ W[e]^T, all [N, K], the first rope_entries
+ * of them with xg_gemm_rope's rotary epilogue (q, k and v of one hidden state). W, out: HOST arrays of device pointers; one
+ * ldw and one ldc. xg_gemm_rope_group_worth_it: 1 where one launch is the faster way (layers that do not fill the chip).
+ */
+int xg_gemm_rope_group(const void* A, const void* const* W, const void* cos, const void* sin, void* const* out,
+                       int64_t count, int64_t rope_entries, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldw,
+                       int64_t ldc, int64_t S, int64_t D, int dtype, void* stream);
+int xg_gemm_rope_group_worth_it(int64_t count, int64_t M, int64_t N, int64_t K);
+
 /* ---- attention ------------------------------------------------------------------------- */
 
 /*

@@ -904,3 +904,32 @@ def test_f32x3_few_tiles(cuda_device, M, N, K):
     assert (parts[:, :, N:] == 0).all()
     for got, want in zip(parts[:, :, :N].unbind(1), _planes(parts.sum(1)[:, :N])):
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K,S,D", [(1, 512, 512, 1, 128), (130, 576, 264, 65, 64), (333, 4096, 1024, 333, 128), (700, 1024, 520, 100, 128)])
+def test_rope_group(cuda_device, M, N, K, S, D, dtype):
+    """q, k and v of one hidden state in one launch: the same bits as one launch each (either tile width accumulates a row of
+    k-blocks in the same order)."""
+    import ctypes
+
+    from xpu_graph_b200 import lib
+
+    L = lib.load()
+    g = torch.Generator().manual_seed(91)
+    x = torch.randn(M, K, generator=g).to(dtype).to(cuda_device)
+    ws = [(torch.randn(N, K, generator=g) * K ** -0.5).to(dtype).to(cuda_device) for _ in range(3)]
+    cos, sin = (torch.randn(S, D, generator=g).to(dtype).to(cuda_device) for _ in range(2))
+    outs = [torch.full((M, N), 7.0, dtype=dtype, device=cuda_device) for _ in range(3)]
+    code = 1 if dtype == torch.bfloat16 else 2
+    rc = L.xg_gemm_rope_group(x.data_ptr(), lib.ptr_array([w.data_ptr() for w in ws]), cos.data_ptr(), sin.data_ptr(),
+                              lib.ptr_array([o.data_ptr() for o in outs]), 3, 2, M, N, K, K, K, N, S, D, code,
+                              ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0, lib.last_error()
+    X = torch.ops.xg_sm100
+    want = [X.dense_rope(x, w, cos, sin, S, D) for w in ws[:2]]
+    torch.cuda.synchronize()
+    assert lib.tc_status() == 0
+    for got, w in zip(outs, want):
+        assert torch.equal(got, w)
+    assert_parity(outs[2], ref_ops.dense(x.cpu(), ws[2].cpu(), True, None, "none"), f"rope group v {M}x{N}x{K}")

@@ -19,6 +19,10 @@ int gemm_swiglu_entry(const void* A, const void* Wg, const void* Wu, void* out, 
                       int64_t lda, int64_t ldw, int64_t ldc, int dtype, cudaStream_t st);
 int gemm_rope_entry(const void* A, const void* W, const void* cos, const void* sin, void* out, int64_t M, int64_t N, int64_t K,
                     int64_t lda, int64_t ldw, int64_t ldc, int64_t S, int64_t D, int dtype, cudaStream_t st);
+int gemm_rope_group_entry(const void* A, const void* const* W, const void* cos, const void* sin, void* const* out, int64_t count,
+                          int64_t rope_entries, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldw, int64_t ldc, int64_t S, int64_t D,
+                          int dtype, cudaStream_t st);
+int64_t gemm_rope_group_worth_it(int64_t count, int64_t M, int64_t N, int64_t K);
 int gemm_f32x3_entry(const void* A3, const void* W3, const void* bias, const void* residual, void* out, int64_t M,
                      int64_t N, int64_t Kp, int64_t ldc, int64_t ldr, int act, int out_planes, cudaStream_t st);
 bool bgemm_single_launch_ok(const void* A, const void* B, int64_t batch, int64_t M, int64_t N, int64_t K, int64_t lda,
@@ -244,6 +248,21 @@ extern "C" int xg_gemm_rope(const void* A, const void* W, const void* cos, const
     if (dtype != XG_BF16 && dtype != XG_F16) return fail(XG_ERR_UNSUPPORTED, "xg_gemm_rope: 16-bit dtypes only");
     if (lda < K || ldw < K || ldc < N) return fail(XG_ERR_INVALID_ARG, "xg_gemm_rope: leading dimension too small");
     return gemm_rope_entry(A, W, cos, sin, out, M, N, K, lda, ldw, ldc, S, D, dtype, reinterpret_cast<cudaStream_t>(stream));
+}
+
+extern "C" int xg_gemm_rope_group_worth_it(int64_t count, int64_t M, int64_t N, int64_t K) {
+    return xg::gemm_rope_group_worth_it(count, M, N, K) ? 1 : 0;
+}
+
+extern "C" int xg_gemm_rope_group(const void* A, const void* const* W, const void* cos, const void* sin, void* const* out, int64_t count,
+                                  int64_t rope_entries, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldw, int64_t ldc, int64_t S,
+                                  int64_t D, int dtype, void* stream) {
+    using namespace xg;
+    if (!A || !W || !cos || !sin || !out) return fail(XG_ERR_INVALID_ARG, "xg_gemm_rope_group: null pointer");
+    if (M < 0 || N < 0 || K <= 0 || rope_entries < 0 || rope_entries > count) return fail(XG_ERR_INVALID_ARG, "xg_gemm_rope_group: bad extents");
+    if (lda < K || ldw < K || ldc < N) return fail(XG_ERR_INVALID_ARG, "xg_gemm_rope_group: leading dimension too small");
+    if (dtype != XG_BF16 && dtype != XG_F16) return fail(XG_ERR_UNSUPPORTED, "xg_gemm_rope_group: 16-bit types only");
+    return gemm_rope_group_entry(A, W, cos, sin, out, count, rope_entries, M, N, K, lda, ldw, ldc, S, D, dtype, reinterpret_cast<cudaStream_t>(stream));
 }
 
 extern "C" int xg_gemm_f32x3(const void* A3, const void* W3, const void* bias, const void* residual, void* out, int64_t M,

@@ -915,7 +915,7 @@ struct GroupTable {
 
 template <typename T, int BN, bool B_MN>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_tc_group_kernel(const __grid_constant__ GroupTable tab, const GemmParams p, const int count) {
+gemm_tc_group_kernel(const __grid_constant__ GroupTable tab, const GemmParams p, const int count, const int rope_entries) {
     using Cfg = GemmCfg<BN>;
     constexpr int STAGES = Cfg::STAGES;
     extern __shared__ uint8_t smem_raw[];
@@ -1048,6 +1048,7 @@ gemm_tc_group_kernel(const __grid_constant__ GroupTable tab, const GemmParams p,
             pe.out = tab.out[entry];
             pe.bias = tab.bias[entry];
             pe.residual = tab.resid[entry];
+            pe.mode = entry < rope_entries ? kModeRope : kModePlain;
             const int64_t row = (int64_t)mb * BM + quad * 32 + lane;
             epilogue_tile<T, BN, false>(pe, tmem_base, acc, quad, row, row < p.M, nb, 0, 0);
             ptx::tc_fence_before();
@@ -1066,14 +1067,14 @@ gemm_tc_group_kernel(const __grid_constant__ GroupTable tab, const GemmParams p,
 }
 
 template <typename T, int BN, bool B_MN>
-int launch_gemm_group(const GroupTable& tab, const GemmParams& p, int count, cudaStream_t st) {
+int launch_gemm_group(const GroupTable& tab, const GemmParams& p, int count, cudaStream_t st, int rope_entries = 0) {
     using Cfg = GemmCfg<BN>;
     auto kern = gemm_tc_group_kernel<T, BN, B_MN>;
     static std::atomic<uint64_t> reserved{0};
     if (!reserve_smem(kern, Cfg::SMEM_BYTES, reserved)) return fail(XG_ERR_LAUNCH, "xg_gemm_group_bias_act: cannot reserve %d bytes of shared memory", Cfg::SMEM_BYTES);
     const int64_t tiles = (int64_t)p.num_m_blocks * p.num_n_blocks * count;
     const int grid = (int)(tiles < num_sms() ? tiles : num_sms());
-    launch(kern, grid, kGemmThreads, Cfg::SMEM_BYTES, st, tab, p, count);
+    launch(kern, grid, kGemmThreads, Cfg::SMEM_BYTES, st, tab, p, count, rope_entries);
     return check_launch("xg_gemm_group_bias_act");
 }
 
@@ -1528,6 +1529,92 @@ int gemm_tc_static_entry(const void* A, const void* B, const void* bias, const v
     if (rc != XG_OK) return rc;
     return gemm_tc_entry(A, B, bias, residual, out, M, N, K, lda, ldb, ldc, ldr, trans_b, act, dtype, scratch,
                          kStaticScratchBytes, st, /*force_split=*/true);
+}
+
+// Whether `count` layers of one input, some with the rotary epilogue, run faster as one launch of the grouped kernel than one
+// after the other, and with which tile width. A single layer with less than a wave of tiles leaves SMs idle and pays for its
+// ramp alone. Microseconds as in plan_gemm: a tile takes in (128 + bn) rows of 128 bytes per k-block at about 118 KB/us,
+// 3 us per launch; the line lies where the model sees 5 %. Measured (K = N = 4096 bf16, three layers, two with RoPE, weights not
+// in L2; one launch / three): 16 rows 24.0 / 49.9 us, 128 rows 28.0 / 60.7, 333 rows 41.7 / 66.4, 512 rows 53.5 / 66.5, 1000 rows
+// 88.1 / 102.5, 2048 rows 180.5 / 176.8; K = N = 512: 16 rows 7.0 / 20.4, 1000 rows 9.8 / 25.6. Layers that fill the chip
+// with 256-row tiles by themselves stay with the CTA-pair kernel.
+static int plan_rope_group(int64_t count, int64_t M, int64_t N, int64_t K) {
+    if (count < 2 || count > kGroupMax || use_cta_pairs(M, N, 256)) return 0;
+    const int64_t sms = num_sms(), mblk = (M + BM - 1) / BM, nkb = (K + BK - 1) / BK;
+    auto cost = [&](int64_t layers, int bn) {
+        const int64_t tiles = layers * mblk * ((N + bn - 1) / bn);
+        return (double)((tiles + sms - 1) / sms) * (double)nkb * (16.0 + bn * 0.125) / 118.0 + 3.0;
+    };
+    const int single = plan_gemm(M, N, K, 0, (int)sms).bn;
+    const double apart = (double)count * cost(1, single < 128 ? 128 : single);
+    const int bn = cost(count, 128) < cost(count, 256) ? 128 : 256;
+    return cost(count, bn) < 0.95 * apart ? bn : 0;
+}
+
+int64_t gemm_rope_group_worth_it(int64_t count, int64_t M, int64_t N, int64_t K) {
+    return M > 0 && N > 0 && K > 0 && plan_rope_group(count, M, N, K) != 0;
+}
+
+// out[e] = A @ W[e]^T, the first rope_entries of them with the rotary epilogue (q, k, v of one hidden state in one launch).
+template <typename T>
+static int gemm_rope_group_dispatch(const void* A, const void* const* W, const void* cos, const void* sin, void* const* out, int64_t count,
+                                    int64_t rope_entries, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldw, int64_t ldc, int64_t S,
+                                    int64_t D, cudaStream_t st) {
+    constexpr bool is_bf16 = std::is_same<T, __nv_bfloat16>::value;
+    int bn = plan_rope_group(count, M, N, K);
+    if (bn == 0) bn = 128;
+    GroupTable tab;
+    GemmParams p;
+    p.out = nullptr;
+    p.bias = nullptr;
+    p.residual = nullptr;
+    p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.ldr = 0;
+    p.act = XG_ACT_NONE;
+    p.mode = kModeRope;
+    p.rope.cos = cos;
+    p.rope.sin = sin;
+    p.rope.S = S;
+    p.rope.D = (int)D;
+    p.num_m_blocks = (int)((M + BM - 1) / BM);
+    p.num_n_blocks = (int)((N + bn - 1) / bn);
+    p.num_k_blocks = (int)((K + BK - 1) / BK);
+    p.splits = 1;
+    p.vec_ok = 1;
+    p.bias_vec_ok = 0;
+    if (!make_tmap_2d_16bit(&tab.a[0], A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BM, BK, is_bf16))
+        return fail(XG_ERR_UNSUPPORTED, "xg_gemm_rope_group: tensor-map encoding failed for A");
+    for (int e = 0; e < kGroupMax; ++e) {  // unused slots: valid descriptors, never dereferenced
+        tab.a[e] = tab.a[0];
+        if (e < count && !make_tmap_2d_16bit(&tab.w[e], W[e], (uint64_t)N, (uint64_t)K, (uint64_t)ldw, (uint32_t)bn, BK, is_bf16))
+            return fail(XG_ERR_UNSUPPORTED, "xg_gemm_rope_group: tensor-map encoding failed for entry %d", e);
+        if (e >= count) tab.w[e] = tab.w[0];
+        tab.out[e] = e < count ? out[e] : nullptr;
+        tab.bias[e] = nullptr;
+        tab.resid[e] = nullptr;
+    }
+    return bn == 256 ? launch_gemm_group<T, 256, false>(tab, p, (int)count, st, (int)rope_entries)
+                     : launch_gemm_group<T, 128, false>(tab, p, (int)count, st, (int)rope_entries);
+}
+
+int gemm_rope_group_entry(const void* A, const void* const* W, const void* cos, const void* sin, void* const* out, int64_t count,
+                          int64_t rope_entries, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldw, int64_t ldc, int64_t S, int64_t D,
+                          int dtype, cudaStream_t st) {
+    if (count < 1 || count > kGroupMax) return fail(XG_ERR_UNSUPPORTED, "xg_gemm_rope_group: 1 to %d layers", kGroupMax);
+    if (D != 64 && D != 128) return fail(XG_ERR_UNSUPPORTED, "xg_gemm_rope_group: head_dim must be 64 or 128");
+    if (N % D != 0 || S <= 0) return fail(XG_ERR_INVALID_ARG, "xg_gemm_rope_group: N must be a multiple of head_dim and S positive");
+    bool ok = aligned16(A) && aligned16(cos) && aligned16(sin) && lda % 8 == 0 && ldw % 8 == 0 && ldc % 8 == 0;
+    for (int64_t e = 0; e < count; ++e) {
+        if (!W[e] || !out[e]) return fail(XG_ERR_INVALID_ARG, "xg_gemm_rope_group: null pointer in entry %lld", (long long)e);
+        ok = ok && aligned16(W[e]) && aligned16(out[e]);
+    }
+    if (!ok) return fail(XG_ERR_UNSUPPORTED, "xg_gemm_rope_group: operands, tables and output rows must be 16-byte addressable");
+    if (M * N == 0) return XG_OK;
+    if (M > (int64_t)BM * 0x7fffff || N > (int64_t)64 * 0x7fffff || K > 0x7fffffff ||
+        count * ((M + BM - 1) / BM) * ((N + 127) / 128) > 0x7fffffffLL)
+        return fail(XG_ERR_TOO_LARGE, "xg_gemm_rope_group: extent too large");
+    return dtype == XG_BF16
+               ? gemm_rope_group_dispatch<__nv_bfloat16>(A, W, cos, sin, out, count, rope_entries, M, N, K, lda, ldw, ldc, S, D, st)
+               : gemm_rope_group_dispatch<__half>(A, W, cos, sin, out, count, rope_entries, M, N, K, lda, ldw, ldc, S, D, st);
 }
 
 int gemm_rope_entry(const void* A, const void* W, const void* cos, const void* sin, void* out, int64_t M, int64_t N, int64_t K,

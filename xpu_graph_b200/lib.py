@@ -71,6 +71,9 @@ SIGNATURES = {
                                c_int64, c_int, c_void_p]),
     "xg_gemm_rope": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_int64,
                              c_int64, c_int64, c_int64, c_int, c_void_p]),
+    "xg_gemm_rope_group": (c_int, [c_void_p, _VPP, c_void_p, c_void_p, _VPP, c_int64, c_int64, c_int64, c_int64, c_int64, c_int64,
+                                   c_int64, c_int64, c_int64, c_int64, c_int, c_void_p]),
+    "xg_gemm_rope_group_worth_it": (c_int, [c_int64, c_int64, c_int64, c_int64]),
     "xg_sdpa_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64,
                             c_int64, _I64P, _I64P, _I64P, _I64P, _I64P, c_float, c_int, c_int, c_void_p]),
     "xg_sdpa_fwd_ws": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64,
@@ -174,7 +177,7 @@ def tc_status(reset: bool = True) -> int:
 
 # entry points that enqueue no kernel (queries and status reads)
 QUERY_ENTRY_POINTS = frozenset({"xg_version", "xg_device_arch_ok", "xg_last_error", "xg_tc_status", "xg_gemm_workspace_bytes", "xg_gemm_copy_bytes",
-                                "xg_sdpa_workspace_bytes",
+                                "xg_sdpa_workspace_bytes", "xg_gemm_rope_group_worth_it",
                                 "xg_gemm_static_scratch_bytes", "xg_gemm_f32x3_padded_k", "xg_gemm_cluster_plan",
                                 "xg_mlp2_supported", "xg_mlp3_supported", "xg_mlp_small_supported"})
 
