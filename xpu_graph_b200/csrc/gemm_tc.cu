@@ -7,8 +7,10 @@
 //   warp 1      : MMA issuer    - one elected thread issues tcgen05.mma (128 x BN x 16) straight from
 //                 shared memory into one of two TMEM accumulator buffers; tcgen05.commit releases the
 //                 ring stage and, after the last k-block, publishes the accumulator;
-//   warps 2..5  : epilogue      - tcgen05.ld the accumulator (each warp owns its 32-lane TMEM quadrant),
-//                 add bias / residual, apply the activation, convert and store, then hand the TMEM
+//   warps 2..9  : epilogue      - tcgen05.ld the accumulator (two warps per 32-lane TMEM quadrant share out its
+//                 32-column chunks: a chunk is a chain of latencies - TMEM, bias, residual, store - and with a warp per
+//                 quadrant the epilogue, not the products, bounded layers of short K: 16384 x 512 x 2048 bf16 with GELU
+//                 89.6 -> 63.8 us, 4728 x 256 x 1024 26.2 -> 19.6, 8192-row layers of K = 4096 unchanged), add bias / residual, apply the activation, convert and store, then hand the TMEM
 //                 buffer back. The second accumulator buffer lets tile i's epilogue overlap tile i+1's
 //                 main loop.
 // Tiles are visited in groups of 16 row-blocks so that the ~148 tiles in flight share A and W tiles in L2.
@@ -118,7 +120,9 @@ namespace {
 constexpr int BM = 128;
 constexpr int BK = 64;       // 64 x 16-bit = one 128-byte swizzled row
 constexpr int UMMA_K = 16;
-constexpr int kGemmThreads = 192;
+constexpr int kEpiWarps = 8;             // two per TMEM lane quadrant
+constexpr int kEpiParts = kEpiWarps / 4;
+constexpr int kGemmThreads = 64 + kEpiWarps * 32;
 constexpr int GROUP_M = 16;
 
 // Scalar kernel parameters. The struct is kept at 128 bytes: next to three tensor maps the parameter block is then
@@ -233,11 +237,11 @@ __device__ __forceinline__ void tile_coords(int t, int num_m, int num_n, int& mb
     nb = in_g / gsz;
 }
 
-// One warp's share of a finished accumulator tile: its 32 TMEM lanes (rows), all output columns of the tile in
-// chunks of 32: TMEM -> registers -> (+bias, +residual, activation | SwiGLU | raw split-K partials) -> global.
+// One warp's share of a finished accumulator tile: its 32 TMEM lanes (rows), every kEpiParts-th of the tile's 32-column
+// chunks, beginning with chunk `part`: TMEM -> registers -> (+bias, +residual, activation | SwiGLU | raw split-K partials) -> global.
 // Warp-collective (tcgen05.ld): all 32 lanes call it, rows past M only skip the stores.
 template <typename T, int BN, bool SWIGLU>
-__device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t tmem_base, int acc, int quad, int64_t row,
+__device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t tmem_base, int acc, int quad, int part, int64_t row,
                                               bool row_ok, int nb, int split, int entry = 0) {
     constexpr int OUT_BN = SWIGLU ? BN / 2 : BN;
     T* out = reinterpret_cast<T*>(p.out);
@@ -258,9 +262,8 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t tmem
         const T* cosr = reinterpret_cast<const T*>(p.rope.cos) + pos * D;
         const T* sinr = reinterpret_cast<const T*>(p.rope.sin) + pos * D;
 #pragma unroll 1
-        for (int c = 0; c < OUT_BN / 32; ++c) {
-            const int in_head = c % (2 * half_chunks);
-            if (in_head >= half_chunks) continue;  // second half: handled with its partner below
+        for (int i = part; i < OUT_BN / 64; i += kEpiParts) {  // chunks of first halves, each with its partner
+            const int c = half_chunks == 1 ? 2 * i : 4 * (i >> 1) + (i & 1);
             const int64_t col0 = (int64_t)nb * OUT_BN + c * 32;
             if (col0 >= p.N) break;
             const int c2 = c + half_chunks;
@@ -294,7 +297,7 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t tmem
         return;
     }
 #pragma unroll 1
-    for (int c = 0; c < OUT_BN / 32; ++c) {
+    for (int c = part; c < OUT_BN / 32; c += kEpiParts) {
         const int64_t col0 = (int64_t)nb * OUT_BN + c * 32;
         if (col0 >= (f32_mode == 2 ? p.f32.out_kp : p.N)) break;  // warp-uniform
         uint32_t r[32];
@@ -459,7 +462,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         }
         for (int a = 0; a < 2; ++a) {
             ptx::mbar_init(&tmem_full[a], 1);
-            ptx::mbar_init(&tmem_empty[a], 4);
+            ptx::mbar_init(&tmem_empty[a], kEpiWarps);
         }
         ptx::mbar_init(drain_bar, 1);
         *abort_flag = 0;
@@ -608,7 +611,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             ptx::tc_fence_after();
             const int64_t row = (int64_t)mb * BM + quad * 32 + lane;
             const bool row_ok = row < p.M;
-            epilogue_tile<T, BN, SWIGLU>(p, tmem_base, acc, quad, row, row_ok, nb, t % p.splits, entry);
+            epilogue_tile<T, BN, SWIGLU>(p, tmem_base, acc, quad, (warp - 2) >> 2, row, row_ok, nb, t % p.splits, entry);
             // All of this warp's TMEM reads are complete (wait::ld above): return the buffer.
             ptx::tc_fence_before();
             __syncwarp();
@@ -635,7 +638,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 // (two accumulator buffers), and each CTA's epilogue warps store their own rows.
 // Barriers: "full" lives in the leader only and counts the bytes of both CTAs' loads; "empty" and "accumulator full"
 // exist in both CTAs and are signalled by the leader's tcgen05.commit (one commit per CTA, no multicast);
-// "accumulator empty" lives in the leader and collects the 8 epilogue warps of the pair.
+// "accumulator empty" lives in the leader and collects the epilogue warps of the pair.
 // ---------------------------------------------------------------------------------------------------------
 constexpr int PAIR_BN = 256;
 constexpr int PAIR_STAGES = 6;
@@ -658,7 +661,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     uint64_t* full_bar = bars;                     // [STAGES]  (used in the leader)
     uint64_t* empty_bar = bars + STAGES;           // [STAGES]  (each CTA its own)
     uint64_t* tmem_full = bars + 2 * STAGES;       // [2]       (each CTA its own)
-    uint64_t* tmem_empty = bars + 2 * STAGES + 2;  // [2]       (used in the leader, 8 arrivals)
+    uint64_t* tmem_empty = bars + 2 * STAGES + 2;  // [2]       (used in the leader, both CTAs' epilogue warps arrive)
     uint64_t* drain_bar = bars + 2 * STAGES + 4;   // [1]
     uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 5);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
@@ -676,7 +679,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         }
         for (int a = 0; a < 2; ++a) {
             ptx::mbar_init(&tmem_full[a], 1);
-            ptx::mbar_init(&tmem_empty[a], 8);
+            ptx::mbar_init(&tmem_empty[a], 2 * kEpiWarps);
         }
         ptx::mbar_init(drain_bar, 1);
         *abort_flag = 0;
@@ -781,7 +784,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             if (!__all_sync(0xffffffffu, ptx::mbar_wait_bounded(&tmem_full[acc], acc_phase, abort_flag))) { ok = false; break; }
             ptx::tc_fence_after();
             const int64_t row = (int64_t)mb * 256 + (int64_t)rank * BM + quad * 32 + lane;
-            epilogue_tile<T, BN, SWIGLU>(p, tmem_base, acc, quad, row, row < p.M, nb, 0);
+            epilogue_tile<T, BN, SWIGLU>(p, tmem_base, acc, quad, (warp - 2) >> 2, row, row < p.M, nb, 0);
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive_cluster(ptx::map_to_cta(ptx::smem_u32(&tmem_empty[acc]), 0));
@@ -940,7 +943,7 @@ gemm_tc_group_kernel(const __grid_constant__ GroupTable tab, const GemmParams p,
         }
         for (int a = 0; a < 2; ++a) {
             ptx::mbar_init(&tmem_full[a], 1);
-            ptx::mbar_init(&tmem_empty[a], 4);
+            ptx::mbar_init(&tmem_empty[a], kEpiWarps);
         }
         ptx::mbar_init(drain_bar, 1);
         *abort_flag = 0;
@@ -1050,7 +1053,7 @@ gemm_tc_group_kernel(const __grid_constant__ GroupTable tab, const GemmParams p,
             pe.residual = tab.resid[entry];
             pe.mode = entry < rope_entries ? kModeRope : kModePlain;
             const int64_t row = (int64_t)mb * BM + quad * 32 + lane;
-            epilogue_tile<T, BN, false>(pe, tmem_base, acc, quad, row, row < p.M, nb, 0, 0);
+            epilogue_tile<T, BN, false>(pe, tmem_base, acc, quad, (warp - 2) >> 2, row, row < p.M, nb, 0, 0);
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&tmem_empty[acc]);
@@ -1162,7 +1165,7 @@ bool use_cta_pairs(int64_t M, int64_t N, int out_bn) {
 // cost model in microseconds fitted to sweeps on B200 (K = 4096; M = 16..128; N = 512..11008; tile widths 64 / 128 /
 // 256; 1..16 splits; CUDA-graph replay):
 //   ingest  : 8.5 us per MB a CTA takes in (about 118 KB/us per SM), times the waves;
-//   tile    : 0.01 us per tile column (the epilogue of a wide tile is served by the same four warps);
+//   tile    : 0.01 us per tile column (the epilogue of a wide tile is served by the same warps);
 //   launch  : 2.5 us;
 //   a split : 4 us more (second launch, drain) and the fp32 partial sums written and read back: 0.13 us per MB while
 //             weights + partial sums stay within L2, 0.67 us per MB beyond that.
