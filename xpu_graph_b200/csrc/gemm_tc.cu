@@ -1154,8 +1154,13 @@ bool use_cta_pairs(int64_t M, int64_t N, int out_bn) {
         return e ? (e[0] == '0' ? 0 : 1) : -1;
     }();
     if (forced >= 0) return forced == 1;
-    const int64_t tiles = ((M + 255) / 256) * ((N + out_bn - 1) / out_bn);
-    return tiles >= num_sms() / 2;  // measured on B200: +10 % (plain) / +8 % (SwiGLU) at 8192 x 4096 x 11008
+    const int64_t sms = num_sms(), nblk = (N + out_bn - 1) / out_bn, tiles = ((M + 255) / 256) * nblk;
+    if (tiles < sms / 2) return false;
+    // On full waves pairs are ahead: +10 % (plain) / +8 % (SwiGLU) at 8192 x 4096 x 11008. A last wave of few tiles costs them
+    // more than 128-row CTAs, which cut the rows finer: those take over where they need a quarter fewer waves. 4728 x 256 x 1024
+    // + GELU (two waves or one) 19.6 -> 11.7 us, the decoder layer on 333 rows (its SwiGLU: three or two) 204 -> 190 us.
+    const int64_t pair_waves = (tiles + sms / 2 - 1) / (sms / 2), cta_waves = (((M + BM - 1) / BM) * nblk + sms - 1) / sms;
+    return 5 * cta_waves >= 4 * pair_waves;
 }
 
 // Tile width and split-K factor for an [M, N, K] problem given `ws_bytes` of fp32 scratch (0 = none).
