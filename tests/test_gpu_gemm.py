@@ -933,3 +933,23 @@ def test_rope_group(cuda_device, M, N, K, S, D, dtype):
     for got, w in zip(outs, want):
         assert torch.equal(got, w)
     assert_parity(outs[2], ref_ops.dense(x.cpu(), ws[2].cpu(), True, None, "none"), f"rope group v {M}x{N}x{K}")
+
+
+@pytest.mark.parametrize("with_res", [True, False])
+@pytest.mark.parametrize("M,N,K", [
+    (4728, 1024, 256),   # two waves of 256-row tiles or one of 128-row ones: CTAs on their own
+    (4865, 1024, 256),   # 20 x 4 tiles and 39 x 4: two waves either way: pairs, short K
+    (4865, 1028, 1024),  # the longest K of the sixteen-warp epilogue, ragged columns (no 16-byte rows of the result)
+    (4865, 1024, 1032),  # just beyond it
+])
+def test_dense_epilogue_shares(cuda_device, M, N, K, with_res):
+    """Both sides of the lines between CTAs on their own and pairs, and between the pairs' epilogues of sixteen and eight warps."""
+    from xpu_graph_b200 import lib
+
+    x, w, b = _mk(M, K, N, torch.bfloat16, 95)
+    r = torch.randn(M, N, generator=torch.Generator().manual_seed(96)).bfloat16() if with_res else None
+    got = torch.ops.xg_sm100.dense(x.to(cuda_device), w.to(cuda_device), True, b.to(cuda_device), r.to(cuda_device) if with_res else None, "silu")
+    torch.cuda.synchronize()
+    assert lib.tc_status() == 0
+    y = x.float() @ w.float().t() + b.float()
+    assert_parity(got, ref_ops._ACTS["silu"](y + r.float() if with_res else y).bfloat16(), f"dense {M}x{K}x{N}")

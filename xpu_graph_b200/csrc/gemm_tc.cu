@@ -237,10 +237,10 @@ __device__ __forceinline__ void tile_coords(int t, int num_m, int num_n, int& mb
     nb = in_g / gsz;
 }
 
-// One warp's share of a finished accumulator tile: its 32 TMEM lanes (rows), every kEpiParts-th of the tile's 32-column
+// One warp's share of a finished accumulator tile: its 32 TMEM lanes (rows), every PARTS-th of the tile's 32-column
 // chunks, beginning with chunk `part`: TMEM -> registers -> (+bias, +residual, activation | SwiGLU | raw split-K partials) -> global.
 // Warp-collective (tcgen05.ld): all 32 lanes call it, rows past M only skip the stores.
-template <typename T, int BN, bool SWIGLU>
+template <typename T, int BN, bool SWIGLU, int PARTS>
 __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t tmem_base, int acc, int quad, int part, int64_t row,
                                               bool row_ok, int nb, int split, int entry = 0) {
     constexpr int OUT_BN = SWIGLU ? BN / 2 : BN;
@@ -262,7 +262,7 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t tmem
         const T* cosr = reinterpret_cast<const T*>(p.rope.cos) + pos * D;
         const T* sinr = reinterpret_cast<const T*>(p.rope.sin) + pos * D;
 #pragma unroll 1
-        for (int i = part; i < OUT_BN / 64; i += kEpiParts) {  // chunks of first halves, each with its partner
+        for (int i = part; i < OUT_BN / 64; i += PARTS) {  // chunks of first halves, each with its partner
             const int c = half_chunks == 1 ? 2 * i : 4 * (i >> 1) + (i & 1);
             const int64_t col0 = (int64_t)nb * OUT_BN + c * 32;
             if (col0 >= p.N) break;
@@ -297,7 +297,7 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t tmem
         return;
     }
 #pragma unroll 1
-    for (int c = part; c < OUT_BN / 32; c += kEpiParts) {
+    for (int c = part; c < OUT_BN / 32; c += PARTS) {
         const int64_t col0 = (int64_t)nb * OUT_BN + c * 32;
         if (col0 >= (f32_mode == 2 ? p.f32.out_kp : p.N)) break;  // warp-uniform
         uint32_t r[32];
@@ -611,7 +611,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             ptx::tc_fence_after();
             const int64_t row = (int64_t)mb * BM + quad * 32 + lane;
             const bool row_ok = row < p.M;
-            epilogue_tile<T, BN, SWIGLU>(p, tmem_base, acc, quad, (warp - 2) >> 2, row, row_ok, nb, t % p.splits, entry);
+            epilogue_tile<T, BN, SWIGLU, kEpiParts>(p, tmem_base, acc, quad, (warp - 2) >> 2, row, row_ok, nb, t % p.splits, entry);
             // All of this warp's TMEM reads are complete (wait::ld above): return the buffer.
             ptx::tc_fence_before();
             __syncwarp();
@@ -642,11 +642,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 // ---------------------------------------------------------------------------------------------------------
 constexpr int PAIR_BN = 256;
 constexpr int PAIR_STAGES = 6;
+// EPI_WARPS: sixteen where the products of a tile do not cover its epilogue (K <= 1024: 16384 x 512 x 2048 + GELU 63.9 -> 53.7 us,
+// with a residual 98.0 -> 81.2; 16384 x 1024 x 1024 41.6 -> 37.4), eight beyond, where more of them only take issue slots and
+// power (the fp32 planes of 16384 x 1728 x 1024 and 1024 x 512: 415 -> 440 us a recommender pass with sixteen).
+constexpr int kPairShortK = 1024 / BK;  // k-blocks
 constexpr int PAIR_STAGE_BYTES = (BM + PAIR_BN / 2) * BK * 2;  // per CTA: A tile + half of the W tile = 32 KiB
 constexpr int PAIR_SMEM_BYTES = PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + 256;
 
-template <typename T, bool SWIGLU>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
+template <typename T, bool SWIGLU, int EPI_WARPS>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + EPI_WARPS * 32, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const __grid_constant__ CUtensorMap tmap_b2, const GemmParams p) {
     constexpr int BN = PAIR_BN;
@@ -679,7 +683,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         }
         for (int a = 0; a < 2; ++a) {
             ptx::mbar_init(&tmem_full[a], 1);
-            ptx::mbar_init(&tmem_empty[a], 2 * kEpiWarps);
+            ptx::mbar_init(&tmem_empty[a], 2 * EPI_WARPS);
         }
         ptx::mbar_init(drain_bar, 1);
         *abort_flag = 0;
@@ -784,7 +788,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             if (!__all_sync(0xffffffffu, ptx::mbar_wait_bounded(&tmem_full[acc], acc_phase, abort_flag))) { ok = false; break; }
             ptx::tc_fence_after();
             const int64_t row = (int64_t)mb * 256 + (int64_t)rank * BM + quad * 32 + lane;
-            epilogue_tile<T, BN, SWIGLU>(p, tmem_base, acc, quad, (warp - 2) >> 2, row, row < p.M, nb, 0);
+            epilogue_tile<T, BN, SWIGLU, EPI_WARPS / 4>(p, tmem_base, acc, quad, (warp - 2) >> 2, row, row < p.M, nb, 0);
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive_cluster(ptx::map_to_cta(ptx::smem_u32(&tmem_empty[acc]), 0));
@@ -803,10 +807,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
 }
 
-template <typename T, bool SWIGLU>
-int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tb2, const GemmParams& p,
+template <typename T, bool SWIGLU, int EPI_WARPS>
+int launch_gemm_pair_with(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tb2, const GemmParams& p,
                      cudaStream_t st) {
-    auto kern = gemm_tc_pair_kernel<T, SWIGLU>;
+    constexpr int kThreads = 64 + EPI_WARPS * 32;
+    auto kern = gemm_tc_pair_kernel<T, SWIGLU, EPI_WARPS>;
     static std::atomic<uint64_t> reserved{0};
     if (!reserve_smem(kern, PAIR_SMEM_BYTES, reserved)) return fail(XG_ERR_LAUNCH, "xg_gemm_bias_act: cannot reserve %d bytes of shared memory", PAIR_SMEM_BYTES);
     const int tiles = p.num_m_blocks * p.num_n_blocks;
@@ -816,7 +821,7 @@ int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtenso
     if (max_pairs == 0) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(2 * (unsigned)(num_sms() / 2));
-        cfg.blockDim = dim3(kGemmThreads);
+        cfg.blockDim = dim3(kThreads);
         cfg.dynamicSmemBytes = PAIR_SMEM_BYTES;
         cudaLaunchAttribute attr;
         attr.id = cudaLaunchAttributeClusterDimension;
@@ -835,8 +840,13 @@ int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtenso
     const int pairs = tiles < max_pairs ? tiles : max_pairs;
     // plain stream order: a persistent kernel of hundreds of microseconds hides no set-up, and placed early (pairs starting
     // at different times) it ran 1.4 % (decoder layer of 16384 tokens) to 2.5 % slower
-    launch_with({.early = false}, kern, 2 * pairs, kGemmThreads, PAIR_SMEM_BYTES, st, ta, tb, tb2, p);
+    launch_with({.early = false}, kern, 2 * pairs, kThreads, PAIR_SMEM_BYTES, st, ta, tb, tb2, p);
     return check_launch("xg_gemm_bias_act (CTA pairs)");
+}
+template <typename T, bool SWIGLU>
+int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tb2, const GemmParams& p, cudaStream_t st) {
+    return p.num_k_blocks <= kPairShortK ? launch_gemm_pair_with<T, SWIGLU, 16>(ta, tb, tb2, p, st)
+                                         : launch_gemm_pair_with<T, SWIGLU, 8>(ta, tb, tb2, p, st);
 }
 
 // Second pass of split-K: out = act(sum_s partial[s] + bias + residual), 4 columns per thread.
@@ -1053,7 +1063,7 @@ gemm_tc_group_kernel(const __grid_constant__ GroupTable tab, const GemmParams p,
             pe.residual = tab.resid[entry];
             pe.mode = entry < rope_entries ? kModeRope : kModePlain;
             const int64_t row = (int64_t)mb * BM + quad * 32 + lane;
-            epilogue_tile<T, BN, false>(pe, tmem_base, acc, quad, (warp - 2) >> 2, row, row < p.M, nb, 0, 0);
+            epilogue_tile<T, BN, false, kEpiParts>(pe, tmem_base, acc, quad, (warp - 2) >> 2, row, row < p.M, nb, 0, 0);
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&tmem_empty[acc]);
