@@ -238,3 +238,17 @@ def test_flash_tc_split_keys(cuda_device, B, H, Sq, Skv, D, mask_kind, causal):
         add = add.masked_fill(~torch.ones(Sq, Skv, dtype=torch.bool).tril(), float("-inf"))
     want = ref_ops.sdpa_math(q.double(), k.double(), v.double(), add, None, False).to(torch.float16)
     assert_parity(got, want, f"split keys {B}x{H}x{Sq}x{Skv}x{D} {mask_kind} causal={causal}")
+
+
+@pytest.mark.parametrize("B,H,Sq,Skv,D", [(5, 61, 100, 333, 128), (4, 80, 129, 500, 64), (6, 60, 64, 256, 64), (64, 5, 3, 131, 64)])
+def test_key_masks_tiles_by_length(cuda_device, B, H, Sq, Skv, D):
+    """More query tiles than fit the chip, entries of different lengths: odd and even numbers of tiles, masks readable in words of
+    1, 4 and 16 bytes, an entry's last key in the bytes behind the last word, as many entries as the kernel keeps."""
+    q, k, v = _qkv(B, H, Sq, Skv, D, torch.float16, 64)
+    lengths = [(37 * b * b + 11 * b) % Skv + 1 for b in range(B)]
+    lengths[-1], lengths[B // 2] = Skv, 1
+    mask = torch.arange(Skv).view(1, 1, 1, Skv) < torch.tensor(lengths).view(B, 1, 1, 1)
+    got = _run(cuda_device, q, k, v, mask, None, False)
+    add = torch.zeros(B, 1, Sq, Skv, dtype=torch.double).masked_fill(~mask, float("-inf"))
+    want = ref_ops.sdpa_math(q.double(), k.double(), v.double(), add, None, False).to(torch.float16)
+    assert_parity(got, want, f"tiles by length {B}x{H}x{Sq}x{Skv}x{D}")

@@ -109,7 +109,7 @@ __device__ __forceinline__ FlashTile flash_tile(const FlashParams& p, const vola
         const int lim = (t.q0 + FM - 1) / FN + 1;  // last block that any row of this tile can see
         if (lim < t.nblk) t.nblk = lim;
     }
-    if (kv_blocks != nullptr && kv_blocks[b] < t.nblk) t.nblk = kv_blocks[b];
+    if (kv_blocks != nullptr && (kv_blocks[b] & 0xffff) < t.nblk) t.nblk = kv_blocks[b] & 0xffff;
     t.j0 = 0;
     if (p.splits > 1) {
         const int sp = (int)blockIdx.x % p.splits, n = t.nblk;
@@ -154,8 +154,18 @@ __device__ __forceinline__ FlashCursor flash_cursor(const FlashParams& p, int q_
 // i-th tile of this CTA (i = 0, 1, 2, ... in order). Returns 0 with the tile in t, -1 when the CTA is done, -2 for
 // the missing second half of a trailing odd pair.
 __device__ __forceinline__ int flash_next(FlashCursor& c, const volatile FlashStride* stride, const volatile int* kv_blocks, int i,
-                                          int num_tiles, int q_tiles, const FlashParams& p, FlashTile& t) {
+                                          int num_tiles, int q_tiles, const FlashParams& p, FlashTile& t, bool by_length) {
     if (p.single && i > 0) return -1;
+    if (by_length) {  // a CTA's pairs take the tiles from both ends of the list that runs from the longest batch entry to the shortest
+        const int pair = (int)blockIdx.x + (i >> 1) * (int)gridDim.x;
+        if (2 * pair >= num_tiles) return -1;
+        const int L = (i & 1) ? num_tiles - 1 - pair : pair;
+        if ((i & 1) && L == pair) return -2;
+        const int rank = L / (p.H * q_tiles), in_entry = L - rank * p.H * q_tiles;
+        const int h = in_entry / q_tiles;
+        t = flash_tile(p, kv_blocks, kv_blocks[rank] >> 16, h, in_entry - h * q_tiles, q_tiles);
+        return 0;
+    }
     if ((i & 1) == 0) {
         if (i > 0) {
             c.L += 2 * (int)gridDim.x;
@@ -211,6 +221,8 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
     int* kv_blocks_s = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(bars) + 256);
     const bool trim = MASK == 1 && p.mask != nullptr && (p.m_sh == 0 || p.H == 1) && p.B <= kFlashMaxB && (int64_t)p.B * p.Skv <= 65536;
     const volatile int* kv_blocks = trim ? kv_blocks_s : nullptr;
+    // Entries of different lengths: neighbouring tiles are equally long, so the longest entry's CTAs would finish last by far.
+    const bool by_length = MASK == 1 && !SPLIT && trim && !p.causal && !p.single;
 
     if ((ptx::smem_u32(smem) & 1023u) != 0) {  // uniform over the CTA: the swizzled tiles need this alignment
         pdl_sync();
@@ -253,18 +265,47 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_sync();  // the tensor memory is held
-    if (MASK == 1 && trim) {  // blocks up to each batch entry's last valid key
-        for (int b = threadIdx.x; b < p.B; b += kFlashThreads) kv_blocks_s[b] = 0;
-        __syncthreads();
-        const uint8_t* m = reinterpret_cast<const uint8_t*>(p.mask);
-        for (int b = 0; b < p.B; ++b) {
+    if (MASK == 1 && trim) {  // blocks up to each batch entry's last valid key (low half), entries by length (high half)
+        // a warp per entry, in the widest words that the rows allow (4096 keys are one round of 16-byte loads)
+        const uint8_t* mask = reinterpret_cast<const uint8_t*>(p.mask);
+        const uintptr_t bits = reinterpret_cast<uintptr_t>(mask) | (p.B > 1 ? (uintptr_t)p.m_sb : 0);
+        const int word = p.m_sk != 1 ? 1 : ((bits & 15) == 0 ? 16 : ((bits & 3) == 0 ? 4 : 1));
+        for (int b = warp; b < p.B; b += kFlashThreads / 32) {
+            const uint8_t* m = mask + b * p.m_sb;
             int last = -1;
+            auto in_word = [&](int at, uint32_t w) {
+                if (w != 0) last = at + ((31 - __clz((int)w)) >> 3);
+            };
+            int c = 0;
+            if (word == 16) {
 #pragma unroll 8
-            for (int c = threadIdx.x; c < p.Skv; c += kFlashThreads)
-                if (m[b * p.m_sb + c * p.m_sk]) last = c;
+                for (c = lane * 16; c + 16 <= p.Skv; c += 512) {
+                    const uint4 w = *reinterpret_cast<const uint4*>(m + c);
+                    in_word(c, w.x);
+                    in_word(c + 4, w.y);
+                    in_word(c + 8, w.z);
+                    in_word(c + 12, w.w);
+                }
+            } else if (word == 4) {
+#pragma unroll 8
+                for (c = lane * 4; c + 4 <= p.Skv; c += 128) in_word(c, *reinterpret_cast<const uint32_t*>(m + c));
+            }
+            const int rest = word == 1 ? 0 : p.Skv - p.Skv % word;  // keys left to single bytes
+#pragma unroll 8
+            for (c = rest + lane; c < p.Skv; c += 32)
+                if (m[c * p.m_sk]) last = c;
             last = __reduce_max_sync(0xffffffffu, last);
-            if ((threadIdx.x & 31) == 0 && last >= 0) atomicMax(&kv_blocks_s[b], last / FN + 1);
+            if (lane == 0) kv_blocks_s[b] = (last + FN) / FN;  // 0 without a valid key
         }
+        __syncthreads();
+        int order = 0, rank = 0;
+        if (by_length && threadIdx.x < p.B) {
+            order = (int)threadIdx.x;
+            for (int b = 0; b < p.B; ++b)
+                rank += kv_blocks_s[b] > kv_blocks_s[order] || (kv_blocks_s[b] == kv_blocks_s[order] && b < order);
+        }
+        __syncthreads();
+        if (by_length && threadIdx.x < p.B) atomicOr(&kv_blocks_s[rank], order << 16);
         __syncthreads();
     }
     constexpr int fmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
@@ -281,7 +322,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
             FlashCursor cur = flash_cursor(p, q_tiles);
             for (int i = 0; ok; ++i) {
                 FlashTile t;
-                const int tile_state = flash_next(cur, stride, kv_blocks, i, num_tiles, q_tiles, p, t);
+                const int tile_state = flash_next(cur, stride, kv_blocks, i, num_tiles, q_tiles, p, t, by_length);
                 if (tile_state == -1) break;
                 if (tile_state == -2) continue;
                 const uint32_t tile_par = tile_n++ & 1u;
@@ -347,7 +388,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
             };
             for (int i = 0; ok; ++i) {
                 FlashTile t;
-                const int tile_state = flash_next(cur, stride, kv_blocks, i, num_tiles, q_tiles, p, t);
+                const int tile_state = flash_next(cur, stride, kv_blocks, i, num_tiles, q_tiles, p, t, by_length);
                 if (tile_state == -1) break;
                 if (tile_state == -2) continue;
                 if (!ptx::mbar_wait_bounded(q_full, tile_n++ & 1u, abort_flag)) { ok = false; break; }
@@ -403,7 +444,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
 
         for (int i = 0; ok; ++i) {
             FlashTile t;
-            const int tile_state = flash_next(cur, stride, kv_blocks, i, num_tiles, q_tiles, p, t);
+            const int tile_state = flash_next(cur, stride, kv_blocks, i, num_tiles, q_tiles, p, t, by_length);
             if (tile_state == -1) break;
             if (tile_state == -2) continue;
             const int q0 = t.q0, nblk = t.nblk;

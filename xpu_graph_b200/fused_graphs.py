@@ -21,7 +21,8 @@ _encoder_block, _decoder_layer, _recommender = _X.encoder_block.default, _X.deco
 class FusedLlamaDecoderLayer(nn.Module):
     """RMSNorm | 2x dense with the RoPE epilogue (q, k) | dense (v) | flash SDPA | dense(+residual) | RMSNorm |
     dual-GEMM SwiGLU | dense(+residual). The two residual adds ride in the GEMM epilogues (the [M, N] addend
-    form of the dense layer) and RoPE in the q/k projections' epilogues, so the block is 9 kernels."""
+    form of the dense layer) and RoPE in the q/k projections' epilogues, so the block is 9 kernels; with few rows
+    the q, k and v projections are one launch (7 kernels)."""
 
     def __init__(self, layer: LlamaDecoderLayer, fuse_swiglu_gemm: bool = True, fuse_rope_gemm: bool = True):
         super().__init__()
@@ -55,8 +56,8 @@ class FusedEncoderBlock(nn.Module):
 
 class FusedRecsysGraph(nn.Module):
     """slice+cat of the dense features (one copy kernel) | 26 embedding lookups + where + stack (one
-    gather kernel) | cat | 3x dense+bias+ReLU (one dense-tower call when the layers are large enough for the fp32
-    tensor-core path)."""
+    gather kernel) | cat | 3x dense+bias+ReLU. Where the first layer is large enough for the fp32 tensor-core path
+    the three copies are one kernel that writes that layer's operand."""
 
     def __init__(self, graph: RecsysGraph):
         super().__init__()
