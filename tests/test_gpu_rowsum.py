@@ -122,8 +122,8 @@ def test_against_reference_fixtures(cuda_device, tag):
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("shape", [(16384, 50, 64), (3000, 21, 100), (700, 9, 5), (3, 50, 8)])  # both vector widths, both sides of "small"
 def test_overlapping_ranges_in_one_walk(cuda_device, shape, dtype):
-    """Ranges of one tensor that overlap without a common first row share one walk; every sum takes its rows in ascending
-    order, as it does on its own, so the results have to be the same bits as one launch per range."""
+    """Ranges of one tensor that overlap without a common first row share one walk. Against one launch per range the additions are
+    grouped by interval: both are within R * 2^-24 of sum |x| of the exact sum, and the result is then rounded to the type once."""
     from xpu_graph_b200.modules import SliceSumCatModule
 
     x = _rand(shape, dtype, 61).to(cuda_device)
@@ -134,7 +134,10 @@ def test_overlapping_ranges_in_one_walk(cuda_device, shape, dtype):
     for ranges in sets:
         got = SliceSumCatModule(ranges)(x)
         want = torch.cat([SliceSumCatModule([r])(x) for r in ranges], dim=-1)
-        assert torch.equal(got, want), (shape, dtype, ranges)
+        mag = torch.cat([x[:, a:b].double().abs().sum(1) for a, b in ranges], dim=-1)
+        step = 2.0 ** -24 if dtype == torch.float32 else 2.0 ** -8
+        bound = 2 * R * 2.0 ** -24 * mag + 2 * step * want.double().abs()
+        assert ((got.double() - want.double()).abs() <= bound).all(), (shape, dtype, ranges)
     want = ref_ops.slice_sum_cat(x.float().cpu(), sets[0]).to(dtype)
     mag = ref_ops.slice_sum_cat(x.float().abs().cpu(), sets[0])
     assert_parity(SliceSumCatModule(sets[0])(x), want, "overlapping ranges", magnitude=mag * (1e-2 if dtype != torch.float32 else 1e-3))

@@ -161,9 +161,9 @@ __global__ void __launch_bounds__(256) rowsum_prefix_kernel(const __grid_constan
 }
 
 // Up to NS ranges of one tensor (a[0], a_bs[0]) in one walk over the rows of their union. The range ends cut the union into
-// intervals whose rows go to the same set of sums (a bit per segment); rows of no range are not read. A sum takes its rows in
-// ascending order, as the general kernel does, so the results are the same bits. HBM-bound: 16384 x 50 x 64 fp32 with ranges
-// 0..50, 0..25, 0..10, 12..37 reads 50 rows instead of 110.
+// intervals whose rows go to the same set of sums (a bit per segment); rows of no range are not read. An interval is summed once,
+// rows ascending, and added to its sums: fp32 throughout, no more additions per result than row by row. HBM-bound: 16384 x 50 x 64 fp32 with ranges
+// 0..50, 0..25, 0..10, 12..37 reads 50 rows instead of 110: 71 -> 37 us; 32768 x 50 x 64 bf16 70 -> 50.
 constexpr int kWalkSegs = 8;
 constexpr int kWalkRows = 8;  // rows in flight per thread
 struct RowWalkParams {
@@ -178,7 +178,7 @@ struct RowWalkParams {
 };
 
 template <typename T, int V, int NS>
-__global__ void __launch_bounds__(256) rowsum_walk_kernel(const __grid_constant__ RowWalkParams p) {
+__global__ void __launch_bounds__(256, NS <= 4 ? 3 : 2) rowsum_walk_kernel(const __grid_constant__ RowWalkParams p) {
     pdl_sync();
     const int cv = p.C / V;
     const int64_t total = p.B * cv;
@@ -195,33 +195,35 @@ __global__ void __launch_bounds__(256) rowsum_walk_kernel(const __grid_constant_
             const uint32_t mask = p.mask[iv];
             if (mask == 0) continue;
             const int r1 = p.row[iv + 1];
+            float part[V];
+#pragma unroll
+            for (int i = 0; i < V; ++i) part[i] = 0.f;
             for (int r = p.row[iv]; r < r1; r += kWalkRows) {
                 const T* ap = base + (int64_t)r * p.C;
-                float x[kWalkRows][V];
+                Vec16<T> x[kWalkRows];  // in the tensor's type until they are added: fewer registers, more CTAs per SM
 #pragma unroll
                 for (int u = 0; u < kWalkRows; ++u) {
                     if (r + u < r1) {
-                        if (V > 1) {
-                            const Vec16<T> v = ld16_stream(ap + (int64_t)u * p.C);
+                        if (V > 1) x[u] = ld16_stream(ap + (int64_t)u * p.C);
+                        else x[u].v[0] = ap[(int64_t)u * p.C];
+                    } else {
 #pragma unroll
-                            for (int i = 0; i < V; ++i) x[u][i] = Cvt<T>::to_f(v.v[i]);
-                        } else {
-                            x[u][0] = Cvt<T>::to_f(ap[(int64_t)u * p.C]);
-                        }
+                        for (int i = 0; i < V; ++i) x[u].v[i] = Cvt<T>::from_f(0.f);
                     }
                 }
 #pragma unroll
-                for (int u = 0; u < kWalkRows; ++u) {
-                    if (r + u < r1) {
+                for (int u = 0; u < kWalkRows; ++u)
 #pragma unroll
-                        for (int s = 0; s < NS; ++s)
-                            if ((mask >> s) & 1u) {
-#pragma unroll
-                                for (int i = 0; i < V; ++i) acc[s][i] += x[u][i];
-                            }
-                    }
-                }
+                    for (int i = 0; i < V; ++i) part[i] += Cvt<T>::to_f(x[u].v[i]);
             }
+            // once per interval: a test per row and sum bound the kernel by its branches (16-bit rows: 118 us instead of 70
+            // for a launch slice per range)
+#pragma unroll
+            for (int s = 0; s < NS; ++s)
+                if ((mask >> s) & 1u) {
+#pragma unroll
+                    for (int i = 0; i < V; ++i) acc[s][i] += part[i];
+                }
         }
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
@@ -372,22 +374,19 @@ extern "C" int xg_rowsum_cat(const void* const* a_ptrs, const void* const* b_ptr
             default: return launch_rowsum<__half>(p, false, true, vec, st);
         }
     }
-    // ranges of one tensor that overlap: the walk kernel, where it reads at least a fifth less. While the grid is below one
-    // CTA per SM the longest chain of loads decides instead of the bytes, and the walk's must not be longer than the ranges'.
+    // ranges of one tensor that overlap: the walk kernel, where it reads at least a fifth less and there is a CTA for every SM
+    // (below that the longest chain of loads decides instead of the bytes, and the walk's is no shorter)
     if (!mul && n > 1 && n <= kWalkSegs) {
         bool same = true;
-        int64_t read = 0, longest = 0;
+        int64_t read = 0;
         for (int64_t k = 0; k < n; ++k) {
-            const int64_t len = row_ranges2[2 * k + 1] - row_ranges2[2 * k];
             same = same && a_ptrs[k] == a_ptrs[0] && a_batch_strides[k] == a_batch_strides[0];
-            read += len;
-            longest = len > longest ? len : longest;
+            read += row_ranges2[2 * k + 1] - row_ranges2[2 * k];
         }
-        if (same) {
+        if (same && B * (vec ? C / V : C) >= 256LL * num_sms()) {
             RowWalkParams w;
             const int64_t rows = plan_walk(row_ranges2, (int)n, w);
-            const bool small = B * (vec ? C / V : C) < 256LL * num_sms();
-            if (5 * rows <= 4 * read && (!small || rows == longest)) {
+            if (5 * rows <= 4 * read) {
                 w.a = a_ptrs[0];
                 w.out = out;
                 w.a_bs = a_batch_strides[0];
