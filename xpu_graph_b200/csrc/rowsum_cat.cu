@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(256) rowsum_prefix_kernel(const __grid_constan
 
 // Up to NS ranges of one tensor (a[0], a_bs[0]) in one walk over the rows of their union. The range ends cut the union into
 // intervals whose rows go to the same set of sums (a bit per segment); rows of no range are not read. An interval is summed once,
-// rows ascending, and added to its sums: fp32 throughout, no more additions per result than row by row. HBM-bound: 16384 x 50 x 64 fp32 with ranges
+// rows ascending, and added to its sums (fp32 throughout). HBM-bound: 16384 x 50 x 64 fp32 with ranges
 // 0..50, 0..25, 0..10, 12..37 reads 50 rows instead of 110: 71 -> 37 us; 32768 x 50 x 64 bf16 70 -> 50.
 constexpr int kWalkSegs = 8;
 constexpr int kWalkRows = 8;  // rows in flight per thread
