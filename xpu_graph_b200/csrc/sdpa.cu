@@ -63,8 +63,7 @@ struct FlashParams {
     int B, H, Sq, Skv;
     float scale;
     int16_t causal, mask_kind;
-    int16_t single;  // one tile per CTA (the tiles fit the chip at once) instead of a list of tile pairs
-    int16_t splits;  // CTAs that share a tile's keys (single only)
+    int16_t splits;  // CTAs that share a tile's keys
 };
 static_assert(sizeof(FlashParams) <= 128, "flash kernel parameter block must stay within 512 bytes");
 
@@ -98,6 +97,7 @@ struct FlashTile {
     int b, h, q0;
     int j0, nblk;  // key blocks [j0, j0 + nblk)
 };
+template <int MODE>
 __device__ __forceinline__ FlashTile flash_tile(const FlashParams& p, const volatile int* kv_blocks, int b, int h, int k, int q_tiles) {
     const int qt = p.causal ? ((k & 1) ? (k >> 1) : (q_tiles - 1 - (k >> 1))) : k;
     FlashTile t;
@@ -111,7 +111,7 @@ __device__ __forceinline__ FlashTile flash_tile(const FlashParams& p, const vola
     }
     if (kv_blocks != nullptr && (kv_blocks[b] & 0xffff) < t.nblk) t.nblk = kv_blocks[b] & 0xffff;
     t.j0 = 0;
-    if (p.splits > 1) {
+    if (MODE == 2) {
         const int sp = (int)blockIdx.x % p.splits, n = t.nblk;
         t.j0 = n * sp / p.splits;
         t.nblk = n * (sp + 1) / p.splits - t.j0;
@@ -142,9 +142,10 @@ __device__ __forceinline__ FlashStride flash_stride(const FlashParams& p, int q_
     s.dh = bh - s.db * p.H;
     return s;
 }
+template <int MODE>
 __device__ __forceinline__ FlashCursor flash_cursor(const FlashParams& p, int q_tiles) {
     FlashCursor c;
-    c.L = p.single ? (int)blockIdx.x / p.splits : 2 * (int)blockIdx.x;
+    c.L = MODE == 0 ? 2 * (int)blockIdx.x : (MODE == 1 ? (int)blockIdx.x : (int)blockIdx.x / p.splits);
     const int bh = c.L / q_tiles;
     c.k = c.L - bh * q_tiles;
     c.b = bh / p.H;
@@ -153,9 +154,10 @@ __device__ __forceinline__ FlashCursor flash_cursor(const FlashParams& p, int q_
 }
 // i-th tile of this CTA (i = 0, 1, 2, ... in order). Returns 0 with the tile in t, -1 when the CTA is done, -2 for
 // the missing second half of a trailing odd pair.
+template <int MODE>
 __device__ __forceinline__ int flash_next(FlashCursor& c, const volatile FlashStride* stride, const volatile int* kv_blocks, int i,
                                           int num_tiles, int q_tiles, const FlashParams& p, FlashTile& t, bool by_length) {
-    if (p.single && i > 0) return -1;
+    if (MODE != 0 && i > 0) return -1;
     if (by_length) {  // a CTA's pairs take the tiles from both ends of the list that runs from the longest batch entry to the shortest
         const int pair = (int)blockIdx.x + (i >> 1) * (int)gridDim.x;
         if (2 * pair >= num_tiles) return -1;
@@ -163,7 +165,7 @@ __device__ __forceinline__ int flash_next(FlashCursor& c, const volatile FlashSt
         if ((i & 1) && L == pair) return -2;
         const int rank = L / (p.H * q_tiles), in_entry = L - rank * p.H * q_tiles;
         const int h = in_entry / q_tiles;
-        t = flash_tile(p, kv_blocks, kv_blocks[rank] >> 16, h, in_entry - h * q_tiles, q_tiles);
+        t = flash_tile<MODE>(p, kv_blocks, kv_blocks[rank] >> 16, h, in_entry - h * q_tiles, q_tiles);
         return 0;
     }
     if ((i & 1) == 0) {
@@ -175,13 +177,13 @@ __device__ __forceinline__ int flash_next(FlashCursor& c, const volatile FlashSt
             flash_carry(c.b, c.h, c.k, q_tiles, p.H);  // k < 2 q_tiles and h <= 2 H - 1 here: one carry each is enough
         }
         if (c.L >= num_tiles) return -1;
-        t = flash_tile(p, kv_blocks, c.b, c.h, c.k, q_tiles);
+        t = flash_tile<MODE>(p, kv_blocks, c.b, c.h, c.k, q_tiles);
         return 0;
     }
     if (c.L + 1 >= num_tiles) return -2;
     int b = c.b, h = c.h, k = c.k + 1;
     flash_carry(b, h, k, q_tiles, p.H);
-    t = flash_tile(p, kv_blocks, b, h, k, q_tiles);
+    t = flash_tile<MODE>(p, kv_blocks, b, h, k, q_tiles);
     return 0;
 }
 
@@ -192,8 +194,11 @@ __device__ __forceinline__ int flash_next(FlashCursor& c, const volatile FlashSt
 // score. (4 x 32 x 500 x 500, head dim 64, padding: 74 us with the general code, see launch_flash_tc for the others.) The
 // common cases are compiled without it: the code of a tile boundary runs once per tile, its instruction fetches miss the
 // instruction caches, and a smaller kernel keeps more of it resident.
-// SPLIT: a tile's keys are shared out over several CTAs; each leaves its unnormalised part in scratch memory.
-template <typename T, int D, int MASK, bool SPLIT>
+// MODE: how tiles come to CTAs; kList: a persistent CTA walks pairs of a list; kSingle: one tile per CTA; kSplit: a tile's keys are
+// shared out over several CTAs, each of which leaves its unnormalised part in scratch memory. Fixed at compile time like the mask:
+// what the long lists do not need (a first key block, warps without rows) would sit in their inner loop.
+enum FlashMode : int { kList = 0, kSingle = 1, kSplit = 2 };
+template <typename T, int D, int MASK, int MODE>
 __global__ void __launch_bounds__(kFlashThreads, 2)
 flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUtensorMap tmk,
                 const __grid_constant__ CUtensorMap tmv, const FlashParams p) {
@@ -222,7 +227,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
     const bool trim = MASK == 1 && p.mask != nullptr && (p.m_sh == 0 || p.H == 1) && p.B <= kFlashMaxB && (int64_t)p.B * p.Skv <= 65536;
     const volatile int* kv_blocks = trim ? kv_blocks_s : nullptr;
     // Entries of different lengths: neighbouring tiles are equally long, so the longest entry's CTAs would finish last by far.
-    const bool by_length = MASK == 1 && !SPLIT && trim && !p.causal && !p.single;
+    const bool by_length = MASK == 1 && MODE == kList && trim && !p.causal;
 
     if ((ptx::smem_u32(smem) & 1023u) != 0) {  // uniform over the CTA: the swizzled tiles need this alignment
         pdl_sync();
@@ -319,10 +324,10 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
             bool ok = true;
             uint32_t n = 0;      // key blocks loaded so far (all tiles)
             uint32_t tile_n = 0; // tiles started so far
-            FlashCursor cur = flash_cursor(p, q_tiles);
+            FlashCursor cur = flash_cursor<MODE>(p, q_tiles);
             for (int i = 0; ok; ++i) {
                 FlashTile t;
-                const int tile_state = flash_next(cur, stride, kv_blocks, i, num_tiles, q_tiles, p, t, by_length);
+                const int tile_state = flash_next<MODE>(cur, stride, kv_blocks, i, num_tiles, q_tiles, p, t, by_length);
                 if (tile_state == -1) break;
                 if (tile_state == -2) continue;
                 const uint32_t tile_par = tile_n++ & 1u;
@@ -364,7 +369,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
             uint32_t nq = 0;  // Q K^T blocks issued so far (all tiles)
             uint32_t np = 0;  // P V blocks issued so far
             uint32_t tile_n = 0;
-            FlashCursor cur = flash_cursor(p, q_tiles);
+            FlashCursor cur = flash_cursor<MODE>(p, q_tiles);
             // Score buffer nq & 1 is free without a barrier of its own: this thread has already waited for
             // p_full of block nq - 2 (the softmax warps had read S and written P by then) and issued that
             // block's P V before this point, and the tensor core runs this thread's MMAs in issue order.
@@ -388,7 +393,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
             };
             for (int i = 0; ok; ++i) {
                 FlashTile t;
-                const int tile_state = flash_next(cur, stride, kv_blocks, i, num_tiles, q_tiles, p, t, by_length);
+                const int tile_state = flash_next<MODE>(cur, stride, kv_blocks, i, num_tiles, q_tiles, p, t, by_length);
                 if (tile_state == -1) break;
                 if (tile_state == -2) continue;
                 if (!ptx::mbar_wait_bounded(q_full, tile_n++ & 1u, abort_flag)) { ok = false; break; }
@@ -440,18 +445,18 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
         bool ok = true;
         uint32_t n = 0;       // key blocks processed so far (all tiles)
         uint32_t tile_n = 0;  // tiles finished so far
-        FlashCursor cur = flash_cursor(p, q_tiles);
+        FlashCursor cur = flash_cursor<MODE>(p, q_tiles);
 
         for (int i = 0; ok; ++i) {
             FlashTile t;
-            const int tile_state = flash_next(cur, stride, kv_blocks, i, num_tiles, q_tiles, p, t, by_length);
+            const int tile_state = flash_next<MODE>(cur, stride, kv_blocks, i, num_tiles, q_tiles, p, t, by_length);
             if (tile_state == -1) break;
             if (tile_state == -2) continue;
             const int q0 = t.q0, nblk = t.nblk;
             const int row = q0 + r_in_tile;
             const int64_t m_off = (int64_t)t.b * p.m_sb + (int64_t)t.h * p.m_sh + (MASK == 2 ? (int64_t)row * p.m_sq : 0);
             const bool has_mask = MASK != 0 && p.mask != nullptr && (MASK == 1 || row < p.Sq);
-            const bool idle = q0 + quad * 32 >= p.Sq;  // none of this warp's rows exists: only the hand-shakes are kept up
+            const bool idle = (MASK != 0 || MODE != kList) && q0 + quad * 32 >= p.Sq;  // none of this warp's rows exists: only the hand-shakes are kept up
             // MASK == 1: keys lane and lane + 32 of a block
             auto key_ok = [&](int col) {
                 return col < skv && (!has_mask || reinterpret_cast<const uint8_t*>(p.mask)[m_off + (int64_t)col * p.m_sk] != 0);
@@ -628,7 +633,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
                 ++tile_n;
             }
             ptx::tc_fence_after();
-            if (SPLIT) {
+            if (MODE == kSplit) {
                 const int64_t unit_row = (int64_t)blockIdx.x * FM + r_in_tile;
                 float* po = p.partial + unit_row * D;
 #pragma unroll 1
@@ -788,17 +793,17 @@ int launch_flash_tc(const SdpaParams& p, void* workspace, int64_t ws_bytes, cuda
     const int64_t tiles = p.B * p.H * q_tiles;
     if (tiles > 0x7fffffffLL) return fail(XG_ERR_TOO_LARGE, "xg_sdpa_fwd: too many tiles");
     const int64_t resident = 2LL * num_sms();  // persistent CTAs, two per SM
-    fp.single = tiles <= resident;
-    int splits = fp.single ? flash_splits(tiles, p.Skv) : 1;
+    const bool single = tiles <= resident;  // one tile per CTA, all at once
+    int splits = single ? flash_splits(tiles, p.Skv) : 1;
     if (splits > 1 && (!workspace || !aligned16(workspace) || ws_bytes < tiles * splits * FM * (D + 2) * 4)) splits = 1;
     fp.splits = (int16_t)splits;
     fp.partial = reinterpret_cast<float*>(workspace);
     // tiles in a list: a CTA takes neighbouring (heavy, light) pairs
     const int64_t pairs = (tiles + 1) / 2;
-    const unsigned grid = (unsigned)(fp.single ? tiles * splits : (pairs < resident ? pairs : resident));
+    const unsigned grid = (unsigned)(single ? tiles * splits : (pairs < resident ? pairs : resident));
     const bool rows_differ = p.mask != nullptr && (p.mask_kind == kMaskAdd || (p.m_sq != 0 && p.Sq > 1));
     const int mask = rows_differ || !(p.scale > 0.f) ? 2 : (p.mask != nullptr || p.Skv % FN != 0 ? 1 : 0);
-    static std::atomic<uint64_t> reserved[6];
+    static std::atomic<uint64_t> reserved[9];
     auto run = [&](auto kern, int slot) {
         if (!reserve_smem(kern, Cfg::SMEM_BYTES, reserved[slot])) return fail(XG_ERR_LAUNCH, "xg_sdpa_fwd: cannot reserve shared memory");
         // plain stream order: placed early, as slots come free, the tile lists ran slower (8 x 32 x 1024 causal 115 us instead of 109,
@@ -806,15 +811,17 @@ int launch_flash_tc(const SdpaParams& p, void* workspace, int64_t ws_bytes, cuda
         launch_with({.early = false}, kern, grid, kFlashThreads, Cfg::SMEM_BYTES, st, tq, tk, tv, fp);
         return check_launch("xg_sdpa_fwd");
     };
-    if (splits == 1) {
+    auto with_mask = [&](auto mode) {
+        constexpr int M = decltype(mode)::value;
         switch (mask) {
-            case 0: return run(flash_tc_kernel<T, D, 0, false>, 0);
-            case 1: return run(flash_tc_kernel<T, D, 1, false>, 1);
-            default: return run(flash_tc_kernel<T, D, 2, false>, 2);
+            case 0: return run(flash_tc_kernel<T, D, 0, M>, 3 * M);
+            case 1: return run(flash_tc_kernel<T, D, 1, M>, 3 * M + 1);
+            default: return run(flash_tc_kernel<T, D, 2, M>, 3 * M + 2);
         }
-    }
-    const int rc = mask == 0 ? run(flash_tc_kernel<T, D, 0, true>, 3)
-                             : (mask == 1 ? run(flash_tc_kernel<T, D, 1, true>, 4) : run(flash_tc_kernel<T, D, 2, true>, 5));
+    };
+    if (!single) return with_mask(std::integral_constant<int, kList>{});
+    if (splits == 1) return with_mask(std::integral_constant<int, kSingle>{});
+    const int rc = with_mask(std::integral_constant<int, kSplit>{});
     if (rc != XG_OK) return rc;
     launch(flash_combine_kernel<T, D>, (unsigned)((p.B * p.H * p.Sq + 3) / 4), 128, 0, st, fp, q_tiles);
     return check_launch("xg_sdpa_fwd (combine)");
