@@ -177,3 +177,42 @@ def test_cuda_graph_replay_llama_small(cuda_device):
     torch.cuda.synchronize()
     assert lib.tc_status() == 0
     assert_parity(got, want, "llama graph replay")
+
+
+@pytest.mark.parametrize("batch,seq,hidden,splits_k", [(1, 16, 4096, True), (1, 128, 4096, True), (1, 333, 4096, True), (3, 37, 1024, False),
+                                                       (2, 500, 512, False)])
+def test_llama_layer_equals_its_op_sequence(cuda_device, batch, seq, hidden, splits_k):
+    """The decoder layer's operator gives the bits of the replacement modules called one after the other, as a graph rewritten
+    op by op calls them - at row counts where q and k share a launch, and where the dense kernels split K for the v projection."""
+    import ctypes
+
+    from tests.helpers import LaunchCounter
+    from xpu_graph_b200 import lib
+    from xpu_graph_b200 import modules as M
+    from xpu_graph_b200.fused_graphs import FusedLlamaDecoderLayer
+    from xpu_graph_b200.workloads import make_llama_layer
+
+    heads = hidden // 128
+    model, (x, cos, sin) = make_llama_layer(seed=3, batch=batch, seq=seq, hidden=hidden, heads=heads, ffn=1376)
+    model = model.to(torch.bfloat16).to(cuda_device)
+    x, cos, sin = x.to(cuda_device), cos.to(cuda_device), sin.to(cuda_device)
+    rows, L = batch * seq, lib.load()
+    S, tn = ctypes.c_int(0), ctypes.c_int(0)
+    clusters = L.xg_gemm_cluster_plan(rows, hidden, hidden, lib.XG_BF16, ctypes.byref(S), ctypes.byref(tn)) and S.value > 1
+    assert bool(clusters or L.xg_gemm_workspace_bytes(rows, hidden, hidden, lib.XG_BF16)) == splits_k
+    with LaunchCounter() as calls:
+        got = FusedLlamaDecoderLayer(model)(x, cos, sin)
+    assert "xg_gemm_rope_group" in calls.names
+    norm, dense, rope = M.RMSNormModule(), M.DenseLayerModule(False), M.DenseRopeModule()
+    with torch.no_grad():
+        x2 = x.reshape(rows, hidden)
+        h = norm(x2, model.input_norm.weight, model.input_norm.eps)
+        q, k = (rope(h, p.weight, cos, sin, batch, seq, heads, 128) for p in (model.q_proj, model.k_proj))
+        v = dense(h, model.v_proj.weight, True, None, "none").view(batch, seq, heads, 128).transpose(1, 2)
+        a = M.SDPAModule()(q, k, v, None, None, True).transpose(1, 2).reshape(rows, hidden)
+        x2 = dense(a, model.o_proj.weight, True, x2, "none")
+        h = norm(x2, model.post_norm.weight, model.post_norm.eps)
+        want = dense(M.DenseSwiGLUModule()(h, model.gate_proj.weight, model.up_proj.weight), model.down_proj.weight, True, x2, "none")
+    torch.cuda.synchronize()
+    assert lib.tc_status() == 0
+    assert torch.equal(got.view(rows, hidden), want)

@@ -923,18 +923,31 @@ Tensor encoder_block(const Tensor& x, const c10::List<optional<Tensor>>& params,
     return dense(h, weight(5), true, bias(5), x1, "none").view({B, S, C});
 }
 
-// The q, k and v projections of one hidden state in one launch where that is the faster way; false: not taken.
+// Whether dense() adds up an output's products in one chain over K, as the grouped kernel does. Where it splits K (split-K through
+// scratch, clusters of several CTA pairs) the partial sums round differently.
+bool dense_sums_in_one_chain(int64_t M, int64_t N, int64_t K, int code) {
+    int splits = 0, tile_n = 0;
+    return xg_gemm_workspace_bytes(M, N, K, code) == 0 && !(xg_gemm_cluster_plan(M, N, K, code, &splits, &tile_n) && splits > 1);
+}
+
+// The q and k projections of one hidden state in one launch where that is the faster way (false: not taken), and v with them
+// where the result is bit for bit that of a launch of its own: a graph rewritten op by op gives the same numbers.
 bool qkv_rope(const Tensor& x_in, const Tensor& wq, const Tensor& wk, const Tensor& wv, const Tensor& cos, const Tensor& sin, int64_t S, int64_t D,
               Tensor* q, Tensor* k, Tensor* v) {
     const at::ScalarType dt = x_in.scalar_type();
     if ((dt != at::kHalf && dt != at::kBFloat16) || (D != 64 && D != 128) || wq.dim() != 2 || x_in.size(0) == 0) return false;
-    const Tensor* ws[3] = {&wq, &wk, &wv};
-    for (const Tensor* w : ws)
-        if (w->dim() != 2 || w->scalar_type() != dt || w->sizes() != wq.sizes() || w->strides() != wq.strides() || w->stride(1) != 1 ||
-            (reinterpret_cast<uintptr_t>(ptr(*w)) & 15u) != 0)
-            return false;
+    const int code = code_of(dt);
     const int64_t M = x_in.size(0), K = x_in.size(1), N = wq.size(0), ldw = row_stride(wq);
-    if (wq.size(1) != K || K == 0 || N == 0 || K % 8 != 0 || ldw % 8 != 0 || N % D != 0 || N % 8 != 0 || !xg_gemm_rope_group_worth_it(3, M, N, K)) return false;
+    if (wq.size(1) != K || K == 0 || N == 0 || K % 8 != 0 || ldw % 8 != 0 || N % D != 0 || N % 8 != 0) return false;
+    const int count = dense_sums_in_one_chain(M, N, K, code) ? 3 : 2;
+    const Tensor* ws[3] = {&wq, &wk, &wv};
+    for (int i = 0; i < count; ++i) {
+        const Tensor& w = *ws[i];
+        if (w.dim() != 2 || w.scalar_type() != dt || w.sizes() != wq.sizes() || w.strides() != wq.strides() || w.stride(1) != 1 ||
+            (reinterpret_cast<uintptr_t>(ptr(w)) & 15u) != 0)
+            return false;
+    }
+    if (!xg_gemm_rope_group_worth_it(count, M, N, K)) return false;
     const On on(x_in);
     const Tensor x = unit_rows(x_in);
     if ((reinterpret_cast<uintptr_t>(ptr(x)) & 15u) != 0 || row_stride(x) % 8 != 0) return false;
@@ -943,12 +956,12 @@ bool qkv_rope(const Tensor& x_in, const Tensor& wq, const Tensor& wk, const Tens
     Tensor* outs[3] = {q, k, v};
     const void* wp[3];
     void* op[3];
-    for (int i = 0; i < 3; ++i) {
+    for (int i = 0; i < count; ++i) {
         *outs[i] = new_tensor({M, N}, dt, x);
         wp[i] = ptr(*ws[i]);
         op[i] = mut(*outs[i]);
     }
-    XG_CALL(xg_gemm_rope_group, ptr(x), wp, ptr(c), ptr(s), op, 3, 2, M, N, K, row_stride(x), ldw, N, S, D, code_of(dt), on.stream);
+    XG_CALL(xg_gemm_rope_group, ptr(x), wp, ptr(c), ptr(s), op, count, 2, M, N, K, row_stride(x), ldw, N, S, D, code, on.stream);
     return true;
 }
 
@@ -968,7 +981,7 @@ Tensor decoder_layer(const Tensor& x, const Tensor& cos, const Tensor& sin, at::
     if (fuse_rope && qkv_rope(h, w[1], w[2], w[3], cos, sin, S, D, &q, &k, &v)) {
         q = heads_view(q, B, S, heads, D, 0);
         k = heads_view(k, B, S, heads, D, 0);
-        v = heads_view(v, B, S, heads, D, 0);
+        if (v.defined()) v = heads_view(v, B, S, heads, D, 0);
     } else if (fuse_rope) {
         q = heads_view(dense_rope(h, w[1], cos, sin, S, D), B, S, heads, D, 0);
         k = heads_view(dense_rope(h, w[2], cos, sin, S, D), B, S, heads, D, 0);

@@ -22,7 +22,8 @@ class FusedLlamaDecoderLayer(nn.Module):
     """RMSNorm | 2x dense with the RoPE epilogue (q, k) | dense (v) | flash SDPA | dense(+residual) | RMSNorm |
     dual-GEMM SwiGLU | dense(+residual). The two residual adds ride in the GEMM epilogues (the [M, N] addend
     form of the dense layer) and RoPE in the q/k projections' epilogues, so the block is 9 kernels; with few rows
-    the q, k and v projections are one launch (7 kernels)."""
+    the q and k projections are one launch (8 kernels), and v with them where the dense layer would not split K for it
+    (7 kernels): every result has the bits that the op sequence gives."""
 
     def __init__(self, layer: LlamaDecoderLayer, fuse_swiglu_gemm: bool = True, fuse_rope_gemm: bool = True):
         super().__init__()
