@@ -557,9 +557,14 @@ int launch_fma(const GemmF32Params& g, int S, cudaStream_t st) {
     const int64_t per_cta = ((g.K + Cfg::KC - 1) / Cfg::KC + S - 1) / S;
     p.stages = (int)(per_cta < kFmaStages ? per_cta : kFmaStages);
     const dim3 grid((unsigned)((g.N + Cfg::BN - 1) / Cfg::BN * S), (unsigned)((g.M + Cfg::BM - 1) / Cfg::BM));
-    // Placed early only above one CTA per SM (see LaunchOptions), and never as clusters: an early cluster of 8 whose peers
-    // read each other's shared memory raised a misaligned-address error behind another launch of itself.
-    launch_with({.cluster = S > 1 ? (unsigned)S : 0u, .early = S == 1 && (int64_t)grid.x * grid.y > num_sms()}, kern, grid, kFmaThreads,
+    // Placed early only above one CTA per SM (see LaunchOptions). Clusters never are: an early one of eight raised a
+    // misaligned-address error behind another launch of itself. What reading excludes: the row pitch of a partial tile (160, 288
+    // or 544 bytes) and the column offsets are multiples of 16 bytes and end inside the partial tiles, the area starts at one
+    // offset in all CTAs, peers have started before the first remote access (cluster barrier) and are there until the last one
+    // (second barrier). What it leaves open: whether the form that faulted still read rows past M from the peers and dropped
+    // them; a load without a consumer can be under way when its owner's shared memory goes to the next kernel. The kernel has no
+    // such loads (see the `continue` above); that they were the cause is not shown.
+    launch_with({.cluster = S > 1 ? (unsigned)S : 0u, .early = (int64_t)grid.x * grid.y > num_sms()}, kern, grid, kFmaThreads,
                 Cfg::smem(p.stages), st, ta, tw, p);
     return check_launch("xg_gemm_bias_act(f32)");
 }

@@ -474,7 +474,8 @@ int launch_ksplit(const void* A, const void* W, const void* bias, const void* re
     p.stages = S > 1 ? KS_STAGES_SPLIT : KS_STAGES_WHOLE;
     const int64_t tiles = (int64_t)p.num_m_blocks * p.num_n_blocks;
     if (tiles * 2 * S > 0x7fffffffLL) return fail(XG_ERR_TOO_LARGE, "xg_gemm_bias_act: too many tiles for one launch");
-    launch_with({.cluster = (unsigned)(2 * S)}, kern, (unsigned)(tiles * 2 * S), KS_THREADS, KS_SMEM_BYTES, st, ta, tw, p);
+    // in plain stream order, as every cluster (placed_early)
+    launch_with({.cluster = (unsigned)(2 * S), .early = false}, kern, (unsigned)(tiles * 2 * S), KS_THREADS, KS_SMEM_BYTES, st, ta, tw, p);
     return check_launch("xg_gemm_bias_act (k-split clusters)");
 }
 
