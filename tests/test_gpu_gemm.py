@@ -507,6 +507,77 @@ def test_dense_fp32_weight_planes_follow_the_weight(cuda_device):
     assert_parity(y2, (y1 * 2.0), "dense fp32 after an in-place weight update")
 
 
+@pytest.mark.parametrize("kn", [False, True])
+def test_dense_fp32_weight_planes_across_streams(cuda_device, kn):
+    """A call that finds the planes of a weight while another stream has still to write them waits for that stream."""
+    from xpu_graph_b200 import ops
+
+    M, K, N = 1024, 1024, 512
+    dense = ops.dense
+    x, w = torch.randn(M, K, device=cuda_device), torch.randn(*((K, N) if kn else (N, K)), device=cuda_device) * K ** -0.5
+    want = (x.double() @ (w.double() if kn else w.double().t())).float().cpu()
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    for stream in (first, second):  # memory for the call, so that it does not wait for the device to get some
+        with torch.cuda.stream(stream):
+            dense(x, w.clone(), not kn, None, None, "none")
+    with torch.cuda.stream(first):
+        junk = torch.full((N, 3 * K), float("nan"), dtype=torch.bfloat16, device=cuda_device)  # what the planes' memory held before
+    torch.cuda.synchronize()
+    del junk
+    with torch.cuda.stream(first):
+        torch.cuda._sleep(200_000_000)
+        a = dense(x, w, not kn, None, None, "none")
+    with torch.cuda.stream(second):
+        b = dense(x, w, not kn, None, None, "none")
+    second.synchronize()
+    assert_parity(b, want, "second stream")
+    torch.cuda.synchronize()
+    assert_parity(a, want, "first stream")
+
+
+@pytest.mark.parametrize("warm", [False, True])
+def test_dense_fp32_weight_planes_and_capture(cuda_device, warm):
+    """A captured layer splits its weight itself: what is made during a capture is not kept for eager calls (it holds nothing
+    before the first replay), and a replay after an in-place update of the weight uses the weight as it is then."""
+    from xpu_graph_b200 import ops
+
+    M, K, N = 1024, 1024, 512
+    dense = ops.dense
+    x, w = torch.randn(M, K, device=cuda_device), torch.randn(N, K, device=cuda_device) * K ** -0.5
+    dense(x, w.clone(), True, None, None, "none")  # one-time set-up of the kernels
+    math = lambda: (x.double() @ w.double().t()).float().cpu()  # noqa: E731
+    if warm:
+        dense(x, w, True, None, None, "none")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = dense(x, w, True, None, None, "none")
+    assert_parity(dense(x, w, True, None, None, "none"), math(), "eager after a capture")
+    graph.replay()
+    assert_parity(y, math(), "first replay")
+    w.mul_(-0.5)
+    assert_parity(dense(x, w, True, None, None, "none"), math(), "eager after an update")
+    junk = [torch.full((N, 3 * K), float("nan"), dtype=torch.bfloat16, device=cuda_device) for _ in range(4)]
+    graph.replay()
+    assert_parity(y, math(), "replay after an update")
+    del junk
+
+
+def test_dense_fp32_weight_planes_are_not_taken_from_copies(cuda_device):
+    """Planes that came along with a deep copy of the weight's attributes are not those of the copy."""
+    import copy
+
+    from xpu_graph_b200 import ops
+
+    x, w = torch.randn(1024, 1024, device=cuda_device), torch.randn(512, 1024, device=cuda_device) / 32
+    ops.dense(x, w, True, None, None, "none")
+    v = copy.deepcopy(w)
+    v._xg_bf16_planes = copy.deepcopy(w._xg_bf16_planes)
+    w._xg_bf16_planes = (w._xg_bf16_planes[0], torch.zeros_like(w._xg_bf16_planes[1]))  # right key, planes without an origin
+    want = (x.double() @ w.double().t()).float().cpu()
+    assert_parity(ops.dense(x, w, True, None, None, "none"), want, "planes without an origin")
+    assert_parity(ops.dense(x, v, True, None, None, "none"), want, "deep copy")
+
+
 def test_dense_swiglu(cuda_device):
     from xpu_graph_b200 import lib
     from xpu_graph_b200.modules import DenseSwiGLUModule

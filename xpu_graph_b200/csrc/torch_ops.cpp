@@ -9,7 +9,9 @@
 // Observers (lib.call_hook) see the calls made from here as well: while a hook is set, every C-ABI call is reported to it
 // with its arguments in the header's order.
 #include <ATen/ATen.h>
+#include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -21,6 +23,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <initializer_list>
+#include <memory>
 #include <string>
 #include <utility>
 #include <vector>
@@ -276,36 +279,79 @@ bool same_ints(PyObject* tuple, at::IntArrayRef v) {
     return true;
 }
 
+// What a kept set of planes was made by: the context of its tensor's storage, so that it lives and goes with the planes (and a
+// copy or an unpickled set, which lacks it, is never taken for one).
+struct PlanesOrigin {
+    Tensor memory;
+    at::cuda::CUDAEvent written;  // recorded behind the split
+    c10::cuda::CUDAStream stream;  // the one that split the weight
+    static void release(void* p) { delete static_cast<PlanesOrigin*>(p); }
+};
+
+Tensor with_origin(const Tensor& planes, const c10::cuda::CUDAStream& stream) {
+    auto origin = std::make_unique<PlanesOrigin>(PlanesOrigin{planes, {}, stream});
+    origin->written.record(stream);
+    void* data = planes.mutable_data_ptr();
+    at::DataPtr hold(data, origin.release(), &PlanesOrigin::release, planes.device());
+    Tensor t = at::detail::make_tensor<at::TensorImpl>(at::Storage(at::Storage::use_byte_size_t(), planes.nbytes(), std::move(hold), nullptr, false),
+                                                       planes.key_set(), planes.dtype());
+    t.unsafeGetTensorImpl()->set_sizes_contiguous(planes.sizes());
+    return t;
+}
+
+bool capturing(void* stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &status) != cudaSuccess) {
+        (void)cudaGetLastError();  // the default stream while a stream that blocks it is captured
+        return true;
+    }
+    return status != cudaStreamCaptureStatusNone;
+}
+
 // The three bf16 planes of an fp32 weight, [N, 3*Kp]. They ride on the weight's Python object (attribute _xg_bf16_planes =
 // (tag, planes)) and are rebuilt when the tag - version counter, address, layout, orientation - changes, so a dense layer's
 // weight is split once in inference and the planes go away with the tensor; a fresh view of a weight is simply split again.
+// A call on another stream than the one that split the weight waits for the split and is recorded with the allocator.
 // In-place updates through weight.data do not move the counter: ops.invalidate_weight_planes drops the planes after those.
-// A captured CUDA graph replays with the planes that existed at capture. Tensors made under torch.inference_mode() have no
-// version counter; their planes are not kept.
-Tensor weight_planes(const Tensor& w, bool trans, int64_t N, int64_t K, void* stream) {
-    const bool tracked = !w.is_inference();
+// While a CUDA graph is captured no kept planes are used and none are kept: the split becomes part of the graph, which so
+// follows the weight (planes made in a capture hold nothing before the first replay, and a graph does not keep tensors alive).
+// Tensors made under torch.inference_mode() have no version counter; their planes are not kept.
+// `keep`: !capturing(stream), asked once per call.
+Tensor weight_planes(const Tensor& w, bool trans, int64_t N, int64_t K, void* stream, bool keep) {
+    const bool tracked = keep && !w.is_inference();
     if (tracked) {
-        Gil gil;
-        PyObject* obj = THPVariable_Wrap(w);
-        PyObject* kept = obj ? PyObject_GetAttrString(obj, "_xg_bf16_planes") : nullptr;
-        if (!kept) PyErr_Clear();
         Tensor hit;
-        if (kept && PyTuple_Check(kept) && PyTuple_GET_SIZE(kept) == 2 && PyTuple_Check(PyTuple_GET_ITEM(kept, 0)) &&
-            PyTuple_GET_SIZE(PyTuple_GET_ITEM(kept, 0)) == 5 && THPVariable_Check(PyTuple_GET_ITEM(kept, 1))) {
-            PyObject* tag = PyTuple_GET_ITEM(kept, 0);
-            if (PyLong_AsLongLong(PyTuple_GET_ITEM(tag, 0)) == (int64_t)w._version() &&
-                PyLong_AsVoidPtr(PyTuple_GET_ITEM(tag, 1)) == w.const_data_ptr() && same_ints(PyTuple_GET_ITEM(tag, 2), w.sizes()) &&
-                same_ints(PyTuple_GET_ITEM(tag, 3), w.strides()) && (PyTuple_GET_ITEM(tag, 4) == Py_True) == trans)
-                hit = THPVariable_Unpack(PyTuple_GET_ITEM(kept, 1));
-            PyErr_Clear();
+        {
+            Gil gil;
+            PyObject* obj = THPVariable_Wrap(w);
+            PyObject* kept = obj ? PyObject_GetAttrString(obj, "_xg_bf16_planes") : nullptr;
+            if (!kept) PyErr_Clear();
+            if (kept && PyTuple_Check(kept) && PyTuple_GET_SIZE(kept) == 2 && PyTuple_Check(PyTuple_GET_ITEM(kept, 0)) &&
+                PyTuple_GET_SIZE(PyTuple_GET_ITEM(kept, 0)) == 5 && THPVariable_Check(PyTuple_GET_ITEM(kept, 1))) {
+                PyObject* tag = PyTuple_GET_ITEM(kept, 0);
+                if (PyLong_AsLongLong(PyTuple_GET_ITEM(tag, 0)) == (int64_t)w._version() &&
+                    PyLong_AsVoidPtr(PyTuple_GET_ITEM(tag, 1)) == w.const_data_ptr() && same_ints(PyTuple_GET_ITEM(tag, 2), w.sizes()) &&
+                    same_ints(PyTuple_GET_ITEM(tag, 3), w.strides()) && (PyTuple_GET_ITEM(tag, 4) == Py_True) == trans)
+                    hit = THPVariable_Unpack(PyTuple_GET_ITEM(kept, 1));
+                PyErr_Clear();
+            }
+            Py_XDECREF(kept);
+            Py_XDECREF(obj);
         }
-        Py_XDECREF(kept);
-        Py_XDECREF(obj);
-        if (hit.defined()) return hit;
+        PlanesOrigin* origin = hit.defined() ? hit.storage().data_ptr().cast_context<PlanesOrigin>(&PlanesOrigin::release) : nullptr;
+        if (origin) {
+            if (origin->stream.stream() != stream) {
+                const c10::cuda::CUDAStream current = c10::cuda::getCurrentCUDAStream(w.device().index());
+                origin->written.block(current);
+                c10::cuda::CUDACachingAllocator::recordStream(origin->memory.storage().data_ptr(), current);
+            }
+            return hit;
+        }
     }
     Tensor w3 = new_tensor({N, 3 * xg_gemm_f32x3_padded_k(K)}, at::kBFloat16, w);
     XG_CALL(xg_split_bf16x3, ptr(w), N, K, row_stride(w), trans ? 0 : 1, mut(w3), stream);
     if (tracked) {
+        w3 = with_origin(w3, c10::cuda::getCurrentCUDAStream(w.device().index()));
         Gil gil;
         PyObject* obj = THPVariable_Wrap(w);
         PyObject* mod = PyImport_ImportModule("xpu_graph_b200.ops");
@@ -338,7 +384,7 @@ Tensor dense(const Tensor& x_in, const Tensor& weight, bool weight_trans, const 
     const int code = code_of(dt), a = act_code(act);
     Tensor out = new_tensor({M, N}, dt, x);
     if (dt == at::kFloat && f32_on_tensor_cores(M, N, K)) {
-        const Tensor w3 = weight_planes(w.t, w.trans, N, K, on.stream);
+        const Tensor w3 = weight_planes(w.t, w.trans, N, K, on.stream, !capturing(on.stream));
         const Tensor a3 = new_tensor({M, 3 * xg_gemm_f32x3_padded_k(K)}, at::kBFloat16, x);
         XG_CALL(xg_split_bf16x3, ptr(x), M, K, row_stride(x), 0, mut(a3), on.stream);
         XG_CALL(xg_gemm_f32x3, ptr(a3), ptr(w3), ptr(bias), ptr(residual), mut(out), M, N, K, N, ldr, a, 0, on.stream);
@@ -572,11 +618,12 @@ Tensor dense_tower(const Tensor& x_in, at::TensorList weights_in, const c10::Lis
     const Tensor x = unit_rows(x_in);
     Tensor a3 = new_tensor({M, 3 * xg_gemm_f32x3_padded_k(dims[0])}, at::kBFloat16, x);
     XG_CALL(xg_split_bf16x3, ptr(x), M, dims[0], row_stride(x), 0, mut(a3), on.stream);
+    const bool keep = !capturing(on.stream);
     for (int i = 0; i < n; ++i) {
         const int64_t K = dims[i], N = dims[i + 1];
         const Tensor wi = unit_rows(w[i]);
         TORCH_CHECK_VALUE((trans[i] ? wi.size(1) : wi.size(0)) == K, "xg_sm100::dense_tower: inner dimensions differ");
-        const Tensor w3 = weight_planes(wi, trans[i], N, K, on.stream);
+        const Tensor w3 = weight_planes(wi, trans[i], N, K, on.stream, keep);
         const Tensor bias = b[i] ? cast(*b[i], at::kFloat).contiguous() : Tensor();
         const bool last = i == n - 1;
         Tensor out = last ? new_tensor({M, N}, at::kFloat, x) : new_tensor({M, 3 * xg_gemm_f32x3_padded_k(N)}, at::kBFloat16, x);
@@ -1056,10 +1103,11 @@ Tensor recommender(const Tensor& features, const Tensor& idx, const Tensor& mask
     if (h.defined()) {
         TORCH_CHECK_VALUE(weights[0].size(1) == k, "xg_sm100::dense: inner dimensions differ");
         const On on(features);
+        const bool keep = !capturing(on.stream);
         for (bool planes = true; planes; ++i) {
             const int64_t N = weights[i].size(0);
             const Tensor w = unit_rows(weights[i]);
-            const Tensor w3 = weight_planes(w, true, N, k, on.stream);
+            const Tensor w3 = weight_planes(w, true, N, k, on.stream, keep);
             const auto b = biases.get(i);
             const Tensor bias = b ? cast(*b, at::kFloat).contiguous() : Tensor();
             planes = on_tensor_cores(i + 1, N);

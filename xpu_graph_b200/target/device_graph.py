@@ -13,8 +13,8 @@ copied into static buffers before each replay (:62-92).
 Two things are added around the reference's lazy runners: a partition whose capture fails at run time (an op that
 synchronises, say) falls back to launch-by-launch execution of that partition instead of failing the call, and
 replayed outputs are cloned by default (``clone_outputs``; the reference returns the static output buffers, which the
-next replay overwrites). Weight planes that the fp32 dense path keeps per weight (weight_planes in csrc/torch_ops.cpp)
-are read as they were at capture. Anything else in the config returns the graph unchanged.
+next replay overwrites). A captured fp32 dense layer splits its weight in every replay (weight_planes in
+csrc/torch_ops.cpp). Anything else in the config returns the graph unchanged.
 """
 from __future__ import annotations
 
