@@ -136,6 +136,15 @@ const void* ptr(const Tensor& t) { return t.defined() ? t.const_data_ptr() : nul
 void* mut(const Tensor& t) { return t.defined() ? t.mutable_data_ptr() : nullptr; }
 const void* ptr(const optional<Tensor>& t) { return t.has_value() ? ptr(*t) : nullptr; }
 
+// The kernels read operands by address and know one set of extents: a tensor on another device, of another dtype or with fewer
+// elements than the extents say would be read past its end. These checks are host compares of a few ns.
+bool elsewhere(const Tensor& x, const Tensor& t) { return t.defined() && t.device() != x.device(); }
+bool elsewhere(const Tensor& x, const optional<Tensor>& t) { return t.has_value() && elsewhere(x, *t); }
+template <typename... T>
+void one_device(const char* who, const Tensor& x, const T&... others) {
+    TORCH_CHECK_VALUE(!(elsewhere(x, others) || ...), "xg_sm100::", who, ": all tensors must be on ", x.device());
+}
+
 // A tensor seen as [rows, cols] with contiguous rows; copied only when its strides do not allow that.
 struct Rows {
     Tensor t;
@@ -177,7 +186,10 @@ template <bool RMS>
 std::pair<Tensor, Tensor> norm(const Tensor& x, const Tensor& residual, const Tensor& weight, const Tensor& bias, double eps,
                                bool want_sum) {
     const On on(x);
+    one_device(RMS ? "rms_norm" : "layer_norm", x, residual, weight, bias);
     const Rows x2(x);
+    TORCH_CHECK_VALUE(weight.numel() == x2.cols && (!bias.defined() || bias.numel() == x2.cols),
+                      "xg_sm100 norm: weight and bias must have one element per column of x");
     optional<Rows> r2;
     if (residual.defined()) {
         TORCH_CHECK_VALUE(residual.sizes() == x.sizes() && residual.scalar_type() == x.scalar_type(),
@@ -230,6 +242,7 @@ Tensor table(const Tensor& t, int64_t S, int64_t D, at::ScalarType dtype) {
 Tensor rope(const Tensor& x_in, const Tensor& cos, const Tensor& sin) {
     TORCH_CHECK_VALUE(x_in.dim() == 4, "xg_sm100::rope expects [B, H, S, D]");
     const On on(x_in);
+    one_device("rope", x_in, cos, sin);
     const Tensor x = x_in.stride(3) == 1 ? x_in : x_in.contiguous();
     const int64_t S = x.size(2), D = x.size(3);
     const Tensor c = table(cos, S, D, x.scalar_type()), s = table(sin, S, D, x.scalar_type());
@@ -242,6 +255,7 @@ Tensor rope(const Tensor& x_in, const Tensor& cos, const Tensor& sin) {
 Tensor swiglu(const Tensor& gate, const Tensor& up) {
     TORCH_CHECK_VALUE(gate.sizes() == up.sizes() && gate.scalar_type() == up.scalar_type(), "xg_sm100::swiglu: gate and up must match");
     const On on(gate);
+    one_device("swiglu", gate, up);
     const Rows g(gate), u(up);
     Tensor out = new_tensor(gate.sizes(), gate.scalar_type(), gate);
     XG_CALL(xg_swiglu, ptr(g.t), ptr(u.t), mut(out), g.rows, g.cols, g.ld, u.ld, g.cols, code_of(gate.scalar_type()), on.stream);
@@ -378,6 +392,11 @@ Tensor dense(const Tensor& x_in, const Tensor& weight, bool weight_trans, const 
     const Weight w = weight_rows(weight, weight_trans);
     const int64_t M = x.size(0), K = x.size(1), N = w.trans ? w.t.size(0) : w.t.size(1);
     TORCH_CHECK_VALUE((w.trans ? w.t.size(1) : w.t.size(0)) == K, "xg_sm100::dense: inner dimensions differ");
+    one_device("dense", x_in, weight, bias_in, residual_in);
+    TORCH_CHECK_VALUE(weight.scalar_type() == dt, "xg_sm100::dense: x and the weight must share a dtype");
+    TORCH_CHECK_VALUE(!bias_in || bias_in->numel() == N, "xg_sm100::dense: the bias must have one element per output column");
+    TORCH_CHECK_VALUE(!residual_in || (residual_in->dim() == 2 && residual_in->size(0) == M && residual_in->size(1) == N),
+                      "xg_sm100::dense: the residual must have the result's shape");
     const Tensor bias = bias_in ? cast(*bias_in, dt).contiguous() : Tensor();
     const Tensor residual = residual_in ? unit_rows(cast(*residual_in, dt)) : Tensor();
     const int64_t ldr = residual.defined() ? row_stride(residual) : 0;
@@ -401,10 +420,14 @@ Tensor dense(const Tensor& x_in, const Tensor& weight, bool weight_trans, const 
 
 Tensor batch_dense(const Tensor& x_in, const Tensor& weight_in, bool weight_trans, const optional<Tensor>& bias_in,
                    const optional<Tensor>& residual_in, c10::string_view act) {
+    TORCH_CHECK_VALUE(x_in.dim() == 3 && weight_in.dim() == 3, "xg_sm100::batch_dense expects 3-D x and weight");
     const On on(x_in);
+    one_device("batch_dense", x_in, weight_in, bias_in, residual_in);
     const at::ScalarType dt = x_in.scalar_type();
     const Tensor x = x_in.contiguous(), w = weight_in.contiguous();
     const int64_t b = x.size(0), M = x.size(1), K = x.size(2), N = weight_trans ? w.size(1) : w.size(2);
+    TORCH_CHECK_VALUE(w.scalar_type() == dt && w.size(0) == b && w.size(weight_trans ? 2 : 1) == K,
+                      "xg_sm100::batch_dense: x and the weight must share a dtype, the batch and the inner dimension");
     const Tensor bias = bias_in ? cast(*bias_in, dt).broadcast_to({b, 1, N}).contiguous() : Tensor();
     const Tensor residual = residual_in ? cast(*residual_in, dt).broadcast_to({b, M, N}).contiguous() : Tensor();
     Tensor out = new_tensor({b, M, N}, dt, x);
@@ -415,7 +438,12 @@ Tensor batch_dense(const Tensor& x_in, const Tensor& weight_in, bool weight_tran
 }
 
 Tensor dense_swiglu(const Tensor& x_in, const Tensor& w_gate, const Tensor& w_up) {
+    TORCH_CHECK_VALUE(x_in.dim() == 2 && w_gate.dim() == 2 && w_gate.sizes() == w_up.sizes() && w_gate.size(1) == x_in.size(1),
+                      "xg_sm100::dense_swiglu expects 2-D x [M, K] and two weights [N, K]");
+    TORCH_CHECK_VALUE(w_gate.scalar_type() == x_in.scalar_type() && w_up.scalar_type() == x_in.scalar_type(),
+                      "xg_sm100::dense_swiglu: x and the weights must share a dtype");
     const On on(x_in);
+    one_device("dense_swiglu", x_in, w_gate, w_up);
     const Tensor x = unit_rows(x_in);
     Tensor g = unit_rows(w_gate), u = unit_rows(w_up);
     if (row_stride(g) != row_stride(u)) {
@@ -429,7 +457,10 @@ Tensor dense_swiglu(const Tensor& x_in, const Tensor& w_gate, const Tensor& w_up
 }
 
 Tensor dense_rope(const Tensor& x_in, const Tensor& weight, const Tensor& cos, const Tensor& sin, int64_t seq_len, int64_t head_dim) {
+    TORCH_CHECK_VALUE(x_in.dim() == 2 && weight.dim() == 2 && weight.size(1) == x_in.size(1) && weight.scalar_type() == x_in.scalar_type(),
+                      "xg_sm100::dense_rope expects 2-D x [M, K] and a weight [N, K] of one dtype");
     const On on(x_in);
+    one_device("dense_rope", x_in, weight, cos, sin);
     const Tensor x = unit_rows(x_in), w = unit_rows(weight);
     const int64_t M = x.size(0), K = x.size(1), N = w.size(0);
     const Tensor c = table(cos, seq_len, head_dim, x.scalar_type()), s = table(sin, seq_len, head_dim, x.scalar_type());
@@ -449,6 +480,7 @@ Buf<int64_t> chain_dims(const Tensor& x, const Weights& ws, int64_t weights_kn, 
         const bool kn = (weights_kn >> l) & 1;
         TORCH_CHECK_VALUE(ws[l].size(kn ? 0 : 1) == dims.back(), "xg_sm100::", who, ": inner dimensions differ");
         TORCH_CHECK_VALUE(ws[l].scalar_type() == x.scalar_type(), "xg_sm100::", who, ": x and the weights must share a dtype");
+        one_device(who, x, ws[l]);
         dims.push_back(ws[l].size(kn ? 1 : 0));
     }
     return dims;
@@ -457,6 +489,7 @@ Buf<int64_t> chain_dims(const Tensor& x, const Weights& ws, int64_t weights_kn, 
 Tensor chain_bias(const optional<Tensor>& b, const Tensor& x, int64_t n, const char* who) {
     if (!b) return {};
     TORCH_CHECK_VALUE(b->numel() == n, "xg_sm100::", who, ": a bias does not match its layer's width");
+    one_device(who, x, b);
     return cast(*b, x.scalar_type()).contiguous();
 }
 
@@ -570,11 +603,16 @@ Tensor dense_tower(const Tensor& x_in, at::TensorList weights_in, const c10::Lis
     bool tensor_cores = dt == at::kFloat;  // every layer qualifies for the fp32 tensor-core path
     for (int i = 0; i < n; ++i) {
         Weight r{weights_in[i], trans_in.get(i)};
+        TORCH_CHECK_VALUE(r.t.dim() == 2 && r.t.size(r.trans ? 1 : 0) == dims.back(), "xg_sm100::dense_tower: inner dimensions differ");
+        TORCH_CHECK_VALUE(r.t.scalar_type() == dt, "xg_sm100::dense_tower: x and the weights must share a dtype");
         dims.push_back(r.trans ? r.t.size(0) : r.t.size(1));
+        const auto bias = biases_in.get(i);
+        TORCH_CHECK_VALUE(!bias || bias->numel() == dims.back(), "xg_sm100::dense_tower: a bias does not match its layer's width");
+        one_device("dense_tower", x_in, r.t, bias);
         if (dt != at::kFloat) r = weight_rows(r.t, r.trans);
         w.push_back(r.t);
         trans.push_back(r.trans);
-        b.push_back(biases_in.get(i));
+        b.push_back(bias);
         tensor_cores = tensor_cores && f32_on_tensor_cores(M, dims[i + 1], dims[i]);
     }
     if (!tensor_cores) {
@@ -622,7 +660,6 @@ Tensor dense_tower(const Tensor& x_in, at::TensorList weights_in, const c10::Lis
     for (int i = 0; i < n; ++i) {
         const int64_t K = dims[i], N = dims[i + 1];
         const Tensor wi = unit_rows(w[i]);
-        TORCH_CHECK_VALUE((trans[i] ? wi.size(1) : wi.size(0)) == K, "xg_sm100::dense_tower: inner dimensions differ");
         const Tensor w3 = weight_planes(wi, trans[i], N, K, on.stream, keep);
         const Tensor bias = b[i] ? cast(*b[i], at::kFloat).contiguous() : Tensor();
         const bool last = i == n - 1;
@@ -635,8 +672,12 @@ Tensor dense_tower(const Tensor& x_in, at::TensorList weights_in, const c10::Lis
 
 // ---- attention -------------------------------------------------------------------------------------------
 Tensor sdpa(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, const optional<Tensor>& mask_in, double scale, bool is_causal) {
-    TORCH_CHECK_VALUE(q_in.dim() == 4, "xg_sm100::sdpa expects 4-D q/k/v");
+    TORCH_CHECK_VALUE(q_in.dim() == 4 && k_in.dim() == 4 && v_in.dim() == 4, "xg_sm100::sdpa expects 4-D q/k/v");
+    TORCH_CHECK_VALUE(k_in.sizes() == v_in.sizes() && k_in.size(0) == q_in.size(0) && k_in.size(1) == q_in.size(1) && k_in.size(3) == q_in.size(3),
+                      "xg_sm100::sdpa: k and v must be [B, H, Skv, D] with q's batch, heads and head dim");
+    TORCH_CHECK_VALUE(k_in.scalar_type() == q_in.scalar_type() && v_in.scalar_type() == q_in.scalar_type(), "xg_sm100::sdpa: q, k and v must share a dtype");
     const On on(q_in);
+    one_device("sdpa", q_in, k_in, v_in, mask_in);
     const Tensor q = unit_rows(q_in), k = unit_rows(k_in), v = unit_rows(v_in);
     const int64_t B = q.size(0), H = q.size(1), Sq = q.size(2), D = q.size(3), Skv = k.size(2);
     Tensor m;
@@ -680,8 +721,9 @@ struct Segments {
     }
 };
 
-Tensor mask_bytes(const optional<Tensor>& mask, int64_t rows) {
+Tensor mask_bytes(const optional<Tensor>& mask, int64_t rows, const Tensor& like) {
     if (!mask) return {};
+    one_device("row mask", like, mask);
     TORCH_CHECK_VALUE(mask->numel() == rows, "xg_sm100: row mask must have one entry per row");
     const Tensor m = mask->contiguous();
     // a bool holds 0 or 1 in one byte: read as it is
@@ -722,7 +764,7 @@ Tensor slice_cat_impl(const Tensor& src_in, at::IntArrayRef starts, at::IntArray
         parts[masked && !masked->get(i) ? 0 : 1].add(ptr(src), segs[i].first * es, ld, mut(out), off * es, total * es, len * es);
         off += len;
     }
-    const Tensor mask = mask_bytes(row_mask, rows);
+    const Tensor mask = mask_bytes(row_mask, rows, src);
     if (!parts[0].src.empty()) parts[0].copy(rows, {}, zero_when, on.stream);
     if (!parts[1].src.empty()) parts[1].copy(rows, mask, zero_when, on.stream);
     return out;
@@ -763,7 +805,7 @@ Tensor multi_slice_impl(const Tensor& src, at::IntArrayRef starts_in, int64_t sl
     Segments parts[2];
     for (int64_t k = 0; k < num; ++k)
         parts[masked && !masked->get(k) ? 0 : 1].add(ptr(s.t), starts[k] * es, s.ld * es, mut(out), k * slab, slice_len * es, slice_len * es);
-    const Tensor mask = mask_bytes(row_mask, s.rows);
+    const Tensor mask = mask_bytes(row_mask, s.rows, src);
     if (!parts[0].src.empty()) parts[0].copy(s.rows, {}, zero_when, on.stream);
     if (!parts[1].src.empty()) parts[1].copy(s.rows, mask, zero_when, on.stream);
     return out;
@@ -814,6 +856,7 @@ Tensor cat_lastdim(at::TensorList xs, const optional<Tensor>& row_mask, bool zer
         parts.emplace_back(x);
         TORCH_CHECK_VALUE(x.scalar_type() == xs[0].scalar_type() && parts.back().rows == parts[0].rows,
                           "xg_sm100::cat_lastdim: inputs must agree in dtype and leading dims");
+        one_device("cat_lastdim", xs[0], x);
         total += parts.back().cols;
     }
     Buf<int64_t> shape(xs[0].sizes().begin(), xs[0].sizes().end());
@@ -825,7 +868,7 @@ Tensor cat_lastdim(at::TensorList xs, const optional<Tensor>& row_mask, bool zer
         all.add(ptr(p.t), 0, p.ld * es, mut(out), off * es, total * es, p.cols * es);
         off += p.cols;
     }
-    all.copy(rows, mask_bytes(row_mask, rows), zero_when, on.stream);
+    all.copy(rows, mask_bytes(row_mask, rows, xs[0]), zero_when, on.stream);
     return out;
 }
 
@@ -841,6 +884,7 @@ Tensor gather_stack(at::TensorList tables, const Tensor& idx, const optional<Ten
     for (const Tensor& t : tables) {
         TORCH_CHECK_VALUE(t.dim() == 2 && t.size(1) == D && t.scalar_type() == tables[0].scalar_type(),
                           "xg_sm100::gather_stack: tables must be 2-D with one embedding dim and dtype");
+        one_device("gather_stack", idx, t);
         if (t.is_contiguous()) {
             ptrs.push_back(ptr(t));
         } else {
@@ -850,7 +894,7 @@ Tensor gather_stack(at::TensorList tables, const Tensor& idx, const optional<Ten
         table_rows.push_back(t.size(0));
     }
     Tensor out = new_tensor({rows, F * D}, tables[0].scalar_type(), idx);
-    const Tensor mask = mask_bytes(row_mask, rows);
+    const Tensor mask = mask_bytes(row_mask, rows, idx);
     XG_CALL(xg_gather_rows, ptrs.data(), table_rows.data(), F, static_cast<const int64_t*>(ptr(idx)), idx.stride(0), idx.stride(1),
             static_cast<const uint8_t*>(ptr(mask)), zero_when ? 1 : 0, mut(out), rows, D, F * D, (int)out.element_size(), on.stream);
     return out;
@@ -867,6 +911,7 @@ std::vector<Tensor> sum3d(at::TensorList inputs, int64_t dim) {
     for (const Tensor& x_in : inputs) {
         TORCH_CHECK_VALUE(x_in.dim() == 3, "xg_sm100::sum3d expects 3-D tensors");
         TORCH_CHECK_VALUE(x_in.scalar_type() == inputs[0].scalar_type(), "xg_sm100::sum3d: inputs must share a dtype");
+        one_device("sum3d", inputs[0], x_in);
         xs.push_back(x_in.contiguous());
         const int64_t s0 = x_in.size(0), s1 = x_in.size(1), s2 = x_in.size(2);
         shapes.append({s0, s1, s2});
@@ -891,6 +936,8 @@ struct RowSums {
         const Tensor x = x_in.contiguous();
         TORCH_CHECK_VALUE(x.dim() == 3 && x.size(2) == C && x.scalar_type() == dtype && (x.size(0) == 1 || x.size(0) == batch),
                           "xg_sm100::rowsum_cat: operands must be [batch or 1, rows, C] tensors of one dtype");
+        if (!keep.empty()) one_device("rowsum_cat", keep[0], x, y_in);
+        else one_device("rowsum_cat", x, y_in);
         a.push_back(ptr(x));
         a_bs.push_back(x.size(0) == 1 && batch != 1 ? 0 : x.size(1) * C);
         keep.push_back(x);
@@ -996,6 +1043,7 @@ bool qkv_rope(const Tensor& x_in, const Tensor& wq, const Tensor& wk, const Tens
     }
     if (!xg_gemm_rope_group_worth_it(count, M, N, K)) return false;
     const On on(x_in);
+    one_device("decoder_layer", x_in, wq, wk, wv, cos, sin);
     const Tensor x = unit_rows(x_in);
     if ((reinterpret_cast<uintptr_t>(ptr(x)) & 15u) != 0 || row_stride(x) % 8 != 0) return false;
     const Tensor c = table(cos, S, D, dt), s = table(sin, S, D, dt);
@@ -1055,10 +1103,12 @@ Tensor recommender_planes(const Tensor& features, const Tensor& idx, const Tenso
         return {};
     const int64_t rows = features.size(0), ld = row_stride(features), D = tables[0].dim() == 2 ? tables[0].size(1) : 0;
     auto aligned = [](const Tensor& t) { return (reinterpret_cast<uintptr_t>(ptr(t)) & 15u) == 0; };
+    one_device("recommender", features, idx, mask);
     if (features.numel() == 0 || idx.size(0) != rows || mask.numel() != rows || D == 0 || D % 4 != 0 || D > 1 << 20 || ld % 4 != 0 || !aligned(features)) return {};
     Buf<const void*> ptrs;
     Buf<int64_t> table_rows, first, len;
     for (const Tensor& t : tables) {
+        one_device("recommender", features, t);
         if (t.dim() != 2 || t.size(1) != D || t.scalar_type() != at::kFloat || !t.is_contiguous() || !aligned(t) || t.size(0) > 0x7fffffff ||
             t.numel() == 0)
             return {};
@@ -1075,7 +1125,7 @@ Tensor recommender_planes(const Tensor& features, const Tensor& idx, const Tenso
     if (cols > 4096 || (rows > 1 && ld < features.size(1))) return {};
     *K = cols + F * D;
     const On on(features);
-    const Tensor hide = mask_bytes(mask, rows);
+    const Tensor hide = mask_bytes(mask, rows, features);
     Tensor out = new_tensor({rows, 3 * xg_gemm_f32x3_padded_k(*K)}, at::kBFloat16, features);
     XG_CALL(xg_gather_planes, ptr(features), ld, first.data(), len.data(), (int64_t)first.size(), ptrs.data(), table_rows.data(), F,
             static_cast<const int64_t*>(ptr(idx)), idx.stride(0), idx.stride(1), static_cast<const uint8_t*>(ptr(hide)), 1, mut(out), rows, D,
@@ -1107,9 +1157,9 @@ Tensor recommender(const Tensor& features, const Tensor& idx, const Tensor& mask
         for (bool planes = true; planes; ++i) {
             const int64_t N = weights[i].size(0);
             const Tensor w = unit_rows(weights[i]);
+            one_device("recommender", features, w);
             const Tensor w3 = weight_planes(w, true, N, k, on.stream, keep);
-            const auto b = biases.get(i);
-            const Tensor bias = b ? cast(*b, at::kFloat).contiguous() : Tensor();
+            const Tensor bias = chain_bias(biases.get(i), features, N, "recommender");
             planes = on_tensor_cores(i + 1, N);
             Tensor out = planes ? new_tensor({M, 3 * xg_gemm_f32x3_padded_k(N)}, at::kBFloat16, h) : new_tensor({M, N}, at::kFloat, h);
             XG_CALL(xg_gemm_f32x3, ptr(h), ptr(w3), ptr(bias), nullptr, mut(out), M, N, k, N, 0, act_code("relu"), planes ? 1 : 0, on.stream);

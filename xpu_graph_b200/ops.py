@@ -314,6 +314,8 @@ def combo_dense(inputs: List[torch.Tensor], weights: List[torch.Tensor], weight_
     T = len(inputs)
     if T == 0 or len(weights) != T or len(biases) != T:
         raise ValueError("xg_sm100::combo_dense: one input, weight and bias entry per layer")
+    if any(t is not None and t.device != inputs[0].device for t in (*inputs, *weights, *biases)):
+        raise ValueError(f"xg_sm100::combo_dense: all tensors must be on {inputs[0].device}")
     grouped = _combo_dense_grouped(inputs, weights, weight_trans, biases, act)
     if grouped is not None:
         return grouped
