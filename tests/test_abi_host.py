@@ -111,6 +111,22 @@ def test_ops_have_no_cpu_kernel():
         torch.ops.xg_sm100.rms_norm(torch.zeros(2, 8), torch.ones(8), 1e-6)
 
 
+def test_libraries_share_the_cxx_runtime():
+    """Neither library carries a C++ runtime of its own: with a static copy in the operators' library, formatting a number into
+    an error message ended the process (stream objects of libtorch's copy, functions of the other)."""
+    import shutil
+    import subprocess
+
+    if not shutil.which("readelf"):
+        pytest.skip("readelf is not installed")
+    for path in (lib.LIB_PATH, lib.TORCH_LIB_PATH):
+        needed = subprocess.run(["readelf", "-d", path], capture_output=True, text=True, check=True).stdout
+        assert "libstdc++.so.6" in needed, path
+        symbols = subprocess.run(["readelf", "--dyn-syms", "-W", path], capture_output=True, text=True, check=True).stdout
+        own = [line for line in symbols.splitlines() if " _ZNSo9_M_insertI" in line and " UND " not in line]
+        assert not own, own[:3]
+
+
 def test_stack_or_view_reuses_slabs_of_one_buffer():
     """Operands of a combo dense call that are consecutive slabs of one buffer are used in place; anything else is
     stacked (host logic only, no GPU needed)."""

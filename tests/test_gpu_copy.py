@@ -62,6 +62,16 @@ def test_multi_slice(cuda_device, shape, starts, length, dtype):
     assert_bit_exact(got, ref_ops.multi_slice(src, starts, length), f"multi_slice {shape}")
 
 
+def test_multi_slice_refuses_slices_outside_the_row(cuda_device):
+    """The operator's own refusal, whose message names the slice and the row (numbers in an error message)."""
+    from xpu_graph_b200 import ops
+
+    with pytest.raises(ValueError, match="slice at 60 of length 8 is outside a row of 64 elements"):
+        ops.multi_slice(torch.zeros(8, 64, device=cuda_device), [60], 8)
+    with pytest.raises(ValueError, match="negative slice length -1"):
+        ops.multi_slice(torch.zeros(8, 64, device=cuda_device), [0], -1)
+
+
 def test_slice_cat_multi(cuda_device):
     from xpu_graph_b200.modules import FuseSliceCatSameInputModule_v2
 

@@ -122,8 +122,11 @@ def build(force: bool = False, verbose: bool = False) -> str:
         import torch
 
         torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+        # The C++ runtime by its file name: a compiler that finds no libstdc++.so of its own takes libstdc++.a without a word, and
+        # streams that cross between that copy and libtorch's end the process (an error message with a number in it did).
         _link([os.environ.get("CXX", "g++"), "-shared", "-o", TORCH_LIB_PATH, torch_obj, f"-L{HERE}", "-l:libxg_sm100.so", "-Wl,-rpath,$ORIGIN",
-               f"-L{torch_lib}", f"-Wl,-rpath,{torch_lib}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch_python"])
+               f"-L{torch_lib}", f"-Wl,-rpath,{torch_lib}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch_python",
+               "-l:libstdc++.so.6"])
     return LIB_PATH
 
 
