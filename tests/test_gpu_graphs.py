@@ -216,3 +216,25 @@ def test_llama_layer_equals_its_op_sequence(cuda_device, batch, seq, hidden, spl
     torch.cuda.synchronize()
     assert lib.tc_status() == 0
     assert torch.equal(got.view(rows, hidden), want)
+
+
+def test_graph_operators_refuse_projections_of_another_width(cuda_device):
+    """A q / k / v projection that is wider or narrower than its heads is an error (its columns used to be reinterpreted), and so
+    is a number of heads that does not divide the width."""
+    from xpu_graph_b200 import ops
+
+    bf = dict(dtype=torch.bfloat16, device=cuda_device)
+    x, cos, sin = torch.zeros(1, 16, 512, **bf), torch.zeros(16, 128, **bf), torch.zeros(16, 128, **bf)
+    t = lambda *s: torch.zeros(*s, **bf)  # noqa: E731
+    for i, width in ((1, 1024), (2, 256), (3, 1024), (3, 256)):
+        w = [t(512), t(512, 512), t(512, 512), t(512, 512), t(512, 512), t(512), t(1376, 512), t(1376, 512), t(512, 1376)]
+        w[i] = t(width, 512)
+        with pytest.raises((RuntimeError, ValueError)):
+            ops.decoder_layer(x, cos, sin, w, 1e-5, 1e-5, 4, True, True)
+    for qkv, heads in ((2048, 4), (1024, 4), (1536, 0), (1536, 5)):
+        p = [t(512), t(512), t(qkv, 512), t(qkv), t(512, 512), t(512), t(512), t(512), t(1024, 512), t(1024), t(512, 1024), t(512)]
+        with pytest.raises((RuntimeError, ValueError)):
+            ops.encoder_block(x, p, 1e-5, 1e-5, heads)
+    w = [t(512), t(512, 512), t(512, 512), t(512, 512), t(512, 512), t(512), t(1376, 512), t(1376, 512), t(512, 1376)]
+    with pytest.raises((RuntimeError, ValueError)):
+        ops.decoder_layer(x, cos, sin, w, 1e-5, 1e-5, 0, True, True)

@@ -994,9 +994,16 @@ Tensor mul_sum_cat(at::TensorList lhs, at::TensorList rhs) {
 // The fused op sequences of fused_graphs.py as one operator each. With a Python frame, a module call, an operator dispatch
 // and several tensor views per kernel the host needed 90-105 us for the seven to nine launches of a small graph, more than
 // the kernels; from here a launch costs 4 us. The operators are for inference only: nothing below is seen by autograd.
-Tensor heads_view(const Tensor& rows, int64_t B, int64_t S, int64_t H, int64_t D, int64_t col0) {
+// Part `part` of `parts` side by side (packed q, k, v) of the rows of a projection as [B, H, S, D].
+Tensor heads_view(const Tensor& rows, int64_t B, int64_t S, int64_t H, int64_t D, int part = 0, int parts = 1) {
+    TORCH_CHECK(rows.size(0) == B * S && rows.size(1) == parts * H * D, "xg_sm100: a projection of ", rows.size(1), " columns is not ", parts, " x ", H,
+                " heads of ", D);
     const int64_t ld = rows.stride(0);
-    return rows.as_strided({B, H, S, D}, {S * ld, D, ld, 1}, rows.storage_offset() + col0);
+    return rows.as_strided({B, H, S, D}, {S * ld, D, ld, 1}, rows.storage_offset() + part * H * D);
+}
+int64_t head_dim(int64_t hidden, int64_t heads, const char* who) {
+    TORCH_CHECK_VALUE(heads > 0 && hidden % heads == 0, "xg_sm100::", who, ": ", hidden, " columns are not ", heads, " heads");
+    return hidden / heads;
 }
 Tensor heads_to_rows(const Tensor& a, int64_t rows, int64_t cols) { return a.transpose(1, 2).reshape({rows, cols}); }
 
@@ -1007,10 +1014,10 @@ Tensor encoder_block(const Tensor& x, const c10::List<optional<Tensor>>& params,
     TORCH_CHECK_VALUE(x.dim() == 3 && params.size() == 12, "xg_sm100::encoder_block: x is [B, S, hidden], params are six (weight, bias) pairs");
     auto weight = [&](int i) -> Tensor { return params.get(2 * i).value(); };
     auto bias = [&](int i) -> optional<Tensor> { return params.get(2 * i + 1); };
-    const int64_t B = x.size(0), S = x.size(1), C = x.size(2), D = C / heads, T = B * S;
+    const int64_t B = x.size(0), S = x.size(1), C = x.size(2), D = head_dim(C, heads, "encoder_block"), T = B * S;
     const Tensor x0 = x.reshape({T, C});
     const Tensor qkv = dense(norm<false>(x0, {}, weight(0), or_none(bias(0)), eps1, false).first, weight(1), true, bias(1), std::nullopt, "none");
-    const Tensor a = sdpa(heads_view(qkv, B, S, heads, D, 0), heads_view(qkv, B, S, heads, D, C), heads_view(qkv, B, S, heads, D, 2 * C),
+    const Tensor a = sdpa(heads_view(qkv, B, S, heads, D, 0, 3), heads_view(qkv, B, S, heads, D, 1, 3), heads_view(qkv, B, S, heads, D, 2, 3),
                           std::nullopt, 1.0 / std::sqrt((double)D), false);
     const Tensor x1 = dense(heads_to_rows(a, T, C), weight(2), true, bias(2), x0, "none");
     const Tensor h = dense(norm<false>(x1, {}, weight(3), or_none(bias(3)), eps2, false).first, weight(4), true, bias(4), std::nullopt, "gelu");
@@ -1066,7 +1073,7 @@ Tensor decoder_layer(const Tensor& x, const Tensor& cos, const Tensor& sin, at::
                      bool fuse_rope, bool fuse_swiglu) {
     at::AutoDispatchBelowADInplaceOrView no_grad;
     TORCH_CHECK_VALUE(x.dim() == 3 && w.size() == 9, "xg_sm100::decoder_layer: x is [B, S, hidden], nine weights");
-    const int64_t B = x.size(0), S = x.size(1), C = x.size(2), D = C / heads, T = B * S;
+    const int64_t B = x.size(0), S = x.size(1), C = x.size(2), D = head_dim(C, heads, "decoder_layer"), T = B * S;
     const Tensor x0 = x.reshape({T, C});
     auto linear = [&](const Tensor& in, const Tensor& weight, const optional<Tensor>& residual) {
         return dense(in, weight, true, std::nullopt, residual, "none");
@@ -1074,17 +1081,17 @@ Tensor decoder_layer(const Tensor& x, const Tensor& cos, const Tensor& sin, at::
     const Tensor h = norm<true>(x0, {}, w[0], {}, eps1, false).first;
     Tensor q, k, v;
     if (fuse_rope && qkv_rope(h, w[1], w[2], w[3], cos, sin, S, D, &q, &k, &v)) {
-        q = heads_view(q, B, S, heads, D, 0);
-        k = heads_view(k, B, S, heads, D, 0);
-        if (v.defined()) v = heads_view(v, B, S, heads, D, 0);
+        q = heads_view(q, B, S, heads, D);
+        k = heads_view(k, B, S, heads, D);
+        if (v.defined()) v = heads_view(v, B, S, heads, D);
     } else if (fuse_rope) {
-        q = heads_view(dense_rope(h, w[1], cos, sin, S, D), B, S, heads, D, 0);
-        k = heads_view(dense_rope(h, w[2], cos, sin, S, D), B, S, heads, D, 0);
+        q = heads_view(dense_rope(h, w[1], cos, sin, S, D), B, S, heads, D);
+        k = heads_view(dense_rope(h, w[2], cos, sin, S, D), B, S, heads, D);
     } else {
-        q = rope(heads_view(linear(h, w[1], std::nullopt), B, S, heads, D, 0), cos, sin);
-        k = rope(heads_view(linear(h, w[2], std::nullopt), B, S, heads, D, 0), cos, sin);
+        q = rope(heads_view(linear(h, w[1], std::nullopt), B, S, heads, D), cos, sin);
+        k = rope(heads_view(linear(h, w[2], std::nullopt), B, S, heads, D), cos, sin);
     }
-    if (!v.defined()) v = heads_view(linear(h, w[3], std::nullopt), B, S, heads, D, 0);
+    if (!v.defined()) v = heads_view(linear(h, w[3], std::nullopt), B, S, heads, D);
     const Tensor a = sdpa(q, k, v, std::nullopt, 1.0 / std::sqrt((double)D), true);
     const Tensor x1 = linear(heads_to_rows(a, T, C), w[4], x0);
     const Tensor h2 = norm<true>(x1, {}, w[5], {}, eps2, false).first;
