@@ -14,6 +14,9 @@ def _t(*shape, dt=torch.bfloat16, dev="cuda"):
 
 F32 = torch.float32
 BAD = {
+    "mul_sum_cat: a second operand is missing": lambda X: X.mul_sum_cat([_t(4, 3, 8)] * 2, [_t(4, 3, 8)]),
+    "slice_sum_cat: an end is missing": lambda X: X.slice_sum_cat(_t(4, 9, 8), [0, 3], [3]),
+    "dense_tower: no layers": lambda X: X.dense_tower(_t(4, 8), [], [], [], ""),
     "norm: weight too short": lambda X: X.rms_norm(_t(4, 64), _t(32), 1e-5),
     "norm: bias too short": lambda X: X.layer_norm(_t(4, 64), _t(64), _t(1), 1e-5),
     "norm: weight on the host": lambda X: X.rms_norm(_t(4, 64), _t(64, dev="cpu"), 1e-5),

@@ -589,7 +589,7 @@ Tensor dense_tower(const Tensor& x_in, at::TensorList weights_in, const c10::Lis
                    c10::string_view act_names) {
     const auto acts = split_names(act_names);
     const int n = (int)weights_in.size();
-    TORCH_CHECK_VALUE(acts.size() == (size_t)n && trans_in.size() == (size_t)n && biases_in.size() == (size_t)n,
+    TORCH_CHECK_VALUE(n > 0 && acts.size() == (size_t)n && trans_in.size() == (size_t)n && biases_in.size() == (size_t)n,
                       "xg_sm100::dense_tower: one weight, orientation, bias and activation per layer");
     const at::ScalarType dt = x_in.scalar_type();
     TORCH_CHECK_VALUE(x_in.dim() == 2 && (dt == at::kFloat || dt == at::kBFloat16 || dt == at::kHalf),
@@ -966,7 +966,7 @@ struct RowSums {
 
 Tensor slice_sum_cat(const Tensor& src, at::IntArrayRef starts, at::IntArrayRef ends) {
     TORCH_CHECK_VALUE(src.dim() == 3, "xg_sm100::slice_sum_cat expects a 3-D tensor");
-    TORCH_CHECK_VALUE(!starts.empty(), "xg_sm100::slice_sum_cat: no ranges");
+    TORCH_CHECK_VALUE(!starts.empty() && starts.size() <= ends.size(), "xg_sm100::slice_sum_cat: one end per start, and at least one of them");
     RowSums sums(src.size(0), src);
     const Tensor x = src.contiguous();
     for (const auto& r : clamp_slices(src.size(1), starts, ends)) sums.add(x, {}, r.first, r.second);
@@ -981,8 +981,8 @@ Tensor sum_cat(at::TensorList inputs) {
 }
 
 Tensor mul_sum_cat(at::TensorList lhs, at::TensorList rhs) {
-    TORCH_CHECK_VALUE(!lhs.empty(), "xg_sm100::mul_sum_cat: no operands");
-    const size_t n = std::min(lhs.size(), rhs.size());
+    TORCH_CHECK_VALUE(!lhs.empty() && lhs.size() <= rhs.size(), "xg_sm100::mul_sum_cat: one second operand per first, and at least one of them");
+    const size_t n = lhs.size();
     int64_t batch = 0;
     for (size_t i = 0; i < n; ++i) batch = std::max({batch, lhs[i].size(0), rhs[i].size(0)});
     RowSums sums(batch, lhs[0]);
