@@ -238,3 +238,30 @@ def test_graph_operators_refuse_projections_of_another_width(cuda_device):
     w = [t(512), t(512, 512), t(512, 512), t(512, 512), t(512, 512), t(512), t(1376, 512), t(1376, 512), t(512, 1376)]
     with pytest.raises((RuntimeError, ValueError)):
         ops.decoder_layer(x, cos, sin, w, 1e-5, 1e-5, 0, True, True)
+
+
+def test_graph_operators_are_inference_only(cuda_device):
+    """A backward through a graph operator is an error, as through every other operator of the library; the fused classes run
+    without gradients."""
+    from xpu_graph_b200 import ops
+    from xpu_graph_b200.fused_graphs import FusedEncoderBlock
+    from xpu_graph_b200.workloads import make_encoder
+
+    model, x = make_encoder(seed=0)
+    model, x = model.to(cuda_device), x.to(cuda_device)
+    params = []
+    for m in (model.ln1, model.qkv, model.proj, model.ln2, model.fc1, model.fc2):
+        params += (m.weight, m.bias)
+    args = (params, model.ln1.eps, model.ln2.eps, model.heads)
+    y = ops.encoder_block(x, *args)  # the parameters require gradients
+    assert y.requires_grad
+    with pytest.raises(RuntimeError, match="encoder_block"):
+        y.sum().backward()
+    fused = FusedEncoderBlock(model)(x.requires_grad_())
+    assert not fused.requires_grad and torch.equal(fused, y.detach())
+    with torch.no_grad():
+        assert not ops.encoder_block(x, *args).requires_grad
+    import torch.autograd.forward_ad as fwd
+
+    with fwd.dual_level(), pytest.raises(NotImplementedError, match="forward-mode"):
+        ops.encoder_block(fwd.make_dual(x.detach(), torch.ones_like(x)), *args)

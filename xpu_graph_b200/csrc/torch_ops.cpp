@@ -16,6 +16,9 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/autograd_not_implemented_fallback.h>
+#include <torch/csrc/autograd/forward_grad.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/library.h>
 
@@ -1180,6 +1183,41 @@ Tensor recommender(const Tensor& features, const Tensor& idx, const Tensor& mask
     return h;
 }
 
+// The autograd kernels of the graph operators: inference only, like the other operators, so that a backward through one of them
+// is an error instead of a gradient that is missing without a word. By hand, since the general fallback boxes its arguments:
+// some forty tensors, a tenth of what a small graph costs.
+void collect(at::TensorList& all, std::vector<Tensor>& out) { out.insert(out.end(), all.begin(), all.end()); }
+void collect(const Tensor& t, std::vector<Tensor>& out) { out.push_back(t); }
+void collect(const c10::List<optional<Tensor>>& all, std::vector<Tensor>& out) {
+    for (size_t i = 0; i < all.size(); ++i) out.push_back(or_none(all.get(i)));
+}
+template <typename T>
+void collect(const T&, std::vector<Tensor>&) {}
+
+template <auto Op>
+struct GraphAutograd;
+template <typename... A, Tensor (*Op)(A...)>
+struct GraphAutograd<Op> {
+    static inline const char* name = nullptr;
+    static Tensor call(c10::DispatchKeySet keys, A... args) {
+        static auto op = c10::Dispatcher::singleton().findSchemaOrThrow(name, "").template typed<Tensor(A...)>();
+        Tensor out = [&] {
+            at::AutoDispatchBelowAutograd below;
+            return op.redispatch(keys & c10::after_autograd_keyset, args...);
+        }();
+        const bool forward_mode = torch::autograd::ForwardADLevel::try_get_by_idx(0) != nullptr;
+        if (at::GradMode::is_enabled() || forward_mode) {
+            std::vector<Tensor> inputs;
+            (collect(args, inputs), ...);
+            for (const Tensor& t : inputs)
+                TORCH_CHECK_NOT_IMPLEMENTED(!forward_mode || !t.defined() || !t._fw_grad(0).defined(), name, " has no forward-mode derivative");
+            if (torch::autograd::compute_requires_grad(inputs))
+                torch::autograd::set_history(out, std::make_shared<torch::autograd::NotImplemented>(name, torch::autograd::collect_next_edges(inputs)));
+        }
+        return out;
+    }
+};
+
 // ---- registration --------------------------------------------------------------------------------------------
 const char* const kSchemas[] = {
     "rms_norm(Tensor x, Tensor weight, float eps) -> Tensor",
@@ -1270,10 +1308,11 @@ TORCH_LIBRARY_IMPL(xg_sm100, Autograd, m) {
         const std::string schema(s);
         m.impl(schema.substr(0, schema.find('(')).c_str(), torch::autograd::autogradNotImplementedFallback());
     }
-    for (const char* s : kGraphSchemas) {
-        const std::string schema(s);
-        m.impl(schema.substr(0, schema.find('(')).c_str(), torch::CppFunction::makeFallthrough());
-    }
+#define XG_GRAPH_IMPL(op) GraphAutograd<&op>::name = "xg_sm100::" #op, m.impl(#op, TORCH_FN(GraphAutograd<&op>::call))
+    XG_GRAPH_IMPL(encoder_block);
+    XG_GRAPH_IMPL(decoder_layer);
+    XG_GRAPH_IMPL(recommender);
+#undef XG_GRAPH_IMPL
 }
 
 // lib.call_hook: Python callables (or None) that see every C-ABI call made from this file. Called with the GIL held.

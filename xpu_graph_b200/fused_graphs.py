@@ -37,7 +37,8 @@ class FusedLlamaDecoderLayer(nn.Module):
         L = self.layer
         weights = [L.input_norm.weight, L.q_proj.weight, L.k_proj.weight, L.v_proj.weight, L.o_proj.weight, L.post_norm.weight,
                    L.gate_proj.weight, L.up_proj.weight, L.down_proj.weight]
-        return _decoder_layer(x, cos, sin, weights, self.eps1, self.eps2, self.heads, self.fuse_rope_gemm, self.fuse_swiglu_gemm)
+        with torch.no_grad():
+            return _decoder_layer(x, cos, sin, weights, self.eps1, self.eps2, self.heads, self.fuse_rope_gemm, self.fuse_swiglu_gemm)
 
 
 class FusedEncoderBlock(nn.Module):
@@ -52,7 +53,8 @@ class FusedEncoderBlock(nn.Module):
         params = []
         for m in (b.ln1, b.qkv, b.proj, b.ln2, b.fc1, b.fc2):
             params += (m.weight, m.bias)
-        return _encoder_block(x, params, b.ln1.eps, b.ln2.eps, b.heads)
+        with torch.no_grad():
+            return _encoder_block(x, params, b.ln1.eps, b.ln2.eps, b.heads)
 
 
 class FusedRecsysGraph(nn.Module):
@@ -74,4 +76,5 @@ class FusedRecsysGraph(nn.Module):
         if len(tables) != len(G.tables):
             tables = list(G.tables)
         weights, biases = [m.weight for m in G.layers], [m.bias for m in G.layers]
-        return _recommender(dense, idx, mask, tables, self.starts, self.ends, weights, biases)
+        with torch.no_grad():
+            return _recommender(dense, idx, mask, tables, self.starts, self.ends, weights, biases)
