@@ -936,6 +936,16 @@ def test_dense_operands_copied_into_addressable_rows(cuda_device, M, K, N, weigh
     assert_parity(got, want.cpu(), f"dense {M}x{K}x{N} {dtype} through copies")
 
 
+@pytest.mark.parametrize("K", [2097120, 2097121, 2200001])
+def test_dense_fp32_long_kn_weights(cuda_device, K):
+    """A [K, N] weight of more rows than 65535 tiles of 32 (it is copied into [N, K] first). Bound as in test_dense_fp32_fma_tiles."""
+    g = torch.Generator().manual_seed(53)
+    x, w = torch.randn(2, K, generator=g), torch.randn(K, 3, generator=g)
+    out = torch.ops.xg_sm100.dense(x.to(cuda_device), w.to(cuda_device), False, None, None, "none")
+    diff = (out.cpu().double() - x.double() @ w.double()).abs()
+    assert (diff <= 4 * K ** 0.5 * 2.0 ** -24 * (x.double().square() @ w.double().square()).sqrt()).all(), diff.max().item()
+
+
 def _planes(x):
     """fp32 -> its three bf16 planes, as fp32 tensors."""
     a = x.bfloat16().float()

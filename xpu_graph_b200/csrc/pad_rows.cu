@@ -47,13 +47,14 @@ __global__ void __launch_bounds__(256) pad_rows16_kernel(const uint16_t* __restr
     }
 }
 
-// out[r][c] = src[c][r] through a 32 x 32 tile of shared memory; 256 threads as 8 rows of 32.
+// out[r][c] = src[c][r] through a 32 x 32 tile of shared memory; 256 threads as 8 rows of 32. One grid dimension: the second one
+// ends at 65535 tiles, which 2,097,120 columns fill.
 template <typename U>
 __global__ void __launch_bounds__(256) pad_transpose_kernel(const U* __restrict__ src, int64_t rows, int64_t cols, int64_t ld,
-                                                            U* __restrict__ out, int64_t out_ld) {
+                                                            U* __restrict__ out, int64_t out_ld, unsigned row_tiles) {
     pdl_sync();
     __shared__ U tile[32][33];
-    const int64_t r0 = (int64_t)blockIdx.x * 32, c0 = (int64_t)blockIdx.y * 32;
+    const int64_t r0 = (int64_t)(blockIdx.x % row_tiles) * 32, c0 = (int64_t)(blockIdx.x / row_tiles) * 32;
     const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < 32; k += 8)
@@ -79,14 +80,14 @@ extern "C" int xg_pad_rows(const void* src, int64_t rows, int64_t cols, int64_t 
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (transpose) {
         const int64_t gx = (rows + 31) / 32, gy = (out_ld + 31) / 32;
-        if (gx > 0x7fffffffLL || gy > 65535) return fail(XG_ERR_TOO_LARGE, "xg_pad_rows: extent too large");
-        const dim3 grid((unsigned)gx, (unsigned)gy);
+        if (gx > 0x7fffffffLL / gy) return fail(XG_ERR_TOO_LARGE, "xg_pad_rows: extent too large");
+        const unsigned grid = (unsigned)(gx * gy);
         if (elem_size == 4)
             launch(pad_transpose_kernel<uint32_t>, grid, 256, 0, st, reinterpret_cast<const uint32_t*>(src), rows, cols, ld,
-                   reinterpret_cast<uint32_t*>(out), out_ld);
+                   reinterpret_cast<uint32_t*>(out), out_ld, (unsigned)gx);
         else
             launch(pad_transpose_kernel<uint16_t>, grid, 256, 0, st, reinterpret_cast<const uint16_t*>(src), rows, cols, ld,
-                   reinterpret_cast<uint16_t*>(out), out_ld);
+                   reinterpret_cast<uint16_t*>(out), out_ld, (unsigned)gx);
     } else {
         const int64_t blocks = (rows * (out_ld * elem_size / 16) + 255) / 256, cap = 16LL * num_sms();
         const unsigned grid = (unsigned)(blocks < cap ? blocks : cap);
