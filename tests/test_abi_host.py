@@ -210,3 +210,27 @@ def test_small_m_plan_and_tower_routing_without_gpu():
     assert not ops.mlp_small_worth_it(16384, (128, 64, 32), torch.float32) and ops.mlp_small_worth_it(2048, (128, 64, 32), torch.float32)
     assert ops._small_run((20, 32, 16, 1), 0, 3, torch.float16, 16) == 3 and ops._small_run((512, 32, 16, 1), 0, 3, torch.float16, 16) == 1
     assert ops._small_run((512, 32, 16, 1), 1, 3, torch.float16, 16) == 2
+
+
+def test_routing_rules_are_the_operators_own():
+    """The rules that choose between the fp32 kernels are stated once: setting a limit through ops moves the operators' decision
+    and the rewrites' alike."""
+    import torch
+
+    from xpu_graph_b200 import ops
+
+    native = lib.load_torch_ops()
+    assert ops.F32_TENSOR_MIN_FLOPS == 1 << 30 and ops.F32_TENSOR_MAX_K == 8192
+    assert native.xg_torch_f32_on_tensor_cores(1024, 512, 1024) and not native.xg_torch_f32_on_tensor_cores(1023, 512, 1024)
+    assert not native.xg_torch_f32_on_tensor_cores(65536, 512, 8193)
+    flops, max_k = ops.F32_TENSOR_MIN_FLOPS, ops.F32_TENSOR_MAX_K
+    try:
+        ops.F32_TENSOR_MIN_FLOPS, ops.F32_TENSOR_MAX_K = 1 << 20, 1000
+        for M, N, K in ((64, 64, 128), (64, 64, 127), (512, 512, 1000), (512, 512, 1001)):
+            want = 2 * M * N * K >= 1 << 20 and K <= 1000
+            assert bool(native.xg_torch_f32_on_tensor_cores(M, N, K)) == want == ops._f32_on_tensor_cores(M, N, K)
+            assert ops.dense_tower_eligible(M, [K, N]) == want
+    finally:
+        ops.F32_TENSOR_MIN_FLOPS, ops.F32_TENSOR_MAX_K = flops, max_k
+    assert not ops._f32_on_tensor_cores(64, 64, 128)
+    assert not ops.mlp_small_worth_it(16, (20, 32), torch.int64) and not ops.mlp_small_worth_it(16, (20,), torch.float32)

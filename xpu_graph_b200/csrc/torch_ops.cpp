@@ -33,6 +33,32 @@
 
 #include "../../include/xg_sm100.h"
 
+// ---- routing rules, also asked by ops.py for the graph rewrites -------------------------------------
+// fp32 dense layers above this many FLOPs run on the bf16 tensor cores from three bf16 planes per operand (fp32-grade results at
+// several times the FMA rate); smaller ones stay on the FMA kernel, whose launch is cheaper. ops.F32_TENSOR_MIN_FLOPS sets it.
+extern "C" {
+int64_t xg_torch_f32_min_flops = []() {
+    const char* set = std::getenv("XG_F32_TENSOR_MIN_FLOPS");
+    return set ? (int64_t)std::atoll(set) : (int64_t)1 << 30;
+}();
+int64_t xg_torch_f32_max_k = 8192;  // measured error vs fp64 grows from 2e-6 (K = 1728) to 6e-6 (K = 4096) of the output scale
+}
+
+extern "C" int xg_torch_f32_on_tensor_cores(int64_t M, int64_t N, int64_t K) {
+    if (2 * M * N * K < xg_torch_f32_min_flops || K > xg_torch_f32_max_k) return 0;
+    const char* e = std::getenv("XG_F32_TENSOR");
+    return !(e && e[0] == '0' && e[1] == 0);
+}
+
+// The one-launch FMA tower (dims: layers + 1 widths) is the faster form where a launch per layer is mostly launch and latency: few
+// rows, or very narrow layers (figures: ops.mlp_small_worth_it).
+extern "C" int xg_torch_small_tower_worth_it(int64_t M, const int64_t* dims, int layers, int dtype) {
+    if (!xg_mlp_small_supported(dims, layers, dtype)) return 0;
+    int64_t weights = 0;
+    for (int l = 0; l < layers; ++l) weights += (dims[l] + 3) / 4 * 4 * dims[l + 1];
+    return M <= 2048 || weights <= 4096;
+}
+
 namespace {
 
 using at::Tensor;
@@ -278,16 +304,7 @@ Weight weight_rows(const Tensor& w, bool trans) {
     return {unit_rows(w), trans};
 }
 
-bool f32_on_tensor_cores(int64_t M, int64_t N, int64_t K) {
-    static const int64_t min_flops = []() {
-        const char* e = std::getenv("XG_F32_TENSOR_MIN_FLOPS");
-        return e ? (int64_t)std::atoll(e) : (int64_t)1 << 30;
-    }();
-    constexpr int64_t max_k = 8192;  // measured error vs fp64 grows from 2e-6 (K = 1728) to 6e-6 (K = 4096) of the output scale
-    if (2 * M * N * K < min_flops || K > max_k) return false;
-    const char* e = std::getenv("XG_F32_TENSOR");
-    return !(e && e[0] == '0' && e[1] == 0);
-}
+bool f32_on_tensor_cores(int64_t M, int64_t N, int64_t K) { return xg_torch_f32_on_tensor_cores(M, N, K) != 0; }
 
 bool same_ints(PyObject* tuple, at::IntArrayRef v) {
     if (!PyTuple_Check(tuple) || (size_t)PyTuple_GET_SIZE(tuple) != v.size()) return false;
@@ -579,15 +596,6 @@ Tensor mlp_small(const Tensor& x, at::TensorList weights, const c10::List<option
     return mlp_small_impl(x, Weights(weights.begin(), weights.end()), b, acts, weights_kn);
 }
 
-// The one-launch FMA tower is the faster form where a launch per layer is mostly launch and latency: few rows, or very
-// narrow layers (the figures are at ops.mlp_small_worth_it, which states the same rule for the graph rewrites).
-bool small_tower_worth_it(int64_t M, const int64_t* dims, int layers, int dtype) {
-    if (!xg_mlp_small_supported(dims, layers, dtype)) return false;
-    int64_t weights = 0;
-    for (int l = 0; l < layers; ++l) weights += (dims[l] + 3) / 4 * 4 * dims[l + 1];
-    return M <= 2048 || weights <= 4096;
-}
-
 Tensor dense_tower(const Tensor& x_in, at::TensorList weights_in, const c10::List<bool>& trans_in, const c10::List<optional<Tensor>>& biases_in,
                    c10::string_view act_names) {
     const auto acts = split_names(act_names);
@@ -643,7 +651,7 @@ Tensor dense_tower(const Tensor& x_in, at::TensorList weights_in, const c10::Lis
             }
             int run = 1;
             for (int r = 3; r >= 2 && run == 1; --r)
-                if (i + r <= n && small_tower_worth_it(M, &dims[i], r, code)) run = r;
+                if (i + r <= n && xg_torch_small_tower_worth_it(M, &dims[i], r, code)) run = r;
             if (run > 1)
                 y = mlp_small_impl(y, Weights(w.begin() + i, w.begin() + i + run), OptList(b.begin() + i, b.begin() + i + run),
                                    Buf<c10::string_view>(acts.begin() + i, acts.begin() + i + run), kn(run));

@@ -144,8 +144,15 @@ def load_torch_ops() -> ctypes.PyDLL:
                 raise XgLibraryError(f"cannot load {TORCH_LIB_PATH}: {e}") from e
             lib.xg_torch_set_hook.argtypes = [ctypes.py_object, ctypes.py_object]
             lib.xg_torch_set_hook.restype = None
+            lib.xg_torch_f32_on_tensor_cores.argtypes = [c_int64, c_int64, c_int64]
+            lib.xg_torch_small_tower_worth_it.argtypes = [c_int64, _I64P, c_int, c_int]
             _torch_lib = lib
     return _torch_lib
+
+
+def torch_setting(name: str) -> c_int64:
+    """A 64-bit variable of libxg_sm100_torch.so."""
+    return c_int64.in_dll(load_torch_ops(), name)
 
 
 def last_error() -> str:

@@ -11,7 +11,8 @@ Registration pattern follows passes/patterns/targets/mlu/triton_kernel/fused_sli
 """
 from __future__ import annotations
 
-import os
+import sys
+import types
 from typing import List, Optional, Sequence
 
 import torch
@@ -158,16 +159,33 @@ def _weight_rows(w: torch.Tensor, weight_trans: bool):
     return _mat(w), weight_trans
 
 
-# fp32 dense layers above this many FLOPs run on the bf16 tensor cores from three bf16 planes per operand
-# (fp32-grade results at several times the FMA rate); smaller ones stay on the FMA kernel, whose launch is cheaper.
-F32_TENSOR_MIN_FLOPS = int(os.environ.get("XG_F32_TENSOR_MIN_FLOPS", str(1 << 30)))
-F32_TENSOR_MAX_K = 8192  # measured error vs fp64 grows from 2e-6 (K = 1728) to 6e-6 (K = 4096) of the output scale
-
-
+# Which fp32 dense layers run on the tensor cores is decided in one place, csrc/torch_ops.cpp; F32_TENSOR_MIN_FLOPS and
+# F32_TENSOR_MAX_K are its variables under these names (see _Settings below), so that setting one moves operators and rewrites alike.
 def _f32_on_tensor_cores(M: int, N: int, K: int) -> bool:
-    if os.environ.get("XG_F32_TENSOR", "1") == "0":
-        return False
-    return 2 * M * N * K >= F32_TENSOR_MIN_FLOPS and K <= F32_TENSOR_MAX_K
+    return bool(_lib.load_torch_ops().xg_torch_f32_on_tensor_cores(int(M), int(N), int(K)))
+
+
+class _Settings(types.ModuleType):
+    """This module's type."""
+
+    @property
+    def F32_TENSOR_MIN_FLOPS(self) -> int:
+        return _lib.torch_setting("xg_torch_f32_min_flops").value
+
+    @F32_TENSOR_MIN_FLOPS.setter
+    def F32_TENSOR_MIN_FLOPS(self, value: int) -> None:
+        _lib.torch_setting("xg_torch_f32_min_flops").value = int(value)
+
+    @property
+    def F32_TENSOR_MAX_K(self) -> int:
+        return _lib.torch_setting("xg_torch_f32_max_k").value
+
+    @F32_TENSOR_MAX_K.setter
+    def F32_TENSOR_MAX_K(self, value: int) -> None:
+        _lib.torch_setting("xg_torch_f32_max_k").value = int(value)
+
+
+sys.modules[__name__].__class__ = _Settings
 
 
 def _planes_tag(weight: torch.Tensor, weight_trans: bool):
@@ -243,10 +261,9 @@ def mlp_small_worth_it(M: int, dims: Sequence[int], dtype: torch.dtype) -> bool:
     """The one-launch FMA tower is the faster form where a launch per layer is mostly launch and latency: few rows, or
     very narrow layers. Measured on B200 (us, one kernel / a launch per layer): 16 rows of 20 -> 32 -> 16 -> 1 fp16
     8.3 / 26.5; 16384 rows of 64 -> 32 -> 16 -> 1 fp32 20.5 / 21.7; 16384 rows of 128 -> 64 -> 32 fp32 43.5 / 24.6."""
-    if not mlp_small_eligible(dims, dtype):
+    if dtype not in _DTYPE_CODE or not 1 <= len(dims) - 1 <= 3:
         return False
-    weights = sum(((dims[i] + 3) // 4 * 4) * dims[i + 1] for i in range(len(dims) - 1))
-    return M <= 2048 or weights <= 4096
+    return bool(_lib.load_torch_ops().xg_torch_small_tower_worth_it(int(M), _lib.i64_array(list(dims)), len(dims) - 1, _DTYPE_CODE[dtype]))
 
 
 def mlp_small_eligible(dims: Sequence[int], dtype: torch.dtype) -> bool:
