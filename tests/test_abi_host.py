@@ -234,3 +234,27 @@ def test_routing_rules_are_the_operators_own():
         ops.F32_TENSOR_MIN_FLOPS, ops.F32_TENSOR_MAX_K = flops, max_k
     assert not ops._f32_on_tensor_cores(64, 64, 128)
     assert not ops.mlp_small_worth_it(16, (20, 32), torch.int64) and not ops.mlp_small_worth_it(16, (20,), torch.float32)
+
+
+def test_operators_library_of_another_torch_is_stale(monkeypatch):
+    """A library built against another torch, Python or C++ ABI is rebuilt, and refused by name when it is loaded all the same."""
+    from xpu_graph_b200 import build
+
+    stamp = build._read_stamp()
+    if not stamp:
+        pytest.skip("the objects were not built here")
+    assert build.built_for() == build.torch_abi()
+    calls = []
+    monkeypatch.setattr(build, "_compile_torch_ops", lambda src, obj: calls.append("compile") or "")
+    monkeypatch.setattr(build, "_compile_one", lambda *a: "")
+    monkeypatch.setattr(build, "_link", lambda cmd: calls.append(os.path.basename(cmd[cmd.index("-o") + 1])))
+    monkeypatch.setattr(build, "torch_abi", lambda: "torch 0.0, C++11 ABI 1, other")
+    monkeypatch.setattr(lib, "_torch_lib", None)
+    with pytest.raises(lib.XgLibraryError, match="was built against torch"):
+        lib.load_torch_ops()
+    try:
+        build.build()
+        assert calls[0] == "compile" and calls[-1] == "libxg_sm100_torch.so"
+    finally:
+        with open(build.TORCH_STAMP, "w") as f:
+            f.write(stamp)

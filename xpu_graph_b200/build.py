@@ -19,6 +19,7 @@ OBJ_DIR = os.path.join(CSRC, "build")
 LIB_PATH = os.path.join(HERE, "libxg_sm100.so")
 TORCH_LIB_PATH = os.path.join(HERE, "libxg_sm100_torch.so")
 TORCH_SOURCE = "torch_ops.cpp"
+TORCH_STAMP = os.path.join(OBJ_DIR, "torch_ops.stamp")  # what the operators' library was built against
 
 SOURCES = [
     "abi.cu",
@@ -51,6 +52,35 @@ def _nvcc() -> str:
     if not os.path.exists(cand):
         raise RuntimeError("nvcc not found; set NVCC or put it on PATH")
     return cand
+
+
+def torch_abi() -> str:
+    """What the operators' library has to agree on with the process that loads it."""
+    import sysconfig
+
+    import torch
+
+    return f"torch {torch.__version__}, C++11 ABI {int(torch._C._GLIBCXX_USE_CXX11_ABI)}, {sysconfig.get_config_var('SOABI')}"
+
+
+def _torch_stamp() -> str:
+    import torch
+
+    # (the library's run path names torch's folder)
+    return f"{torch_abi()}\n{os.path.dirname(torch.__file__)}\n{os.environ.get('CXX', 'g++')}\n"
+
+
+def _read_stamp() -> str:
+    try:
+        with open(TORCH_STAMP) as f:
+            return f.read()
+    except OSError:
+        return ""
+
+
+def built_for() -> str:
+    """torch_abi() of the build, empty when that is not known."""
+    return _read_stamp().split("\n")[0]
 
 
 def _cuda_home() -> str:
@@ -109,6 +139,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
     kernels = [job(name) for name in SOURCES]
     torch_src, torch_obj, torch_stale = job(TORCH_SOURCE)
+    torch_stale = torch_stale or _read_stamp() != _torch_stamp()
     with cf.ThreadPoolExecutor(max_workers=8) as pool:
         futs = [pool.submit(_compile_torch_ops, torch_src, torch_obj)] if torch_stale else []
         futs += [pool.submit(_compile_one, nvcc, s, o, verbose) for s, o, stale in kernels if stale]
@@ -127,6 +158,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
         _link([os.environ.get("CXX", "g++"), "-shared", "-o", TORCH_LIB_PATH, torch_obj, f"-L{HERE}", "-l:libxg_sm100.so", "-Wl,-rpath,$ORIGIN",
                f"-L{torch_lib}", f"-Wl,-rpath,{torch_lib}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch_python",
                "-l:libstdc++.so.6"])
+        with open(TORCH_STAMP, "w") as f:
+            f.write(_torch_stamp())
     return LIB_PATH
 
 

@@ -133,11 +133,16 @@ def load_torch_ops() -> ctypes.PyDLL:
     global _torch_lib
     import torch  # noqa: F401  (the library links against it)
 
+    from . import build
+
     load()
     with _lock:
         if _torch_lib is None:
             if not os.path.exists(TORCH_LIB_PATH):
                 raise XgLibraryError(f"{TORCH_LIB_PATH} not found: build it with `python -m xpu_graph_b200.build`.")
+            built, here = build.built_for(), build.torch_abi()
+            if built and built != here:
+                raise XgLibraryError(f"{TORCH_LIB_PATH} was built against {built}, this is {here}: `python -m xpu_graph_b200.build`.")
             try:
                 lib = ctypes.PyDLL(TORCH_LIB_PATH)
             except OSError as e:  # pragma: no cover - depends on the environment
