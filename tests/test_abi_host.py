@@ -258,3 +258,20 @@ def test_operators_library_of_another_torch_is_stale(monkeypatch):
     finally:
         with open(build.TORCH_STAMP, "w") as f:
             f.write(stamp)
+
+
+def test_operands_are_copied_where_that_was_measured_to_pay():
+    """From which K operands that no tensor map addresses are copied: the measured points on both sides of every line (148 SMs)."""
+    L = lib.load()
+
+    def copied(M, K, N, trans, dtype):
+        return L.xg_gemm_copy_bytes(4096, 4096, M, N, K, K, K if trans else N, 1 if trans else 0, dtype) > 0
+
+    for M, N, trans, dtype, k in ((64, 1000, True, lib.XG_BF16, 96), (256, 5000, False, lib.XG_F16, 96), (2048, 504, True, lib.XG_BF16, 96),
+                                  (2048, 500, True, lib.XG_BF16, 128), (1000, 1001, False, lib.XG_F16, 128), (300, 3500, True, lib.XG_BF16, 240),
+                                  (2048, 500, False, lib.XG_F32, 96), (2048, 500, True, lib.XG_F32, 224), (640, 1003, True, lib.XG_F32, 128),
+                                  (256, 1000, True, lib.XG_F32, 96), (1500, 1500, True, lib.XG_F32, 96), (8192, 1000, True, lib.XG_F32, 96)):
+        for K in range(k - 9, k + 10):
+            if K % (4 if dtype == lib.XG_F32 else 8):  # rows that no tensor map addresses
+                assert copied(M, K, N, trans, dtype) == (K >= k), (M, N, K, trans, dtype)
+    assert not copied(2048, 512, 500, True, lib.XG_F32)  # addressable as they are

@@ -63,16 +63,34 @@ int validate_gemm(const char* name, const void* A, const void* B, const void* re
 
 // Which operands of a dense layer are copied into 16-byte rows before the kernels that want such rows (TMA-fed: tensor
 // cores for 16-bit types, FMA for fp32, which also wants its weights as [N, K]), and the row pitch of each copy.
-// From K = 96 on: the scalar-load kernel that takes the operands as they are needs about 1.2 us per 16 elements of K
-// (2 x 731 x 5280 fp16: 52 us), the copies and the fast kernel together 9-15 us.
 struct OperandCopies {
     bool a = false, b = false, turn_b = false;
     int64_t a_ld = 0, b_ld = 0, a_rows = 0, b_rows = 0, b_cols = 0, a_bytes = 0, b_bytes = 0;
 };
+
+// The K from which copies and the fast kernel are ahead of the scalar-load kernel that reads the operands in place. Measured on B200
+// (us, copies / in place, launches of a CUDA graph):
+//   up to one 64 x 64 tile per SM, or more than two: even at K = 97..113, then the in-place kernel's 1 us (3 us with more than two
+//     tiles per SM) per 16 elements of K decide: bf16 64 x 1000 10.0 / 11.6 at K = 97, 10.4 / 23.3 at 257; 1 x 33 9.5 / 8.9 and
+//     10.0 / 19.5; 256 x 5000 13.2 / 26.2 and 14.4 / 54.8; fp32 256 x 1000 8.9 / 10.0 and 12.8 / 19.0.
+//   one to two tiles per SM is where the in-place kernel is at its best, and two kinds of layer come later there:
+//   - 16-bit results whose rows are no multiples of 16 bytes leave the fast kernel element by element: 2048 x 500 bf16 17.7 / 14.4
+//     at 97, 17.0 / 17.4 at 129; 1000 x 1001 17.6 / 14.5, 17.9 / 17.4; where its 128 x 64 tiles need two waves 300 x 3500
+//     27.0 / 14.3, 27.5 / 28.7 at 257.
+//   - fp32 layers with [N, K] weights, whose fast kernel has the same FMA rate: 2048 x 500 15.7 / 13.4 at 97, 22.2 / 20.9 at 193,
+//     26.2 / 26.0 at 257; 512 x 2000 23.6 / 23.6 at 225; at the beginning of that range 640 x 1003 15.3 / 15.6 at 129.
+int64_t copies_from_k(int64_t M, int64_t N, int trans_b, int dtype) {
+    const int64_t sms = num_sms(), tiles = ((M + 63) / 64) * ((N + 63) / 64);
+    if (tiles <= sms || tiles > 2 * sms) return 96;
+    if (dtype == XG_F32) return !trans_b ? 96 : (5 * tiles <= 6 * sms ? 128 : 224);
+    if (N % 8 == 0) return 96;
+    return ((M + 127) / 128) * ((N + 63) / 64) <= sms ? 128 : 240;
+}
+
 OperandCopies plan_copies(const void* A, const void* B, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int trans_b, int dtype) {
     OperandCopies c;
     const int es = dtype_size(dtype);
-    if (es == 0 || K < 96 || M <= 0 || N <= 0) return c;
+    if (es == 0 || M <= 0 || N <= 0 || K < copies_from_k(M, N, trans_b, dtype)) return c;
     const int64_t unit = 16 / es;
     c.turn_b = dtype == XG_F32 && !trans_b;
     c.a = lda % unit != 0 || !aligned16(A);
