@@ -18,7 +18,7 @@ def cuda_device():
 
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
-    from xpu_graph_b200 import lib
+    from xpu_graph_b200 import lib, ops  # noqa: F401  (registers torch.ops.xg_sm100)
 
     L = lib.load()  # raises if the library is missing: GPU tests never run on a silent fallback
     assert L.xg_device_arch_ok(torch.cuda.current_device()) == 1, "kernels are built for sm_100a only"

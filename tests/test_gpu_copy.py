@@ -8,7 +8,7 @@ import pytest
 import torch
 
 from oracle import ref_ops
-from tests.helpers import assert_bit_exact
+from tests.helpers import LaunchCounter, assert_bit_exact
 
 pytestmark = pytest.mark.gpu
 
@@ -218,11 +218,13 @@ def test_recommender_forms(cuda_device):
     mask = (torch.rand(rows, 1, generator=g) < 0.3).to(cuda_device)
     wide = torch.randn(rows, 65, generator=g).to(cuda_device)
 
-    def check(feats, idx, tables, starts, ends, dims):
+    def check(feats, idx, tables, starts, ends, dims, planes):
         k = sum(e - s for s, e in zip(starts, ends)) + F * D
         ws = [(torch.randn(n, m, generator=g) * m ** -0.5).to(cuda_device) for m, n in zip([k] + dims, dims)]
         bs = [torch.randn(n, generator=g).to(cuda_device) for n in dims]
-        got = torch.ops.xg_sm100.recommender(feats, idx, mask, tables, starts, ends, ws, bs)
+        with LaunchCounter() as calls:
+            got = torch.ops.xg_sm100.recommender(feats, idx, mask, tables, starts, ends, ws, bs)
+        assert ("xg_gather_planes" in calls.names) == planes and ("xg_gather_rows" in calls.names) != planes
         emb = torch.stack([t[idx[:, f]] for f, t in enumerate(tables)], 1).masked_fill(mask[:, :, None], 0).flatten(1)
         h = torch.cat([feats[:, s:e] for s, e in zip(starts, ends)] + [emb], 1).double()
         for w, b in zip(ws, bs):
@@ -234,8 +236,8 @@ def test_recommender_forms(cuda_device):
 
     even = wide[:, :64].contiguous()
     for dims in ([1024, 1024, 256], [1024, 64], [1024]):  # planes to planes, planes to the FMA layers, one layer
-        check(even, idx, tables, [32, 0], [64, 32], dims)
-    check(even, idx, tables, [1, 30], [30, 64], [1024])
-    check(wide[:, 1:], idx, tables, [32, 0], [64, 32], [1024])
-    check(wide.t().contiguous().t(), idx, tables, [0], [64], [1024])
-    check(even, idx.t().contiguous().t(), [t.t().contiguous().t() for t in tables], [0], [64], [1024])
+        check(even, idx, tables, [32, 0], [64, 32], dims, True)
+    check(even, idx, tables, [1, 30], [30, 64], [1024], False)
+    check(wide[:, 1:], idx, tables, [32, 0], [64, 32], [1024], False)
+    check(wide.t().contiguous().t(), idx, tables, [0], [64], [1024], False)
+    check(even, idx.t().contiguous().t(), [t.t().contiguous().t() for t in tables], [0], [64], [1024], False)

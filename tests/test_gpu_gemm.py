@@ -915,8 +915,11 @@ def test_dense_fp32_fma_tiles(cuda_device, M, K, N, with_res):
                                                        (260, 96, 31, False, 0)])
 def test_dense_operands_copied_into_addressable_rows(cuda_device, M, K, N, weight_trans, offset, dtype):
     """Row lengths and bases that are no multiples of 16 bytes, [K, N] weights: the operands are copied into rows the fast
-    kernels can address inside the one call; same result as with the scratch withheld (the kernel that reads them in place)."""
+    kernels can address inside the one call; same result as with the scratch withheld (the kernel that reads them in place) and as
+    64-bit math."""
     from xpu_graph_b200 import lib
+
+    code = {torch.float32: lib.XG_F32, torch.bfloat16: lib.XG_BF16, torch.float16: lib.XG_F16}[dtype]
 
     g = torch.Generator().manual_seed(52)
     flat = torch.randn(M * K + offset, generator=g).to(dtype).to(cuda_device)
@@ -929,11 +932,13 @@ def test_dense_operands_copied_into_addressable_rows(cuda_device, M, K, N, weigh
     assert calls.names == ["xg_gemm_bias_act_ws"]
     want = torch.empty_like(got)
     L = lib.load()
+    copied = L.xg_gemm_copy_bytes(x.data_ptr(), w.data_ptr(), M, N, K, x.stride(0), w.stride(0), 1 if weight_trans else 0, code)
+    assert copied > 0, "a case whose operands are copied"
     lib.check(L.xg_gemm_bias_act(x.data_ptr(), w.data_ptr(), b.data_ptr(), None, want.data_ptr(), M, N, K, x.stride(0), w.stride(0), N, 0,
-                                 1 if weight_trans else 0, lib.ACT_CODES["silu"],
-                                 {torch.float32: lib.XG_F32, torch.bfloat16: lib.XG_BF16, torch.float16: lib.XG_F16}[dtype],
-                                 torch.cuda.current_stream().cuda_stream), "xg_gemm_bias_act")
+                                 1 if weight_trans else 0, lib.ACT_CODES["silu"], code, torch.cuda.current_stream().cuda_stream), "xg_gemm_bias_act")
     assert_parity(got, want.cpu(), f"dense {M}x{K}x{N} {dtype} through copies")
+    exact = torch.nn.functional.silu(x.double() @ (w.double().t() if weight_trans else w.double()) + b.double())
+    assert_parity(got, exact.to(dtype).cpu(), f"dense {M}x{K}x{N} {dtype} through copies, 64-bit math")
 
 
 @pytest.mark.parametrize("K", [2097120, 2097121, 2200001])

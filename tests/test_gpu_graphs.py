@@ -265,3 +265,63 @@ def test_graph_operators_are_inference_only(cuda_device):
 
     with fwd.dual_level(), pytest.raises(NotImplementedError, match="forward-mode"):
         ops.encoder_block(fwd.make_dual(x.detach(), torch.ones_like(x)), *args)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_traced_layouts_are_the_real_ones(cuda_device, dtype):
+    """What the compiler is told about attention's and RoPE's results (shape, strides, dtype) is what the operators return, for the
+    layouts that projections leave: packed q, k, v, separate buffers, contiguous heads, one head, one position, broadcast heads."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    X = torch.ops.xg_sm100
+    rnd = lambda *s: torch.randn(*s, device=cuda_device).to(dtype)  # noqa: E731
+    packed = rnd(2, 40, 3, 4, 64)
+    layouts = {
+        "packed": [packed[:, :, i].transpose(1, 2) for i in range(3)],
+        "packed by head": [rnd(2, 40, 4, 3, 64)[:, :, :, i].transpose(1, 2) for i in range(3)],
+        "projections": [rnd(2, 40, 4, 64).transpose(1, 2) for _ in range(3)],
+        "contiguous": [rnd(2, 4, 40, 64) for _ in range(3)],
+        "one head": [rnd(2, 40, 1, 64).transpose(1, 2) for _ in range(3)],
+        "one position": [rnd(2, 1, 4, 64).transpose(1, 2) for _ in range(3)],
+        "broadcast heads": [rnd(2, 1, 40, 64).expand(2, 4, 40, 64) for _ in range(3)],
+        "strided elements": [rnd(2, 4, 64, 40).transpose(2, 3) for _ in range(3)],
+    }
+    for name, (q, k, v) in layouts.items():
+        cos, sin = rnd(q.shape[2], 64), rnd(q.shape[2], 64)
+        mask = torch.rand(2, 1, 1, k.shape[2], device=cuda_device) < 0.9
+        calls = [lambda q, k, v, c, s, m: X.sdpa(q, k, v, None, 0.125, False), lambda q, k, v, c, s, m: X.sdpa(q, k, v, m, 0.125, True),
+                 lambda q, k, v, c, s, m: X.rope(q, c, s)]
+        for i, call in enumerate(calls):
+            real = call(q, k, v, cos, sin, mask)
+            with FakeTensorMode() as mode:
+                fake = call(*(mode.from_tensor(t) for t in (q, k, v, cos, sin, mask)))
+            assert (fake.shape, fake.stride(), fake.dtype, fake.device) == (real.shape, real.stride(), real.dtype, real.device), (name, i)
+
+
+@pytest.mark.parametrize("dynamic", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_modules_compile_to_the_same_bits(cuda_device, dtype, dynamic):
+    """The replacement modules under torch.compile (traced through the operators' fake implementations, run by their CUDA
+    kernels) give the bits of the same modules called one by one, also when the batch is a symbol."""
+    from xpu_graph_b200 import modules as M
+
+    H, D, S = 4, 64, 37
+    C = H * D
+    dense, norm, sdpa = M.DenseLayerModule(False), M.RMSNormModule(), M.SDPAModule()
+
+    def block(x, g, w_qkv, b_qkv, w_o):
+        B = x.shape[0]
+        h = norm(x.reshape(B * S, C), g, 1e-5)
+        qkv = dense(h, w_qkv, True, b_qkv, "none").view(B, S, 3, H, D)
+        q, k, v = (qkv[:, :, i].transpose(1, 2) for i in range(3))
+        a = sdpa(q, k, v, None, 0.125, True).transpose(1, 2).reshape(B * S, C)
+        return dense(a, w_o, True, None, "gelu").view(B, S, C)
+
+    rnd = lambda *s: torch.randn(*s, device=cuda_device).to(dtype) * 0.05  # noqa: E731
+    weights = (rnd(C), rnd(3 * C, C), rnd(3 * C), rnd(C, C))
+    torch._dynamo.reset()
+    compiled = torch.compile(block, backend="aot_eager", fullgraph=True, dynamic=dynamic)
+    with torch.no_grad():
+        for B in (2, 5, 3) if dynamic else (2,):
+            x = rnd(B, S, C)
+            assert torch.equal(compiled(x, *weights), block(x, *weights))
