@@ -325,3 +325,46 @@ def test_modules_compile_to_the_same_bits(cuda_device, dtype, dynamic):
         for B in (2, 5, 3) if dynamic else (2,):
             x = rnd(B, S, C)
             assert torch.equal(compiled(x, *weights), block(x, *weights))
+
+
+@pytest.mark.parametrize("rows,mlp", [(500, (1024, 512, 256)), (4096, (1024, 512, 256)), (40, (64, 32))])
+def test_recommender_equals_its_op_sequence(cuda_device, rows, mlp):
+    """The recommender's operator gives the bits of the replacement modules called one after the other: all layers on the tensor
+    cores, some of them, none."""
+    from xpu_graph_b200 import modules as M
+    from xpu_graph_b200.fused_graphs import FusedRecsysGraph
+    from xpu_graph_b200.workloads import RecsysGraph
+
+    torch.manual_seed(5)
+    graph = RecsysGraph(64, 16, 26, 64, 1000, mlp).to(cuda_device)
+    dense, idx = torch.randn(rows, 64, device=cuda_device), torch.randint(0, 1000, (rows, 26), device=cuda_device)
+    mask = torch.rand(rows, 1, device=cuda_device) < 0.3
+    fused = FusedRecsysGraph(graph)
+    with torch.no_grad():
+        h = M.CatLastDimModule()([M.FuseSliceCatSameInputModule()(dense, list(zip(fused.starts, fused.ends))),
+                                  M.GatherStackModule()(list(graph.tables), idx, mask, True)])
+        for layer in graph.layers:
+            h = M.DenseLayerModule(False)(h, layer.weight, True, layer.bias, "relu")
+    assert torch.equal(fused(dense, idx, mask), h)
+
+
+@pytest.mark.parametrize("batch,seq,dtype", [(2, 128, torch.float32), (3, 197, torch.float16), (24, 197, torch.bfloat16)])
+def test_encoder_block_equals_its_op_sequence(cuda_device, batch, seq, dtype):
+    """The encoder block's operator gives the bits of the replacement modules called one after the other."""
+    from xpu_graph_b200 import modules as M
+    from xpu_graph_b200.fused_graphs import FusedEncoderBlock
+    from xpu_graph_b200.workloads import make_encoder
+
+    b, _ = make_encoder(seed=0)
+    b = b.to(cuda_device).to(dtype)
+    C, H, T = b.ln1.weight.shape[0], b.heads, batch * seq
+    x = torch.randn(batch, seq, C, device=cuda_device).to(dtype)
+    norm, dense, res = M.LayerNormModule(), M.DenseLayerModule(False), M.DenseResidualModule()
+    with torch.no_grad():
+        x0 = x.reshape(T, C)
+        qkv = dense(norm(x0, b.ln1.weight, b.ln1.bias, b.ln1.eps), b.qkv.weight, True, b.qkv.bias, "none").view(batch, seq, 3, H, C // H)
+        a = M.SDPAModule()(*(qkv[:, :, i].transpose(1, 2) for i in range(3)), None, None, False).transpose(1, 2).reshape(T, C)
+        x1 = res(a, b.proj.weight, True, b.proj.bias, x0, "none")
+        h = dense(norm(x1, b.ln2.weight, b.ln2.bias, b.ln2.eps), b.fc1.weight, True, b.fc1.bias, "gelu")
+        want = res(h, b.fc2.weight, True, b.fc2.bias, x1, "none")
+    assert torch.equal(FusedEncoderBlock(b)(x).view(T, C), want)
