@@ -644,7 +644,8 @@ constexpr int PAIR_BN = 256;
 constexpr int PAIR_STAGES = 6;
 // EPI_WARPS: sixteen where the products of a tile do not cover its epilogue (K <= 1024: 16384 x 512 x 2048 + GELU 63.9 -> 53.7 us,
 // with a residual 98.0 -> 81.2; 16384 x 1024 x 1024 41.6 -> 37.4), eight beyond, where more of them only take issue slots and
-// power (the fp32 planes of 16384 x 1728 x 1024 and 1024 x 512: 415 -> 440 us a recommender pass with sixteen).
+// power (the fp32 planes of 16384 x 1728 x 1024 and 1024 x 512: 415 -> 440 us with sixteen for a recommender pass replayed as a CUDA
+// graph; a pass launched by the operator is 480).
 constexpr int kPairShortK = 1024 / BK;  // k-blocks
 constexpr int PAIR_STAGE_BYTES = (BM + PAIR_BN / 2) * BK * 2;  // per CTA: A tile + half of the W tile = 32 KiB
 constexpr int PAIR_SMEM_BYTES = PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + 256;
@@ -1180,7 +1181,8 @@ bool use_cta_pairs(int64_t M, int64_t N, int out_bn) {
 // cost model in microseconds fitted to sweeps on B200 (K = 4096; M = 16..128; N = 512..11008; tile widths 64 / 128 /
 // 256; 1..16 splits; CUDA-graph replay):
 //   ingest  : 8.5 us per MB a CTA takes in (about 118 KB/us per SM), times the waves;
-//   tile    : 0.01 us per tile column (the epilogue of a wide tile is served by the same warps);
+//   tile    : 0.01 us per tile column (a wide tile has no more epilogue warps than a narrow one; fitted when they were four, not again since they
+//             are eight, which makes it a little too much);
 //   launch  : 2.5 us;
 //   a split : 4 us more (second launch, drain) and the fp32 partial sums written and read back: 0.13 us per MB while
 //             weights + partial sums stay within L2, 0.67 us per MB beyond that.
@@ -1551,7 +1553,8 @@ int gemm_tc_static_entry(const void* A, const void* B, const void* bias, const v
 
 // Whether `count` layers of one input, some with the rotary epilogue, run faster as one launch of the grouped kernel than one
 // after the other, and with which tile width. A single layer with less than a wave of tiles leaves SMs idle and pays for its
-// ramp alone. Microseconds as in plan_gemm: a tile takes in (128 + bn) rows of 128 bytes per k-block at about 118 KB/us,
+// ramp alone. (Callers group only layers that one by one would not split K: the grouped kernel adds a row up in one chain.)
+// Microseconds as in plan_gemm: a tile takes in (128 + bn) rows of 128 bytes per k-block at about 118 KB/us,
 // 3 us per launch; the line lies where the model sees 5 %. Measured (K = N = 4096 bf16, three layers, two with RoPE, weights not
 // in L2; one launch / three): 16 rows 24.0 / 49.9 us, 128 rows 28.0 / 60.7, 333 rows 41.7 / 66.4, 512 rows 53.5 / 66.5, 1000 rows
 // 88.1 / 102.5, 2048 rows 180.5 / 176.8; K = N = 512: 16 rows 7.0 / 20.4, 1000 rows 9.8 / 25.6. Layers that fill the chip

@@ -499,7 +499,7 @@ bool ksplit_shape_ok(int S, int tn, int64_t nkb) {
 // K = 4096 means 128 < M <= 512 at N = 4096 (13.3 vs 15.7 us at M = 256, 19.6 vs 26.9 us at M = 512) and M <= 256 at
 // N = 11008 (22.3 vs 36.3 us), and shapes with between one and two waves of 256 x 256 tiles (512 x 11008: 43 vs
 // 51 us for the pair kernel). Smaller M stays with split-K through scratch, which is ahead there; fp32 problems
-// (`f32x3`, K = 6 x the padded K) have no such path and come here at any M.
+// (`f32x3`, K = 6 x the padded K) have no such path and come here at any M. (All of it was measured in plain stream order.)
 static bool plan_clusters(bool f32x3, int64_t M, int64_t N, int64_t K, int dtype, int* S_out, int* tn_out) {
     static const int forced_s = []() {
         const char* e = getenv("XG_GEMM_KSPLIT");
@@ -555,7 +555,9 @@ static bool plan_clusters(bool f32x3, int64_t M, int64_t N, int64_t K, int dtype
     double other = (double)((ctas + sms - 1) / sms) * (double)nkb * (16.0 + bn * 0.125) / 127.0 + 3.0;
     if (tiles256 >= sms / 2) {
         // between one and two waves of 256 x 256 tiles the dispatcher would take the persistent pair kernel, whose last
-        // wave is mostly empty (86 tiles on 74 pairs: 51 us at 512 x 4096 x 11008 against 43 us for 138 tiles of 160 columns)
+        // wave is mostly empty (86 tiles on 74 pairs: 51 us at 512 x 4096 x 11008 against 43 us for 138 tiles of 160 columns),
+        // or 128-row CTAs where those need a quarter fewer waves (use_cta_pairs); by this model they are then the cheaper ones
+        // too, so that counting the pair kernel as well changes no choice (all M <= 4096, N <= 16384 gone through)
         const double pair = (double)((tiles256 + sms / 2 - 1) / (sms / 2)) * ((double)nkb * per_kblock(32.0, 256) + 3.6);
         if (pair < other) other = pair;
     }

@@ -1,10 +1,12 @@
 """The benchmark graphs after the ``cuda_sm100`` rewrite, assembled directly from the target's operators.
 
-Each class takes the eager model from ``workloads.py``, shares its parameters (no copies except the
-stated re-layouts) and issues, in ``forward``, exactly the fused-op sequence that xpu_graph's pattern
-pass produces for that model with this target, as one native operator (csrc/torch_ops.cpp). They let the fused path run
-(and be measured) where the xpu_graph package itself is not installed; tests/test_target_patterns.py checks, where it is,
-that compiling the eager model through XpuGraph yields the same op sequence. Inference only: results carry no gradient.
+Each class takes the eager model from ``workloads.py``, shares its parameters (no copies) and runs, in ``forward``, the fused-op
+sequence that xpu_graph's pattern pass produces for that model with this target, as one native operator (csrc/torch_ops.cpp): bit
+for bit the results of the replacement modules called one after the other, with fewer launches where the operator joins two (q
+and k of few rows; the recommender's copies and lookups). A compiled graph calls the modules; no pattern emits these operators.
+They let the fused path run (and be measured) where the xpu_graph package itself is not installed; tests/test_target_patterns.py
+checks, where it is, that compiling the eager model through XpuGraph yields that op sequence. Inference only: results carry no
+gradient.
 """
 from __future__ import annotations
 
